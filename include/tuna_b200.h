@@ -241,11 +241,13 @@ int tuna_matmul_sequence_reduce(const tuna_gemm_desc *gemms, int count, const vo
 /*
  * Quantizer: w fp16 [m, k] row-major -> packed codes q [m/8, k/8, 32] + absmax fp32 [m], for the
  * codebook `code` fp32 [16].  Replaces the reference's quantize_blockwise_dynamic_4bit(w,
- * block_size = k, preprocess = True) (test.py:7-68, a chain of torch kernels) with two kernels;
+ * block_size = k, preprocess = True) (test.py:7-68, a chain of torch kernels) with one kernel;
  * bit-identical results: absmax = max |w| per row, code = first index of the nearest codebook
  * entry to fp32(w) / absmax (fp32 division).  m and k multiples of 8; w and q 16-byte aligned.
  */
 int tuna_quantize(const void *w, const void *code, void *q, void *absmax, int m, int k, void *stream);
+/* The same with the NF4 levels, which are also written to code_out fp32 [16]: nothing to upload. */
+int tuna_quantize_nf4(const void *w, void *q, void *absmax, void *code_out, int m, int k, void *stream);
 
 const char *tuna_status_string(int status);
 

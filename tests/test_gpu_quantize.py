@@ -62,3 +62,28 @@ def test_rejects_bad_arguments():
         tuna_b200.quantize(torch.zeros((8, 8), dtype=torch.float32, device="cuda"))
     with pytest.raises(tuna_b200.TunaError):
         tuna_b200.quantize(torch.zeros((12, 8), dtype=torch.float16, device="cuda"))
+
+
+# one CTA per row group up to 4096 columns, clusters above, the two-pass kernels beyond 112000; rows of every kind
+@pytest.mark.parametrize("m,k", [(16, 8), (32, 4088), (16, 4096), (16, 4104), (48, 10008), (8, 28672), (16, 32776), (8, 112000), (16, 112008)])
+@pytest.mark.parametrize("book", ["nf4", "unsorted", "close", "duplicate"])
+def test_every_share_and_codebook_is_bit_exact(m, k, book):
+    rng = np.random.default_rng(m + k)
+    w = (rng.standard_normal((m, k)) * 0.05).astype(np.float16)
+    w[1] = 0
+    w[2] *= np.float16(1e-3)           # 63 / absmax overflows fp16: the literal expression
+    w[3] = rng.integers(-8, 9, k) / 8  # exact midpoints and end points
+    w[4, 0] = 60000
+    w[5, k - 1] = np.float16(-6e-8)
+    code = orc.NF4_CODE.copy()
+    if book == "unsorted":             # sign-magnitude order
+        code = np.array([0.01, 0.1, 0.2, 0.3, 0.45, 0.6, 0.8, 1, -0.02, -0.1, -0.2, -0.3, -0.45, -0.6, -0.8, -1.5], dtype=np.float32)
+    elif book == "close":              # two thresholds in one bucket
+        code[8] = 0.001
+    elif book == "duplicate":
+        code[8] = 0.0
+    q, (absmax, c) = tuna_b200.quantize(torch.from_numpy(w).cuda(), None if book == "nf4" else torch.from_numpy(code).cuda())
+    q_ref, a_ref, _ = orc.quantize_blockwise_dynamic_4bit(w, code)
+    assert np.array_equal(c.cpu().numpy(), code)
+    assert np.array_equal(absmax.cpu().numpy(), a_ref)
+    assert np.array_equal(q.cpu().numpy(), q_ref)

@@ -72,6 +72,7 @@ SYMBOLS = {
     "tuna_lookup_config": (c_int, [c_int] * 3 + [ctypes.POINTER(TunaConfig)]),
     "tuna_dequant": (c_int, [c_void_p] * 4 + [c_int] * 2 + [c_void_p]),
     "tuna_quantize": (c_int, [c_void_p] * 4 + [c_int] * 2 + [c_void_p]),
+    "tuna_quantize_nf4": (c_int, [c_void_p] * 4 + [c_int] * 2 + [c_void_p]),
     "tuna_check_device_status": (c_int, [c_void_p]),
     "tuna_selftest_bounded_wait": (c_int, [c_void_p]),
     "tuna_status_string": (c_char_p, [c_int]),

@@ -45,7 +45,8 @@ bool make_tensor_map_3d(CUtensorMap *map, CUtensorMapDataType dt, const void *ba
 bool make_tensor_map_nd(CUtensorMap *map, CUtensorMapDataType dt, const void *base, int rank, const uint64_t *dims,
                         const uint64_t *strides, const uint32_t *box, CUtensorMapSwizzle swizzle);
 
-cudaError_t launch_quantize(const void *w, const void *code, void *q, void *absmax, int m, int k, int sm_count,
+// code == nullptr: NF4, written to code_out (which may be nullptr)
+cudaError_t launch_quantize(const void *w, const void *code, void *code_out, void *q, void *absmax, int m, int k, int sm_count,
                             cudaStream_t stream);
 cudaError_t launch_dequant(const void *q, const void *absmax, const void *code, void *o, int m,
                            int k, int sm_count, cudaStream_t stream);

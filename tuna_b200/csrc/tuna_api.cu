@@ -286,7 +286,17 @@ extern "C" int tuna_quantize(const void *w, const void *code, void *q, void *abs
     int st = check_shape(m, 1, k);
     if (st != TUNA_OK) return st;
     if (!aligned(w, 16) || !aligned(q, 16) || !aligned(absmax, 4) || !aligned(code, 4)) return TUNA_ERR_MISALIGNED;
-    cudaError_t e = launch_quantize(w, code, q, absmax, m, k, device_sm_count(), (cudaStream_t)stream);
+    cudaError_t e = launch_quantize(w, code, nullptr, q, absmax, m, k, device_sm_count(), (cudaStream_t)stream);
+    return e == cudaSuccess ? TUNA_OK : TUNA_ERR_LAUNCH;
+}
+
+extern "C" int tuna_quantize_nf4(const void *w, void *q, void *absmax, void *code_out, int m, int k, void *stream)
+{
+    if (!w || !code_out || !q || !absmax) return TUNA_ERR_NULL_POINTER;
+    int st = check_shape(m, 1, k);
+    if (st != TUNA_OK) return st;
+    if (!aligned(w, 16) || !aligned(q, 16) || !aligned(absmax, 4) || !aligned(code_out, 4)) return TUNA_ERR_MISALIGNED;
+    cudaError_t e = launch_quantize(w, nullptr, code_out, q, absmax, m, k, device_sm_count(), (cudaStream_t)stream);
     return e == cudaSuccess ? TUNA_OK : TUNA_ERR_LAUNCH;
 }
 

@@ -429,20 +429,23 @@ def quantize(w, codebook=None):
     `quantize_blockwise_dynamic_4bit(w, block_size=k, preprocess=True)` (test.py:7-68) with the
     same return structure `(q, (absmax, code))`: `q` uint8 `[m/8, k/8, 32]`, `absmax` fp32 `[m]`,
     `code` fp32 `[16]` (NF4 unless `codebook` is given)."""
-    from .codebooks import nf4_tensor
-
     if not isinstance(w, torch.Tensor) or not w.is_cuda:
         raise ValueError("w must be a CUDA tensor (there is no CPU path)")
     if w.dtype != torch.float16 or w.dim() != 2 or not w.is_contiguous():
         raise ValueError("w must be a contiguous fp16 [m, k] tensor")
     m, k = w.shape
-    code = nf4_tensor(w.device) if codebook is None else codebook
-    _expect(code, "codebook", torch.float32, 16, w.device)
+    if codebook is not None:
+        _expect(codebook, "codebook", torch.float32, 16, w.device)
     q = torch.empty((m // 8, k // 8, 32), dtype=torch.uint8, device=w.device)
     absmax = torch.empty((m,), dtype=torch.float32, device=w.device)
+    code = torch.empty((16,), dtype=torch.float32, device=w.device) if codebook is None else codebook
     with torch.cuda.device(w.device):
-        check(_lib.load().tuna_quantize(w.data_ptr(), code.data_ptr(), q.data_ptr(), absmax.data_ptr(), m, k,
-                                        _stream_ptr(w.device)))
+        if codebook is None:  # the kernel knows the NF4 levels: no upload, no synchronisation
+            check(_lib.load().tuna_quantize_nf4(w.data_ptr(), q.data_ptr(), absmax.data_ptr(), code.data_ptr(), m, k,
+                                                _stream_ptr(w.device)))
+        else:
+            check(_lib.load().tuna_quantize(w.data_ptr(), code.data_ptr(), q.data_ptr(), absmax.data_ptr(), m, k,
+                                            _stream_ptr(w.device)))
     return q, (absmax, code)
 
 
