@@ -58,7 +58,7 @@ WORKLOADS = {
 FALLBACK_HBM_GBS = 6650.0
 NOMINAL_FP16_TFLOPS = 2250.0
 TARGET_TIMED_SECONDS = 1.0
-KERNEL_NAMES = {1: "gemm_stream_kernel (mma.sync)", 2: "gemm_w4a16_umma_kernel (tcgen05, TMA-staged)",
+KERNEL_NAMES = {1: "gemm_stream_kernel (mma.sync)", 2: "gemm_w4a16_pair_kernel (tcgen05, two SMs per tile)",
                 3: "gemm_w4a16_tstream_kernel (tcgen05 weight streaming)"}
 
 

@@ -46,7 +46,7 @@ typedef enum tuna_status {
 typedef enum tuna_path {
     TUNA_PATH_AUTO = 0,
     TUNA_PATH_STREAM = 1, /* register-streaming mma.sync kernel, small token counts       */
-    TUNA_PATH_UMMA = 2,   /* tcgen05/TMEM kernel: TMA-staged, dequant into TMEM       */
+    TUNA_PATH_UMMA = 2,   /* tcgen05 kernel, two SMs per tile: large token counts     */
     TUNA_PATH_TSTREAM = 3 /* tcgen05 weight-streaming kernel: ld.global -> table ->   *
                            * tcgen05.st fragments, small token counts                 */
 } tuna_path;
@@ -57,19 +57,19 @@ typedef enum tuna_path {
 typedef struct tuna_config {
     int32_t path;          /* tuna_path                                               */
     int32_t tile_tok;      /* tokens per pass: stream 8|16|32; tstream 16|32|64|128;  *
-                            * umma 16|32|64|128|256                                   */
+                            * umma 16|32|64|128|256 (the largest tile; 0 = by shape)  */
     int32_t rows_per_warp; /* stream: 32-row blocks per warp (1|2)                    */
     int32_t warps_m;       /* stream: consumer warps along output rows (power of 2)   */
     int32_t warps_k;       /* stream: consumer warps along K (power of 2, m*k <= 16)  */
     int32_t k_steps;       /* stream: 32-column steps per warp per unit (8|16|32|64); *
                             * tstream: 32-column steps per slot (4|8)                 */
     int32_t ctas;          /* persistent CTAs (0 = one per SM)                        */
-    int32_t stages_w;      /* umma: packed-weight ring depth (64-column stages)       */
-    int32_t stages_x;      /* umma: unit stages (activation tile + A-operand slots)   */
-    int32_t dequant_warps; /* umma: warps converting codes into TMEM (mult of 4)      */
-    int32_t row_blocks;    /* umma, tstream: 128-row blocks per CTA tile (1|2|4)      */
-    int32_t stages_a;      /* umma: derived (stages_x * row_blocks TMEM operand slots) */
-    int32_t k_accs;        /* umma: accumulators per row block along K (1|2|4)        */
+    int32_t stages_w;      /* umma: 0, or 4..16 (range-checked; the kernel derives it) */
+    int32_t stages_x;      /* umma: 0, or 2..16 (the same)                            */
+    int32_t dequant_warps; /* umma: 0, 8 or 16 (the same)                             */
+    int32_t row_blocks;    /* tstream: 128-row blocks per CTA tile (1|2|4); umma as above */
+    int32_t stages_a;      /* ignored                                                 */
+    int32_t k_accs;        /* umma: 0 or 1 (as above)                                 */
     int32_t reserved[3];
 } tuna_config;
 

@@ -829,11 +829,10 @@ static int launch_ts_dispatch(const TsLaunch<MAXG> &L, int tile_tok, int steps, 
 
 // Fills the table entry of one GEMM (tensor maps, geometry); `unit0` / `tile0` are where its units
 // and tiles start in the launch.  Returns its unit count, or a negative status.
-static bool ts_wmode1_shape(int m, int k) { return m % 32 == 0 && k % 64 == 0; }
-
 static long long ts_fill_gemm(TsGemm *g, const void *q, const void *x, const float *absmax, void *o, int m, int n, int k,
-                              int row_blocks, int steps, int tile_tok, int unit0, int tile0, int w_mode)
+                              int row_blocks, int steps, int tile_tok, int unit0, int tile0, const int w_mode_wanted)
 {
+    int w_mode = w_mode_wanted;
     const int chunk_k = 32 * steps;
     std::memset(g, 0, sizeof(*g));
     g->absmax = absmax; g->o = (__half *)o;
@@ -842,33 +841,8 @@ static long long ts_fill_gemm(TsGemm *g, const void *q, const void *x, const flo
     g->row_tiles = div_up(m, kBlockRows * row_blocks);
     g->unit0 = unit0;
     g->tile0 = tile0;
-    // Packed weights (a row group is 4k bytes = k 32-bit words; word index = column index).  One
-    // step of a slot is a box of 16 row groups x 32 words (128 bytes), 128-byte swizzled.  Where k
-    // is a multiple of 32 the matrix also has the 3-D view [k/32 steps][m/8 row groups][32 words]
-    // (strides 128 bytes and 4k bytes) and a slot is one box of `steps` x 16 x 32; otherwise, or if
-    // the driver refuses that view, the 2-D view and one box per step.  Rows, columns and steps
-    // past the matrix are zero-filled by the copy.
-    // w_mode 1: 32-row blocks x pairs of steps, [m/32][k/64][4 row groups][2 steps][32 words] with
-    // strides 16k, 256, 4k and 128 bytes; a slot is one box of 4 x steps/2 x 4 x 2 x 32 words.
-    g->q3d = 0;
-    if (w_mode == 1) {
-        const uint64_t dims[5] = {32, 2, 4, (uint64_t)k / 64, (uint64_t)m / 32};
-        const uint64_t strides[4] = {128, (uint64_t)k * 4, 256, (uint64_t)k * 16};
-        const uint32_t box[5] = {32, 2, 4, (uint32_t)steps / 2, 4};
-        if (!ts_wmode1_shape(m, k) || !make_tensor_map_nd(&g->map_q, CU_TENSOR_MAP_DATA_TYPE_UINT32, q, 5, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B))
-            return TUNA_ERR_BAD_CONFIG;
-    } else
-#ifdef TS_FORCE_Q2D  // timing experiment: one 2-D box per step even where the 3-D view exists
-    if (false &&
-#else
-    if (k % 32 == 0 &&
-#endif
-        make_tensor_map_3d(&g->map_q, CU_TENSOR_MAP_DATA_TYPE_UINT32, q, 32, (uint64_t)m / 8, (uint64_t)k / 32, (uint64_t)k * 4, 128,
-                           32, 16, (uint32_t)steps, CU_TENSOR_MAP_SWIZZLE_128B))
-        g->q3d = 1;
-    else if (!make_tensor_map_2d(&g->map_q, CU_TENSOR_MAP_DATA_TYPE_UINT32, q, (uint64_t)k, (uint64_t)m / 8, (uint64_t)k * 4, 32, 16,
-                                 CU_TENSOR_MAP_SWIZZLE_128B))
-        return TUNA_ERR_NO_DEVICE;
+    if (!make_weight_map(&g->map_q, q, m, k, steps, &w_mode, &g->q3d)) return TUNA_ERR_NO_DEVICE;
+    if (w_mode != w_mode_wanted) return TUNA_ERR_BAD_CONFIG;  // the driver refused the 5-D view: the caller falls back
     // activations as [n tokens] x [k] fp16; box = tile_tok tokens x 64 columns (128-byte rows, swizzled)
     if (!make_tensor_map_2d(&g->map_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, x, (uint64_t)k, (uint64_t)n, (uint64_t)k * 2, 64,
                             (uint32_t)tile_tok, CU_TENSOR_MAP_SWIZZLE_128B))
@@ -899,7 +873,7 @@ int launch_gemm_tstream(const GemmArgs &a, const tuna_config &c)
     if (a.workspace == nullptr || a.workspace_bytes < gemm_tstream_workspace_bytes(a.m, a.n, a.k, c, a.sm_count))
         return TUNA_ERR_WORKSPACE;
     ts_fill_common(&L.c, c, steps, a.workspace, a.sm_count);
-    L.c.w_mode = ts_wmode1_shape(a.m, a.k) ? 1 : 0;
+    L.c.w_mode = weight_map_has_runs(a.m, a.k) ? 1 : 0;
     long long units = ts_fill_gemm(&L.g[0], a.q, a.x, a.absmax, a.o, a.m, a.n, a.k, c.row_blocks, steps, c.tile_tok, 0, 0, L.c.w_mode);
     if (units == TUNA_ERR_BAD_CONFIG && L.c.w_mode == 1) {  // the driver refused the 5-D view
         L.c.w_mode = 0;
@@ -986,7 +960,7 @@ int launch_gemm_tstream_sequence(const tuna_gemm_desc *d, int count, const float
         // one stage layout per launch: the 256-byte-run one if every GEMM has it
         L.c.w_mode = 1;
         for (int i = 0; i < cnt; ++i)
-            if (!ts_wmode1_shape(d[first + i].m, d[first + i].k)) L.c.w_mode = 0;
+            if (!weight_map_has_runs(d[first + i].m, d[first + i].k)) L.c.w_mode = 0;
         long long units = 0;
         const int tile0_launch = tile0;
         for (int attempt = 0; attempt < 2; ++attempt) {

@@ -98,6 +98,35 @@ bool make_tensor_map_nd(CUtensorMap *map, CUtensorMapDataType dt, const void *ba
               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+bool weight_map_has_runs(int m, int k) { return m % 32 == 0 && k % 64 == 0; }
+
+// Tensor map of the packed weights for stages of `steps` 32-column steps x 128 rows (a row group is 4k bytes = k 32-bit
+// words; word index = column index), 128-byte swizzled.
+//   *w_mode 1: 32-row blocks x pairs of steps, [m/32][k/64][4 row groups][2 steps][32 words] with strides 16k, 256, 4k
+//              and 128 bytes; a stage is one box of 4 x steps/2 x 4 x 2 x 32 words (256-byte runs of global memory);
+//   *w_mode 0: where k is a multiple of 32 the 3-D view [k/32 steps][m/8 row groups][32 words] (strides 128 bytes and
+//              4k bytes; *q3d = 1), a stage being one box of steps x 16 x 32; otherwise, or if the driver refuses that
+//              view, the 2-D view and one box of 16 row groups x 32 words per step.
+// A refused 5-D view sets *w_mode to 0.  Rows, columns and steps past the matrix are zero-filled by the copy.
+bool make_weight_map(CUtensorMap *map, const void *q, int m, int k, int steps, int *w_mode, int *q3d)
+{
+    *q3d = 0;
+    if (*w_mode == 1) {
+        const uint64_t dims[5] = {32, 2, 4, (uint64_t)k / 64, (uint64_t)m / 32};
+        const uint64_t strides[4] = {128, (uint64_t)k * 4, 256, (uint64_t)k * 16};
+        const uint32_t box[5] = {32, 2, 4, (uint32_t)steps / 2, 4};
+        if (weight_map_has_runs(m, k) && make_tensor_map_nd(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, q, 5, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B))
+            return true;
+        *w_mode = 0;
+    }
+    if (k % 32 == 0 && make_tensor_map_3d(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, q, 32, (uint64_t)m / 8, (uint64_t)k / 32, (uint64_t)k * 4, 128, 32, 16,
+                                          (uint32_t)steps, CU_TENSOR_MAP_SWIZZLE_128B)) {
+        *q3d = 1;
+        return true;
+    }
+    return make_tensor_map_2d(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, q, (uint64_t)k, (uint64_t)m / 8, (uint64_t)k * 4, 32, 16, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
 }  // namespace tuna
 
 // ------------------------------------------------------------------ self-test of the bounded waits

@@ -45,6 +45,10 @@ bool make_tensor_map_3d(CUtensorMap *map, CUtensorMapDataType dt, const void *ba
 bool make_tensor_map_nd(CUtensorMap *map, CUtensorMapDataType dt, const void *base, int rank, const uint64_t *dims,
                         const uint64_t *strides, const uint32_t *box, CUtensorMapSwizzle swizzle);
 
+// Tensor maps of the packed weights, shared by the TMA kernels (see host_util.cu).
+bool weight_map_has_runs(int m, int k);
+bool make_weight_map(CUtensorMap *map, const void *q, int m, int k, int steps, int *w_mode, int *q3d);
+
 // code == nullptr: NF4, written to code_out (which may be nullptr)
 cudaError_t launch_quantize(const void *w, const void *code, void *code_out, void *q, void *absmax, int m, int k, int sm_count,
                             cudaStream_t stream);
@@ -59,7 +63,7 @@ int gemm_stream_normalize_config(int m, int n, int k, int sm_count, tuna_config 
 size_t gemm_stream_compact_scratch_bytes(int m, int k, const tuna_config &cfg, size_t *counter_bytes);
 int launch_gemm_stream_compact(const GemmArgs &a, const tuna_config &cfg, void *scratch, size_t counter_bytes, DeviceStatus *status);
 
-// tcgen05/TMEM kernel.  Returns a tuna_status.
+// tcgen05 kernel for large token counts (CTA pairs).  Returns a tuna_status.
 int launch_gemm_umma(const GemmArgs &a, const tuna_config &cfg);
 size_t gemm_umma_workspace_bytes(int m, int n, int k, const tuna_config &cfg, int sm_count);
 int gemm_umma_normalize_config(int m, int n, int k, int sm_count, tuna_config *cfg);

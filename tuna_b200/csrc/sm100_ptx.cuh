@@ -79,6 +79,43 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, vo
     return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, where)) != 0;
 }
 
+// ---- CTA pairs: barriers that the other CTA of the cluster arrives at
+
+__device__ __forceinline__ uint32_t cluster_ctarank()
+{
+    uint32_t r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// Address, in the cluster's shared window, of what lies at `addr` in CTA `rank`.
+__device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, int rank)
+{
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+// What these barriers order between the CTAs is tensor memory (tcgen05 fences on both sides) and TMA copies seen complete,
+// never generic stores, so the default scope of the release and of the waits is enough; a release at cluster scope
+// made every arrival wait ~1000 clocks (57344x8192 at 2048 tokens: 2460 us instead of 1357).
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar)
+{
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
+__device__ __forceinline__ void cluster_sync_all()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Named barrier of `threads` threads that answers, to all of them, whether any came with `v`.
+__device__ __forceinline__ bool bar_any(int id, int threads, bool v)
+{
+    uint32_t r;
+    asm volatile("{\n .reg .pred p, q;\n setp.ne.b32 p, %3, 0;\n barrier.cta.red.or.pred q, %1, %2, p;\n selp.u32 %0, 1, 0, q;\n}"
+                 : "=r"(r)
+                 : "r"(id), "r"(threads), "r"((uint32_t)v)
+                 : "memory");
+    return r != 0;
+}
+
 // True in exactly one lane of a converged warp.
 __device__ __forceinline__ bool elect_one_sync()
 {
@@ -111,6 +148,13 @@ __device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap *map
         : "memory");
 }
 
+// Shared -> global, clipped at the tensor's bounds; the caller commits and waits for the bulk group.
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap *map, int c0, int c1, uint32_t src)
+{
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(map), "r"(c0), "r"(c1), "r"(src)
+                 : "memory");
+}
+
 // Position in a ring of n mbarrier-guarded buffers: slot index and the parity of its current use.
 struct Ring {
     int idx;
@@ -121,11 +165,5 @@ struct Ring {
         if (++idx == n) { idx = 0; phase ^= 1u; }
     }
 };
-
-// The CTA i whose contiguous range [floor(i*U/G), floor((i+1)*U/G)) holds unit u.
-__device__ __forceinline__ int cta_of_unit(long long u, long long units, int ctas)
-{
-    return (int)(((u + 1) * ctas + units - 1) / units) - 1;
-}
 
 }  // namespace tuna

@@ -40,9 +40,8 @@ TSTREAM_SPACE = {
     "row_blocks": (1, 2, 4),
     "k_steps": (4, 8),
 }
-# The TMA-staged kernel is measured with its own defaults only (0 = default): two searches over
-# its stage counts, dequant warps and accumulator split ended in a launch failure on 57344x8192
-# (64- and 256-token tiles) with combinations no GPU test exercises, so the tuner does not explore them.
+# The kernel for large token counts derives its tile, stages and work split from the shape
+# (gemm_pair_sm100a.cu): there is nothing to search, 0 = its own choice.
 UMMA_SPACE = {
     "row_blocks": (0,),
     "stages_w": (0,),
