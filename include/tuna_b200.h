@@ -158,10 +158,10 @@ int tuna_matmul_noalloc(const void *q, const void *x, const void *code, const vo
  * `batch` independent GEMMs of one shape in one call: matrix b uses q + b*q_stride,
  * x + b*x_stride (0 = the same activations for all), absmax + b*absmax_stride and writes
  * o + b*o_stride (strides in bytes, multiples of 16; `code` is shared).  For token counts of the
- * streaming kernel (n <= 32) this is ONE launch whose work split runs across the matrices, so
- * the fixed cost per launch is paid once: the Mixtral expert projections (8 GEMMs of
- * 14336 -> 4096, per-expert activations) or the reference's "combined" 14336 -> 32768 GEMM
- * (make_configs.py:105-106, README.md:18: x_stride = 0).  Larger n: one launch per matrix.
+ * weight-streaming kernels (n <= 64) this is ONE launch (one per 64 matrices) whose work split runs
+ * across the matrices, so the fixed cost per launch is paid once: the Mixtral expert projections
+ * (8 GEMMs of 14336 -> 4096, per-expert activations) or the reference's "combined" 14336 -> 32768
+ * GEMM (make_configs.py:105-106, README.md:18: x_stride = 0).  Larger n: one launch per matrix.
  * Workspace: tuna_matmul_batched_workspace_bytes (zero before the first use, left clean).
  */
 int tuna_matmul_batched(const void *q, const void *x, const void *code, const void *absmax, void *o,

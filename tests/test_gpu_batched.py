@@ -50,3 +50,38 @@ def test_batched_equals_separate_calls_bit_for_bit_and_is_repeatable():
     o = first.cpu().numpy()
     for b in range(batch):
         check_parity(o[b], orc.matmul_ref(x[b], per[b][1], per[b][2], code, m, n, k), 1e-2)
+
+
+def _batched_abi(xd, qd, sd, cd, out, batch, m, n, k, ws, o_stride=None):
+    lib = tuna_b200._lib.load()
+    return lib.tuna_matmul_batched(qd.data_ptr(), xd.data_ptr(), cd.data_ptr(), sd.data_ptr(), out.data_ptr(), m, n, k, batch, m * k // 2,
+                                   n * k * 2, m * 4, n * m * 2 if o_stride is None else o_stride, ws.data_ptr(), ws.numel(),
+                                   torch.cuda.current_stream().cuda_stream)
+
+
+@pytest.mark.parametrize("batch,m,n,k", [(70, 136, 16, 264), (66, 64, 33, 128)])
+def test_batched_more_matrices_than_one_launch_and_small_workspaces(batch, m, n, k):
+    """Batches beyond one launch's table, and workspaces that hold the counters of one matrix only: the same results."""
+    lib = tuna_b200._lib.load()
+    per, x, q, s, code = _case(batch, m, n, k, 1200 + n, False)
+    xd, qd, sd, cd = (torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (x, q, s, code))
+    for need in (lib.tuna_matmul_batched_workspace_bytes(m, n, k, batch), lib.tuna_matmul_workspace_bytes(m, n, k)):
+        out = torch.full((batch, n, m), float("nan"), dtype=torch.float16, device="cuda")
+        ws = torch.zeros(need, dtype=torch.uint8, device="cuda")
+        assert _batched_abi(xd, qd, sd, cd, out, batch, m, n, k, ws) == 0
+        torch.cuda.synchronize()
+        assert lib.tuna_check_device_status(torch.cuda.current_stream().cuda_stream) == 0
+        o = out.cpu().numpy()
+        for b in range(batch):
+            check_parity(o[b], orc.matmul_ref(x[b], per[b][1], per[b][2], code, m, n, k), 1e-2)
+
+
+def test_batched_outputs_that_share_memory_are_written_in_order():
+    batch, m, n, k = 3, 256, 16, 512
+    per, x, q, s, code = _case(batch, m, n, k, 77, False)
+    xd, qd, sd, cd = (torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (x, q, s, code))
+    ws = torch.zeros(tuna_b200._lib.load().tuna_matmul_batched_workspace_bytes(m, n, k, batch), dtype=torch.uint8, device="cuda")
+    out = torch.empty((n, m), dtype=torch.float16, device="cuda")
+    assert _batched_abi(xd, qd, sd, cd, out, batch, m, n, k, ws, o_stride=0) == 0
+    torch.cuda.synchronize()
+    check_parity(out.cpu().numpy(), orc.matmul_ref(x[2], per[2][1], per[2][2], code, m, n, k), 1e-2)

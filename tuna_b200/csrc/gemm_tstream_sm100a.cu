@@ -113,7 +113,7 @@ constexpr int kTsDequantWarp0 = 8;
 constexpr int kTsDequantWarps = TS_DEQUANT_WARPS;
 constexpr int kTsThreads = 32 * (kTsDequantWarp0 + kTsDequantWarps);
 
-constexpr int kTsMaxSeq = 64;  // GEMMs of one launch (tuna_matmul_sequence)
+constexpr int kTsMaxSeq = kSequenceMax;  // GEMMs of one launch (tuna_matmul_sequence)
 constexpr int kMaxPeers = TUNA_MAX_PEERS;
 
 // One GEMM of a launch.  The two tensor maps are what the copy producer hands to TMA; everything
@@ -903,6 +903,26 @@ size_t gemm_tstream_sequence_workspace_bytes(const tuna_gemm_desc *d, int count,
     return partial_region_bytes(sm_count) + (tiles * 16 + 255) / 256 * 256;
 }
 
+// Token tile and row blocks per tile of a launch whose largest token count is max_n: as many row
+// blocks as the accumulator columns allow, because they share one activation stage (measured on the
+// Mistral MLP sweep: 3.53 / 4.00 / 4.27 TB/s with 1 / 2 / 4 row blocks); the sequence as a whole is
+// still balanced at unit granularity (64 KB).
+static int ts_sequence_tile_tok(int max_n) { return max_n <= 16 ? 16 : (max_n <= 32 ? 32 : 64); }
+static int ts_sequence_row_blocks(int tile_tok) { return 64 / tile_tok; }
+
+size_t gemm_tstream_sequence_min_workspace_bytes(const tuna_gemm_desc *d, int count, int sm_count)
+{
+    size_t tiles = 0;
+    for (int first = 0; first < count; first += kTsMaxSeq) {
+        const int cnt = count - first < kTsMaxSeq ? count - first : kTsMaxSeq;
+        int max_n = 1;
+        for (int i = 0; i < cnt; ++i) max_n = d[first + i].n > max_n ? d[first + i].n : max_n;
+        const int rows = kBlockRows * ts_sequence_row_blocks(ts_sequence_tile_tok(max_n));
+        for (int i = 0; i < cnt; ++i) tiles += (size_t)div_up(d[first + i].m, rows);
+    }
+    return partial_region_bytes(sm_count) + (tiles * 16 + 255) / 256 * 256;
+}
+
 // Whether the sequence kernel can take these GEMMs (token counts of one pass; the rest is checked by the caller).
 bool gemm_tstream_sequence_supported(const tuna_gemm_desc *d, int count)
 {
@@ -915,7 +935,7 @@ bool gemm_tstream_sequence_supported(const tuna_gemm_desc *d, int count)
 int launch_gemm_tstream_sequence(const tuna_gemm_desc *d, int count, const float *code, void *workspace, size_t workspace_bytes,
                                  int sm_count, cudaStream_t stream, const tuna_exchange *ex)
 {
-    if (workspace == nullptr || workspace_bytes < gemm_tstream_sequence_workspace_bytes(d, count, sm_count)) return TUNA_ERR_WORKSPACE;
+    if (workspace == nullptr || workspace_bytes < gemm_tstream_sequence_min_workspace_bytes(d, count, sm_count)) return TUNA_ERR_WORKSPACE;
     DeviceStatus *status = device_status_word();
     if (!status) return TUNA_ERR_NO_DEVICE;
     int tile0 = 0;  // tiles of the GEMMs launched so far: every launch has its own counters
@@ -926,11 +946,8 @@ int launch_gemm_tstream_sequence(const tuna_gemm_desc *d, int count, const float
         tuna_config c;
         std::memset(&c, 0, sizeof(c));
         c.path = TUNA_PATH_TSTREAM;
-        c.tile_tok = max_n <= 16 ? 16 : (max_n <= 32 ? 32 : 64);
-        // as many row blocks per tile as the accumulator columns allow: they share one activation stage
-        // (measured on the Mistral MLP sweep: 3.53 / 4.00 / 4.27 TB/s with 1 / 2 / 4 row blocks); the
-        // sequence as a whole is still balanced at unit granularity (64 KB)
-        c.row_blocks = 64 / c.tile_tok;
+        c.tile_tok = ts_sequence_tile_tok(max_n);
+        c.row_blocks = ts_sequence_row_blocks(c.tile_tok);
         c.k_steps = 8;
         c.ctas = sm_count;
         static thread_local TsLaunch<kTsMaxSeq> L;  // ~20 KB: not on the stack

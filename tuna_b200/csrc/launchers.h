@@ -73,8 +73,10 @@ int launch_gemm_tstream(const GemmArgs &a, const tuna_config &cfg);
 size_t gemm_tstream_workspace_bytes(int m, int n, int k, const tuna_config &cfg, int sm_count);
 int gemm_tstream_normalize_config(int m, int n, int k, int sm_count, tuna_config *cfg);
 // The same kernel walking a table of independent GEMMs in one persistent launch (up to 64 per launch).
+constexpr int kSequenceMax = 64;
 bool gemm_tstream_sequence_supported(const tuna_gemm_desc *d, int count);
-size_t gemm_tstream_sequence_workspace_bytes(const tuna_gemm_desc *d, int count, int sm_count);
+size_t gemm_tstream_sequence_workspace_bytes(const tuna_gemm_desc *d, int count, int sm_count);      // whatever the token counts
+size_t gemm_tstream_sequence_min_workspace_bytes(const tuna_gemm_desc *d, int count, int sm_count);  // for these token counts
 // `ex` != nullptr: every GEMM is a K-split partial whose finished rows go to all ranks' exchange buffers,
 // and each launch is followed by the kernel that sums them into o (exchange_sm100a.cu).
 int launch_gemm_tstream_sequence(const tuna_gemm_desc *d, int count, const float *code, void *workspace, size_t workspace_bytes,
@@ -82,7 +84,7 @@ int launch_gemm_tstream_sequence(const tuna_gemm_desc *d, int count, const float
 
 // Exchange buffers (layout in exchange_sm100a.cu): header, then two parity regions.
 constexpr int kExMaxPeers = TUNA_MAX_PEERS;
-constexpr int kExMaxItems = 64;          // GEMMs per launch, as in the sequence kernel
+constexpr int kExMaxItems = kSequenceMax;  // GEMMs per launch, as in the sequence kernel
 constexpr int kExHeaderBytes = 4096;
 constexpr int kExFlag0Words = 64;        // flag of source rank j: 32-bit word 64 + 32 j of the header
 constexpr int kExFlagStrideWords = 32;

@@ -94,6 +94,10 @@ static int launch_gemm(const GemmArgs &a, const tuna_config &c)
     return launch_gemm_umma(a, c);
 }
 
+// Whether equal-shape GEMMs share persistent launches of the sequence kernel: every token count it
+// takes (eight 4096x14336 GEMMs of 16 tokens: 132 us as a launch each, 69 as one).
+static bool batched_as_sequence(const tuna_config &c, int n) { return c.path == TUNA_PATH_TSTREAM && n <= 64; }
+
 }  // namespace tuna
 
 using namespace tuna;
@@ -148,9 +152,28 @@ extern "C" int tuna_matmul_batched(const void *q, const void *x, const void *cod
         a.batch = batch; a.q_stride = q_stride; a.x_stride = x_stride; a.absmax_stride = absmax_stride; a.o_stride = o_stride;
         return launch_gemm_stream(a, c);
     }
-    // the tcgen05 kernels: one launch per matrix
     const size_t need = workspace_for(m, n, k, c, sms);
     if (workspace == nullptr || workspace_bytes < need) return TUNA_ERR_WORKSPACE;
+    if (batched_as_sequence(c, n) && batch > 1 && o_stride >= (size_t)n * m * 2) {
+        // persistent launches over up to 64 matrices each (as many as the workspace has counters for: at least one).
+        // Launches on a stream follow one another and leave the counters zero, so all use the same ones.
+        tuna_gemm_desc d[kSequenceMax];
+        for (int first = 0; first < batch;) {
+            int cnt = 0;
+            while (cnt < kSequenceMax && first + cnt < batch) {
+                const size_t b = (size_t)(first + cnt);
+                d[cnt] = {(const uint8_t *)q + b * q_stride, (const uint8_t *)x + b * x_stride, (const uint8_t *)absmax + b * absmax_stride,
+                          (uint8_t *)o + b * o_stride, m, n, k, 0};
+                if (cnt > 0 && gemm_tstream_sequence_min_workspace_bytes(d, cnt + 1, sms) > workspace_bytes) break;
+                ++cnt;
+            }
+            st = launch_gemm_tstream_sequence(d, cnt, a.code, workspace, workspace_bytes, sms, a.stream);
+            if (st != TUNA_OK) return st;
+            first += cnt;
+        }
+        return TUNA_OK;
+    }
+    // one launch per matrix
     for (int b = 0; b < batch; ++b) {
         a.q = (const uint8_t *)q + (size_t)b * q_stride;
         a.x = (const uint8_t *)x + (size_t)b * x_stride;
@@ -168,7 +191,16 @@ extern "C" size_t tuna_matmul_batched_workspace_bytes(int m, int n, int k, int b
     const int sms = device_sm_count();
     tuna_config c;
     if (resolve_config(m, n, k, sms, nullptr, &c) != TUNA_OK) return 0;
-    return c.path == TUNA_PATH_STREAM ? gemm_stream_workspace_bytes(m, n, k, c, sms, batch) : workspace_for(m, n, k, c, sms);
+    if (c.path == TUNA_PATH_STREAM) return gemm_stream_workspace_bytes(m, n, k, c, sms, batch);
+    size_t need = workspace_for(m, n, k, c, sms);
+    if (batched_as_sequence(c, n)) {
+        tuna_gemm_desc d[kSequenceMax] = {};
+        const int cnt = batch < kSequenceMax ? batch : kSequenceMax;
+        for (int i = 0; i < cnt; ++i) { d[i].m = m; d[i].n = n; d[i].k = k; }
+        const size_t w = gemm_tstream_sequence_min_workspace_bytes(d, cnt, sms);
+        need = w > need ? w : need;
+    }
+    return need;
 }
 
 // The GEMMs of a sequence that have tokens (n = 0 is an expert nobody was routed to: nothing to do).
@@ -211,9 +243,12 @@ extern "C" int tuna_matmul_sequence(const tuna_gemm_desc *g, int count, const vo
     if (st != TUNA_OK) return st;
     if (live.empty()) return TUNA_OK;
     const int sms = device_sm_count();
-    if (gemm_tstream_sequence_supported(live.data(), (int)live.size()))
+    if (gemm_tstream_sequence_supported(live.data(), (int)live.size())) {
+        if (workspace == nullptr || workspace_bytes < gemm_tstream_sequence_workspace_bytes(live.data(), (int)live.size(), sms))
+            return TUNA_ERR_WORKSPACE;
         return launch_gemm_tstream_sequence(live.data(), (int)live.size(), (const float *)code, workspace, workspace_bytes, sms,
                                             (cudaStream_t)stream);
+    }
     for (const tuna_gemm_desc &d : live) {
         st = tuna_matmul(d.q, d.x, code, d.absmax, d.o, d.m, d.n, d.k, workspace, workspace_bytes, stream);
         if (st != TUNA_OK) return st;
@@ -242,6 +277,8 @@ extern "C" int tuna_matmul_sequence_reduce(const tuna_gemm_desc *g, int count, c
         if (!aligned(d.q, 16) || !aligned(d.x, 16) || !aligned(d.o, 16) || !aligned(d.absmax, 4)) return TUNA_ERR_MISALIGNED;
     }
     if (ex->bytes < tuna_exchange_bytes(g, count, ex->world)) return TUNA_ERR_WORKSPACE;
+    if (workspace == nullptr || workspace_bytes < gemm_tstream_sequence_workspace_bytes(g, count, device_sm_count()))
+        return TUNA_ERR_WORKSPACE;
     return launch_gemm_tstream_sequence(g, count, (const float *)code, workspace, workspace_bytes, device_sm_count(),
                                         (cudaStream_t)stream, ex);
 }
