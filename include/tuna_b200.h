@@ -103,6 +103,11 @@ int tuna_matmul_cfg(const void *q, const void *x, const void *code, const void *
  * the workspace tuna_matmul needs.  Host-only arithmetic, no CUDA call. */
 size_t tuna_matmul_workspace_bytes(int m, int n, int k);
 
+/* Bytes at the start of every workspace that hold partial sums (the same for every shape on the
+ * current device).  They are written before they are read: only what follows them, the arrival
+ * counters, has to be zero before the first call. */
+size_t tuna_workspace_scratch_bytes(void);
+
 /* The configuration tuna_matmul would use for (m, n, k) on the current device:
  * exact table entry if param_map.json had one for the shape and token bucket,
  * otherwise a heuristic.  Replaces the 122-arm if-chain of kernel.cu:3022-3155;
@@ -178,8 +183,8 @@ size_t tuna_matmul_batched_workspace_bytes(int m, int n, int k, int batch);
  * weight-streaming GEMMs are meant to be issued when their inputs do not depend on each other
  * (QKV and gate+up of a layer, the experts of a mixture, a benchmark sweep); the reference has no
  * counterpart (its README sums single-GEMM times, README.md:25-27).  Shapes, layouts and results
- * as tuna_matmul; token counts up to 64 run in the sequence kernel (64 GEMMs per launch), a
- * sequence with a larger token count is issued GEMM by GEMM.  Every GEMM has its own token
+ * as tuna_matmul; token counts up to 64 run in the sequence kernel (64 GEMMs per launch), GEMMs
+ * with more tokens one by one after it.  Every GEMM has its own token
  * count n, so this is also the grouped GEMM of a mixture of experts with a per-expert token
  * list (the step the reference fakes with one combined GEMM over all experts,
  * make_configs.py:105-106): one entry per expert, x and o pointing at that expert's rows, n its

@@ -71,6 +71,7 @@ def test_batched_more_matrices_than_one_launch_and_small_workspaces(batch, m, n,
         assert _batched_abi(xd, qd, sd, cd, out, batch, m, n, k, ws) == 0
         torch.cuda.synchronize()
         assert lib.tuna_check_device_status(torch.cuda.current_stream().cuda_stream) == 0
+        assert int(ws[lib.tuna_workspace_scratch_bytes():].sum()) == 0
         o = out.cpu().numpy()
         for b in range(batch):
             check_parity(o[b], orc.matmul_ref(x[b], per[b][1], per[b][2], code, m, n, k), 1e-2)

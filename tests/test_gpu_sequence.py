@@ -77,6 +77,27 @@ def test_sequence_with_more_tokens_than_one_pass_falls_back_per_gemm():
     _check(shapes, cases, holders)
 
 
+def test_sequence_of_small_and_large_token_counts():
+    """The GEMMs of up to 64 tokens share a launch, wherever they stand; with a workspace that has no room for their
+    counters every GEMM is launched alone."""
+    shapes = [(1024, 5, 512), (512, 100, 512), (256, 64, 1024), (640, 300, 264), (1024, 1, 264)]
+    cases, gemms, holders, code = _build(shapes, seed0=17)
+    lib = _lib.load()
+    small = torch.zeros(max(lib.tuna_matmul_workspace_bytes(m, n, k) for m, n, k in shapes), dtype=torch.uint8, device="cuda")
+    descs = (_lib.TunaGemmDesc * len(gemms))(*[_lib.TunaGemmDesc(q.data_ptr(), x.data_ptr(), s.data_ptr(), o.data_ptr(), m, n, k, 0)
+                                              for x, q, s, o, m, n, k in gemms])
+    for ws in (None, small):
+        for h in holders:
+            h.view.fill_(float("nan"))
+        if ws is None:
+            tuna_b200.matmul_sequence(gemms, code)
+        else:
+            assert lib.tuna_matmul_sequence(descs, len(gemms), code.data_ptr(), ws.data_ptr(), ws.numel(), stream_ptr()) == 0
+        torch.cuda.synchronize()
+        assert lib.tuna_check_device_status(stream_ptr()) == 0
+        _check(shapes, cases, holders)
+
+
 def test_sequence_token_tiles_32_and_64():
     for n in (24, 48):
         shapes = [(640, n, 520), (1024, n - 7, 1024), (256, n, 2048)]

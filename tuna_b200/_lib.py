@@ -60,6 +60,7 @@ SYMBOLS = {
     "tuna_matmul_batched": (c_int, [c_void_p] * 5 + [c_int] * 4 + [c_size_t] * 4 + [c_void_p, c_size_t, c_void_p]),
     "tuna_matmul_batched_workspace_bytes": (c_size_t, [c_int] * 4),
     "tuna_matmul_noalloc": (c_int, [c_void_p] * 5 + [c_int] * 3 + [c_void_p]),
+    "tuna_workspace_scratch_bytes": (c_size_t, []),
     "tuna_matmul_sequence": (c_int, [ctypes.POINTER(TunaGemmDesc), c_int, c_void_p, c_void_p, c_size_t, c_void_p]),
     "tuna_matmul_sequence_workspace_bytes": (c_size_t, [ctypes.POINTER(TunaGemmDesc), c_int]),
     "tuna_matmul_sequence_reduce": (c_int, [ctypes.POINTER(TunaGemmDesc), c_int, c_void_p, c_void_p, c_size_t,

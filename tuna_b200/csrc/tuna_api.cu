@@ -4,6 +4,7 @@
 // compile-time if-chain and silently launches nothing for an unknown one; here
 // the table is data (generated from param_map.json), lookup happens at run
 // time and every failure is a status code.
+#include <algorithm>
 #include <cstring>
 #include <mutex>
 #include <vector>
@@ -249,7 +250,18 @@ extern "C" int tuna_matmul_sequence(const tuna_gemm_desc *g, int count, const vo
         return launch_gemm_tstream_sequence(live.data(), (int)live.size(), (const float *)code, workspace, workspace_bytes, sms,
                                             (cudaStream_t)stream);
     }
-    for (const tuna_gemm_desc &d : live) {
+    // GEMMs of more than 64 tokens are issued one by one; the others still share a launch, where the
+    // workspace has room for their counters (the larger GEMMs alone may need less).
+    const auto large = std::stable_partition(live.begin(), live.end(), [](const tuna_gemm_desc &d) { return d.n <= 64; });
+    int together = (int)(large - live.begin());
+    if (together < 2 || workspace == nullptr || workspace_bytes < gemm_tstream_sequence_min_workspace_bytes(live.data(), together, sms))
+        together = 0;
+    if (together > 0) {
+        st = launch_gemm_tstream_sequence(live.data(), together, (const float *)code, workspace, workspace_bytes, sms, (cudaStream_t)stream);
+        if (st != TUNA_OK) return st;
+    }
+    for (size_t i = (size_t)together; i < live.size(); ++i) {
+        const tuna_gemm_desc &d = live[i];
         st = tuna_matmul(d.q, d.x, code, d.absmax, d.o, d.m, d.n, d.k, workspace, workspace_bytes, stream);
         if (st != TUNA_OK) return st;
     }
@@ -297,6 +309,8 @@ extern "C" size_t tuna_matmul_workspace_bytes(int m, int n, int k)
     if (resolve_config(m, n, k, sms, nullptr, &c) != TUNA_OK) return 0;
     return workspace_for(m, n, k, c, sms);
 }
+
+extern "C" size_t tuna_workspace_scratch_bytes(void) { return partial_region_bytes(device_sm_count()); }
 
 extern "C" int tuna_lookup_config(int m, int n, int k, tuna_config *out)
 {
