@@ -8,7 +8,9 @@ a bad argument raises instead of corrupting memory.
 
 from __future__ import annotations
 
+import contextlib
 import ctypes
+import functools
 
 import torch
 
@@ -19,10 +21,14 @@ _workspaces: dict = {}
 
 
 def _stream_ptr(device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    index = device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
 
 def _expect(t: torch.Tensor, name: str, dtype, numel: int, device=None):
+    if (isinstance(t, torch.Tensor) and t.dtype is dtype and t.is_cuda and t.is_contiguous() and t.numel() == numel
+            and (device is None or t.device == device)):
+        return
     if not isinstance(t, torch.Tensor):
         raise TypeError(f"{name} must be a torch.Tensor")
     if not t.is_cuda:
@@ -33,8 +39,21 @@ def _expect(t: torch.Tensor, name: str, dtype, numel: int, device=None):
         raise TypeError(f"{name} must be {dtype}, got {t.dtype}")
     if not t.is_contiguous():
         raise ValueError(f"{name} must be contiguous")
-    if t.numel() != numel:
-        raise ValueError(f"{name} has {t.numel()} elements, expected {numel}")
+    raise ValueError(f"{name} has {t.numel()} elements, expected {numel}")
+
+
+_no_switch = contextlib.nullcontext()
+
+
+def _on_device(device):
+    """`torch.cuda.device(device)`, without its cost where `device` is current already."""
+    return _no_switch if device.index == torch.cuda.current_device() else torch.cuda.device(device)
+
+
+@functools.lru_cache(maxsize=4096)
+def _workspace_bytes(index, m, n, k) -> int:
+    with torch.cuda.device(index):
+        return int(_lib.load().tuna_matmul_workspace_bytes(m, n, k))
 
 
 def workspace_for(m: int, n: int, k: int, device) -> torch.Tensor:
@@ -43,10 +62,9 @@ def workspace_for(m: int, n: int, k: int, device) -> torch.Tensor:
     The kernels leave the workspace clean after every call, so one buffer serves
     consecutive calls on a stream; it only grows.
     """
-    lib = _lib.load()
-    with torch.cuda.device(device):
-        need = int(lib.tuna_matmul_workspace_bytes(m, n, k))
-    key = (torch.device(device).index, _stream_ptr(device))
+    device = torch.device(device)
+    need = _workspace_bytes(torch.cuda.current_device() if device.index is None else device.index, m, n, k)
+    key = (device.index, _stream_ptr(device))
     ws = _workspaces.get(key)
     if ws is None or ws.numel() < need:
         ws = torch.zeros(max(need, 1 << 20), dtype=torch.uint8, device=device)
@@ -83,7 +101,7 @@ def matmul(x, q, s, c, o, m: int, n: int, k: int, *, config: TunaConfig | None =
     _expect(c, "c", torch.float32, 16, dev)
     _expect(o, "o", torch.float16, n * m, dev)
     lib = _lib.load()
-    with torch.cuda.device(dev):
+    with _on_device(dev):
         ws = workspace if workspace is not None else workspace_for(m, n, k, dev)
         args = (q.data_ptr(), x.data_ptr(), c.data_ptr(), s.data_ptr(), o.data_ptr(), m, n, k,
                 ws.data_ptr(), ws.numel() * ws.element_size(), _stream_ptr(dev))
@@ -109,10 +127,10 @@ def matmul_batched(x, q, s, c, o, m: int, n: int, k: int, *, workspace=None) -> 
     shared = x.dim() == 2
     _expect(x, "x", torch.float16, n * k if shared else batch * n * k, dev)
     lib = _lib.load()
-    with torch.cuda.device(dev):
+    with _on_device(dev):
         need = int(lib.tuna_matmul_batched_workspace_bytes(m, n, k, batch))
         if workspace is None:
-            key = ("batched", dev.index, torch.cuda.current_stream(dev).cuda_stream)
+            key = ("batched", dev.index, _stream_ptr(dev))
             ws = _workspaces.get(key)
             if ws is None or ws.numel() < need:
                 ws = torch.zeros(max(need, 1 << 20), dtype=torch.uint8, device=dev)
@@ -165,7 +183,7 @@ class MatmulSequence:
         self.workspace = workspace
 
     def run(self) -> None:
-        with torch.cuda.device(self.device):
+        with _on_device(self.device):
             check(_lib.load().tuna_matmul_sequence(self._descs, self.count, self.code.data_ptr(), self.workspace.data_ptr(),
                                                    self.workspace.numel() * self.workspace.element_size(), _stream_ptr(self.device)))
 
@@ -428,7 +446,7 @@ def dequant(q, absmax, codebook, o, m: int, k: int) -> None:
     _expect(absmax, "absmax", torch.float32, m, dev)
     _expect(codebook, "codebook", torch.float32, 16, dev)
     _expect(o, "o", torch.float16, m * k, dev)
-    with torch.cuda.device(dev):
+    with _on_device(dev):
         check(_lib.load().tuna_dequant(q.data_ptr(), absmax.data_ptr(), codebook.data_ptr(), o.data_ptr(),
                                        m, k, _stream_ptr(dev)))
 
@@ -448,7 +466,7 @@ def quantize(w, codebook=None):
     q = torch.empty((m // 8, k // 8, 32), dtype=torch.uint8, device=w.device)
     absmax = torch.empty((m,), dtype=torch.float32, device=w.device)
     code = torch.empty((16,), dtype=torch.float32, device=w.device) if codebook is None else codebook
-    with torch.cuda.device(w.device):
+    with _on_device(w.device):
         if codebook is None:  # the kernel knows the NF4 levels: no upload, no synchronisation
             check(_lib.load().tuna_quantize_nf4(w.data_ptr(), q.data_ptr(), absmax.data_ptr(), code.data_ptr(), m, k,
                                                 _stream_ptr(w.device)))
