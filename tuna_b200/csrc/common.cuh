@@ -71,4 +71,34 @@ struct DeviceStatus {
     int detail;
 };
 
+// A table of 16 fp16 values in registers, as byte planes for prmt: the low and high bytes of
+// entries 4i .. 4i + 3 in lo[i] / hi[i].
+struct CodePlanes {
+    uint32_t lo[4], hi[4];
+    // from eight words of two fp16 entries each
+    __device__ __forceinline__ void init(const uint32_t (&e)[8])
+    {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            lo[i] = __byte_perm(e[2 * i], e[2 * i + 1], 0x6420);
+            hi[i] = __byte_perm(e[2 * i], e[2 * i + 1], 0x7531);
+        }
+    }
+    // The eight weights of one row of a packed tile -> four half2 (byte b: high nibble first).  Per four
+    // nibbles and plane: one of entries 0-7 and one of 8-15 by the nibbles' low three bits, then the
+    // right one of the two by their top bits.  21 instructions, no memory access.
+    __device__ __forceinline__ void convert(uint32_t w, uint32_t *o) const
+    {
+        const uint32_t s = w & 0x77777777u, t = ((w >> 1) & 0x44444444u) | 0x32103210u;
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            const uint32_t sh = s >> (16 * half), th = t >> (16 * half);
+            const uint32_t l = __byte_perm(__byte_perm(lo[0], lo[1], sh), __byte_perm(lo[2], lo[3], sh), th);
+            const uint32_t h = __byte_perm(__byte_perm(hi[0], hi[1], sh), __byte_perm(hi[2], hi[3], sh), th);
+            o[2 * half] = __byte_perm(l, h, 0x4051);
+            o[2 * half + 1] = __byte_perm(l, h, 0x6273);
+        }
+    }
+};
+
 }  // namespace tuna

@@ -4,63 +4,86 @@
 // bit-exact to it: out = (half)(code[nibble] * absmax[row]) with the multiply
 // in fp32 (kernel.cu:3223-3228).  HBM-bound: reads m*k/2 bytes, writes 2*m*k.
 //
-// Mapping: one warp owns one 8-row group and walks along K.  A lane reads 16
-// packed bytes (half of an 8x8 tile: 4 rows x 8 columns) with one 128-bit
-// load, looks every nibble up in a per-row 16-entry fp16 table held in shared
-// memory (built once per warp with the fp32 multiply), and writes four 16-byte
-// row segments.  Across a warp each of those stores covers 256 contiguous
-// bytes per row.
+// Mapping: one warp owns one 8-row group and walks along K.  A lane reads 16 packed bytes (half of
+// an 8x8 tile: 4 rows x 8 columns) with one 128-bit load, turns each row's word into fp16 with the
+// row's table in registers (CodePlanes; the tables are built once per warp with the fp32 multiply)
+// and writes four 16-byte row segments.  Across a warp each of those stores covers 256 contiguous
+// bytes of two rows.
+// Writes bound it: filling the output alone (torch's fill kernel) takes 64 us at 28672x4096, a copy of as many
+// bytes in all 47.  28672x4096: 58.9 -> 49.5 us (5.93 TB/s) against lookups in a per-row table in shared memory, one
+// load in flight.
+#include <algorithm>
 #include "common.cuh"
 #include "launchers.h"
 
 namespace tuna {
 
 constexpr int kDqWarps = 8;
+constexpr int kDqUnroll = 2;     // loads in flight per lane
+constexpr int kDqCtasPerSm = 3;  // 80 registers: four tables of 8 and two passes of data
+constexpr int kDqWaves = 6;      // 28672x4096: 56.5 us with one wave of longer-lived warps, 53.4 with 4, 49.5 with 6, 49.3 with 8
 
-__global__ void __launch_bounds__(kDqWarps * 32)
+__global__ void __launch_bounds__(kDqWarps * 32, kDqCtasPerSm)
 dequant_w4_kernel(const uint8_t *__restrict__ q, const float *__restrict__ absmax,
-                  const float *__restrict__ code, __half *__restrict__ out, int m, int k,
-                  int tiles_per_split)
+                  const float *__restrict__ code, __half *__restrict__ out, int k, int per_warp, int extra)
 {
     __shared__ __align__(16) __half lut[kDqWarps][8][kCodeSize];
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int rg = blockIdx.x * kDqWarps + warp;  // 8-row group
-    const int n_rg = m >> 3, n_kt = k >> 3;
-    if (rg < n_rg) {
-        // 128 table entries per warp, 4 per lane: row = e / 16, nibble = e % 16
-        for (int e = lane; e < 8 * kCodeSize; e += 32) {
-            float v = code[e & 15] * absmax[rg * 8 + (e >> 4)];
-            lut[warp][e >> 4][e & 15] = __float2half_rn(v);
-        }
-    }
-    __syncwarp();
-    if (rg >= n_rg) return;
-
-    const int kt_begin = blockIdx.y * tiles_per_split;
-    const int kt_end = min(n_kt, kt_begin + tiles_per_split);
+    const int n_kt = k >> 3;
     const int half_sel = lane & 1;  // which 4 rows of the tile this lane holds
-    const uint8_t *src_rg = q + (size_t)rg * row_group_bytes(k);
-    const __half *my_lut = &lut[warp][half_sel * 4][0];
-    __half *dst_rows = out + (size_t)(rg * 8 + half_sel * 4) * k;
+    constexpr int kPassTiles = 16 * kDqUnroll;
+    const int passes = (n_kt + kPassTiles - 1) / kPassTiles;  // of a row group
+    // this warp's contiguous range of (row group, pass)
+    const int w = blockIdx.x * kDqWarps + warp;
+    int it = w * per_warp + min(w, extra);
+    const int it_end = it + per_warp + (w < extra ? 1 : 0);
 
-    for (int kt = kt_begin + (lane >> 1); kt < kt_end; kt += 16) {
-        uint4 v = ldg_stream_u4(src_rg + (size_t)kt * 32 + half_sel * 16);
-        const uint32_t words[4] = {v.x, v.y, v.z, v.w};
+    while (it < it_end) {
+        const int rg = it / passes, p0 = it - rg * passes;
+        const int n_pass = min(passes - p0, it_end - it);
+        it += n_pass;
+        const int kt_end = min(n_kt, (p0 + n_pass) * kPassTiles);
+        const uint8_t *src = q + (size_t)rg * row_group_bytes(k) + half_sel * 16;
+        __half *dst_rows = out + (size_t)(rg * 8 + half_sel * 4) * k;
+        int kt = p0 * kPassTiles + (lane >> 1);
+        uint4 v[kDqUnroll];
+        auto load = [&](int kt0) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {  // row 4*half_sel + i, columns 8kt .. 8kt+7
-            const uint32_t w = words[i];
-            const __half *l = my_lut + i * kCodeSize;
-            uint32_t o[4];
+            for (int u = 0; u < kDqUnroll; ++u) v[u] = ldg_stream_pred(src + (size_t)(kt0 + 16 * u) * 32, kt0 + 16 * u < kt_end);
+        };
+        load(kt);  // in flight while the tables are built
+
+        // 128 table entries per warp, 4 per lane: row = e / 16, nibble = e % 16
+        __syncwarp();  // the previous row group's tables have been read
+        for (int e = lane; e < 8 * kCodeSize; e += 32)
+            lut[warp][e >> 4][e & 15] = __float2half_rn(code[e & 15] * absmax[rg * 8 + (e >> 4)]);
+        __syncwarp();
+        CodePlanes row[4];
 #pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                const uint32_t byte = (w >> (8 * b)) & 0xffu;
-                const __half hi = l[byte >> 4];  // even column: high nibble
-                const __half lo = l[byte & 15];
-                o[b] = (uint32_t)__half_as_ushort(hi) | ((uint32_t)__half_as_ushort(lo) << 16);
+        for (int i = 0; i < 4; ++i) {
+            const uint4 *t = reinterpret_cast<const uint4 *>(&lut[warp][half_sel * 4 + i][0]);
+            const uint4 a = t[0], b = t[1];
+            const uint32_t e[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+            row[i].init(e);
+        }
+
+        for (; kt < kt_end; kt += kPassTiles) {
+            uint4 c[kDqUnroll];
+#pragma unroll
+            for (int u = 0; u < kDqUnroll; ++u) c[u] = v[u];
+            load(kt + kPassTiles);
+#pragma unroll
+            for (int u = 0; u < kDqUnroll; ++u) {
+                if (kt + 16 * u >= kt_end) break;
+                const uint32_t words[4] = {c[u].x, c[u].y, c[u].z, c[u].w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {  // row 4*half_sel + i, columns 8kt .. 8kt+7
+                    uint32_t o[4];
+                    row[i].convert(words[i], o);
+                    *reinterpret_cast<uint4 *>(dst_rows + (size_t)i * k + (size_t)(kt + 16 * u) * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+                }
             }
-            *reinterpret_cast<uint4 *>(dst_rows + (size_t)i * k + (size_t)kt * 8) =
-                make_uint4(o[0], o[1], o[2], o[3]);
         }
     }
 }
@@ -68,17 +91,11 @@ dequant_w4_kernel(const uint8_t *__restrict__ q, const float *__restrict__ absma
 cudaError_t launch_dequant(const void *q, const void *absmax, const void *code, void *o, int m,
                            int k, int sm_count, cudaStream_t stream)
 {
-    const int n_rg = m / 8, n_kt = k / 8;
-    const int gx = div_up(n_rg, kDqWarps);
-    // enough CTAs to fill the machine a few times over, at least 16 tiles (one warp pass) each
-    int want_y = div_up(sm_count * 8, gx);
-    int max_y = div_up(n_kt, 16);
-    int gy = max(1, min(want_y, max_y));
-    int tiles_per_split = div_up(div_up(n_kt, gy), 16) * 16;
-    gy = div_up(n_kt, tiles_per_split);
-    dequant_w4_kernel<<<dim3(gx, gy), kDqWarps * 32, 0, stream>>>(
-        (const uint8_t *)q, (const float *)absmax, (const float *)code, (__half *)o, m, k,
-        tiles_per_split);
+    const int items = (m / 8) * div_up(k / 8, 16 * kDqUnroll);  // below 2^31: m * k <= 2^41
+    const int grid = std::min(sm_count * kDqCtasPerSm * kDqWaves, div_up(items, kDqWarps));
+    const int warps = grid * kDqWarps;
+    dequant_w4_kernel<<<grid, kDqWarps * 32, 0, stream>>>((const uint8_t *)q, (const float *)absmax, (const float *)code, (__half *)o, k,
+                                                          items / warps, items % warps);
     return cudaGetLastError();
 }
 
