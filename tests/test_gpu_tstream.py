@@ -133,3 +133,10 @@ def test_tstream_benchmark_shapes_m16(m, k):
     got = out.cpu().numpy().reshape(n, m // 8, 8)[:, rows].reshape(n, -1)
     check_parity(got, ref, TOL)
     assert holder.guards_intact()
+
+
+@pytest.mark.parametrize("ctas", [3, 18, 148])  # 1-2, 9 and 16 segments per tile
+@pytest.mark.parametrize("n", [1, 4, 5, 8, 9, 16, 17, 33, 43, 64])
+def test_tstream_cut_tiles_at_every_token_group(n, ctas):
+    """Tiles cut across CTAs exchange only the four-token groups that exist."""
+    _run(256, n, 4096, seed=n, row_blocks=1, k_steps=8, ctas=ctas)

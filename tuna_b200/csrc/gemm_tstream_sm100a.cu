@@ -51,15 +51,18 @@
 //
 // Work decomposition ("stream-K"): a unit is (tile of 128*row_blocks rows, 128- or 256-column chunk) =
 // row_blocks slots; the units, tile-major, are cut into one contiguous range per CTA so that
-// every SM streams the same number of bytes whatever the shape.  A tile cut across CTAs is
-// finished by whichever CTA arrives last at the tile's counter (per 32-row quarter): it adds
-// the fp32 partials from the workspace in range order, so the result does not depend on
-// arrival order (the reference adds fp16 partials with atomicAdd, kernel.cu:2739-2745).  No
-// floating-point atomics, no zero-filled output.
+// every SM streams the same number of bytes whatever the shape.  A tile cut across CTAs is finished by whichever CTA arrives last at
+// the tile's counter (per 32-row quarter): it adds the fp32 partials from the workspace in range order, so the
+// result does not depend on arrival order (the reference adds fp16 partials with atomicAdd, kernel.cu:2739-2745).  No
+// floating-point atomics, no zero-filled output.  This tail is what a single small GEMM waits for: at 28672x4096 and 16
+// tokens the last MMA was done at 16.7 us of 24.1.  Hence only token groups that exist are exchanged, one
+// acquire-release atomic per warp replaces two fences, and at the end of the range all 24 warps add up the tile, four
+// tokens of 32 rows each, instead of four warps 16 tokens at a time (graph replay, 16 tokens unless said, us):
+// 4096x4096 10.3 -> 9.9, 57344x8192 67.0 -> 65.2, 4096x4096 at 64 tokens 20.1 -> 14.2, 768x4096 at 64 49.7 -> 12.9.
 //
-// Programmatic dependent launch: the kernel lets its successor start as SMs free up and itself
-// waits for its predecessors only before it touches what they may have written (activations,
-// workspace, output); the weights and the codebook are constants and are requested before.
+// Programmatic dependent launch: the kernel lets its successor start as SMs free up and itself waits for its predecessors
+// only before it touches what they may have written (activations, workspace, output); the weights and the
+// codebook are constants, requested before, and dequantised into the A-slot ring meanwhile.
 //
 // Every wait is bounded: when one runs out the CTA records where in the device status word,
 // raises a CTA-wide abort flag and unwinds to the common exit, where tensor memory is released.
@@ -183,6 +186,9 @@ __device__ __forceinline__ uint32_t ts_lookup256(uint32_t w, uint32_t key, uint3
     return v;
 }
 
+template <int V>
+struct Int { static constexpr int value = V; };
+
 // The CTA whose range holds unit u.
 __device__ __forceinline__ int ts_cta_of_unit(const TsParams &p, int u)
 {
@@ -261,6 +267,8 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_w4a16_tstream_kernel(const
     __shared__ __align__(8) uint64_t bars[2 * kTsMaxASlots + 2 * kTsMaxXStages + 4 + 2 * kTsMaxWStages];
     __shared__ uint32_t s_tmem_base;
     __shared__ int s_abort;
+    __shared__ int s_fix[4];   // quarters of the CTA's last tile that this CTA finishes
+    __shared__ int s_last[4];  // its GEMM, tile, first CTA and segments
 
     TS_PROF_DECL
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
@@ -308,6 +316,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_w4a16_tstream_kernel(const
 
     if (threadIdx.x == 0) {
         s_abort = 0;
+        s_fix[0] = s_fix[1] = s_fix[2] = s_fix[3] = 0;
         for (int i = 0; i < kTsMaxASlots; ++i) { mbar_init(a_full + 8 * i, 4 * kHalves); mbar_init(a_empty + 8 * i, 1); }
         for (int i = 0; i < kTsMaxXStages; ++i) { mbar_init(x_full + 8 * i, 1); mbar_init(x_empty + 8 * i, 1); }
         for (int i = 0; i < 2; ++i) { mbar_init(d_full + 8 * i, 1); mbar_init(d_empty + 8 * i, 4); }
@@ -327,8 +336,10 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_w4a16_tstream_kernel(const
 
     // Rest of the prologue, run by every warp inside its own role's branch: the byte -> half2
     // table (even column = high nibble in the low half), one copy per bank - the codebook is a
-    // constant, so this runs before the dependency wait - then the wait, then the CTA barrier
-    // that publishes the table and the tensor-memory base.
+    // constant, so this needs no dependency wait - then the CTA barrier that publishes the table and the
+    // tensor-memory base.  Only what reads or writes data of the kernels before this one waits for
+    // them (depend(): the copies of x, the epilogue, and before their bounded waits the MMA warp and
+    // whoever has filled its ring), so the dequant warps fill the A-slot ring meanwhile.
     auto finish_prologue = [&]() -> uint32_t {
         const float cv = p.code[lane & 15];
         const uint32_t ch = (uint32_t)__half_as_ushort(__float2half_rn(cv));
@@ -336,13 +347,92 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_w4a16_tstream_kernel(const
             const uint32_t v = __shfl_sync(0xffffffffu, ch, e >> 4) | (__shfl_sync(0xffffffffu, ch, e & 15) << 16);
             asm volatile("st.shared.u32 [%0], %1;" ::"r"(lut_addr + (uint32_t)e * (kLut256 ? 256 : 128) + lane * 4), "r"(v) : "memory");
         }
-        asm volatile("griddepcontrol.wait;" ::: "memory");
         tc_fence_before();
         __syncthreads();
         tc_fence_after();
         TS_PROF_MARK(1)
         return s_tmem_base;
     };
+    auto depend = [] { asm volatile("griddepcontrol.wait;" ::: "memory"); };
+
+    const size_t slot_floats = (size_t)RB * kBlockRows * N_TILE;
+    // the row of a block that lane `lane` of quarter q holds
+    auto row_in_block = [&](int q) { return WMODE == 1 ? 32 * q + lane : 8 * lane_row_group(q, lane) + (lane & 7); };
+    // groups of four tokens of the tile that exist (an exchange slab takes the whole tile)
+    auto token_groups = [&](const TsGemm &G) { return p.n_peers > 0 ? N_TILE / 4 : (min(G.n - p.tok0, N_TILE) + 3) >> 2; };
+    // NT tokens from token `t0` of the tile on of one finished row, scaled: to o, or (16 tokens) to every rank's slab
+    auto store_row = [&](const TsGemm &G, int row, int t0, const auto &v, float sc) __attribute__((always_inline)) {
+        constexpr int NT = sizeof(v) / sizeof(float);
+        if (NT == 16 && p.n_peers > 0 && G.slab_off >= 0) {
+            uint32_t h[NT / 2];
+#pragma unroll
+            for (int i = 0; i < NT / 2; ++i) {
+                const __half2 t = __floats2half2_rn(v[2 * i] * sc, v[2 * i + 1] * sc);
+                h[i] = *reinterpret_cast<const uint32_t *>(&t);
+            }
+            // where this launch's slabs start: every caller is past the dependency wait
+            const long long region = p.region0 + (long long)((__ldcg(p.epoch) + 1u) & 1u) * p.region_bytes;
+            const long long off = region + G.slab_off + ((long long)row * N_TILE + t0) * 2;
+            for (int pr = 0; pr < p.n_peers; ++pr) {
+                uint4 *dst = reinterpret_cast<uint4 *>(p.peer[pr] + off);
+#pragma unroll
+                for (int i = 0; i < NT / 8; ++i) dst[i] = make_uint4(h[4 * i], h[4 * i + 1], h[4 * i + 2], h[4 * i + 3]);
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < NT; ++i) {
+                const int tok = p.tok0 + t0 + i;
+                if (tok < G.n) G.o[(size_t)tok * G.m + row] = __float2half_rn(v[i] * sc);
+            }
+        }
+    };
+    // Adds the partials of GR four-token groups from group g0 on of 32 rows (block rb, quarter q of the tile) over its
+    // segments, which CTAs `first` .. first + nseg - 1 wrote, and stores the rows.  The loads of SG segments are
+    // in flight at a time, the adds keep the range order.
+    auto add_partials = [&](auto gr, auto sg, const TsGemm &G, int tile, int first, int nseg, int q, int rb, int g0) __attribute__((always_inline)) {
+        constexpr int GR = decltype(gr)::value, SG = decltype(sg)::value;
+        const int row = (tile * RB + rb) * kBlockRows + row_in_block(q);
+        if (row >= G.m) return;
+        const float sc = G.absmax[row];
+        float acc[4 * GR];
+#pragma unroll
+        for (int i = 0; i < 4 * GR; ++i) acc[i] = 0.f;
+#pragma unroll 1
+        for (int sgm = 0; sgm < nseg; sgm += SG) {
+            float4 a[SG][GR];
+#pragma unroll
+            for (int j = 0; j < SG; ++j) {
+                const int seg = min(sgm + j, nseg - 1);
+                const float4 *src = reinterpret_cast<const float4 *>(p.partials + (size_t)(2 * (first + seg) + (seg == 0 ? 1 : 0)) * slot_floats) +
+                                    ((size_t)rb * (N_TILE / 4) + g0) * kBlockRows + 32 * q + lane;
+#pragma unroll
+                for (int i = 0; i < GR; ++i) a[j][i] = __ldcg(src + i * kBlockRows);
+            }
+#pragma unroll
+            for (int j = 0; j < SG; ++j) {
+                const bool live = sgm + j < nseg;
+#pragma unroll
+                for (int i = 0; i < GR; ++i)
+                    if (live) { acc[4 * i] += a[j][i].x; acc[4 * i + 1] += a[j][i].y; acc[4 * i + 2] += a[j][i].z; acc[4 * i + 3] += a[j][i].w; }
+            }
+        }
+        store_row(G, row, 4 * g0, acc, sc);
+    };
+    // The flagged quarters of a tile whose partials are all there, shared out over warps `w0`, w0 + step, ... : a warp
+    // takes four tokens of 32 rows at a time (small code: it runs once per CTA, out of a cold instruction cache),
+    // in exchange launches 16, whole sectors of a peer's slab.
+    auto finish_tile = [&](const TsGemm &G, int tile, int first, int nseg, int w0, int step, auto flagged) __attribute__((always_inline)) {
+        const int groups4 = token_groups(G), per = p.n_peers > 0 ? 4 : 1, rb_shift = RB >> 1;
+        for (int item = w0; item * per < 4 * RB * groups4; item += step) {
+            const int q = item & 3, rest = item >> 2;
+            const int g = rest >> rb_shift, rb = rest & (RB - 1);  // RB is 1, 2 or 4
+            if (!flagged(q)) continue;
+            if (per == 1) add_partials(Int<1>(), Int<4>(), G, tile, first, nseg, q, rb, g);
+            else add_partials(Int<4>(), Int<2>(), G, tile, first, nseg, q, rb, 4 * g);
+        }
+    };
+    auto first_cta = [&](const TsGemm &G, int tile) { return ts_cta_of_unit(p, G.unit0 + tile * G.chunks); };
+    auto last_cta = [&](const TsGemm &G, int tile) { return ts_cta_of_unit(p, G.unit0 + (tile + 1) * G.chunks - 1); };
     uint32_t tmem = 0;
 
     if (warp == 0) {
@@ -352,6 +442,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_w4a16_tstream_kernel(const
         // is constant (8-token groups 1024 bytes apart, version 1, layout type 2), the low word is the
         // start address; 16 columns further along K is 32 bytes further inside the 128-byte row.
         tmem = finish_prologue();
+        depend();
         constexpr uint32_t idesc = make_idesc(N_TILE);
         constexpr uint32_t desc_hi = (1024u >> 4) | (1u << 14) | (2u << 29);
         Ring ra, rx, rd;
@@ -469,41 +560,13 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_w4a16_tstream_kernel(const
         };
         issue_w_until(min(WS, total_slots), false);
         tmem = finish_prologue();
+        depend();
         issue_w_until(total_slots, true);
         issue_x(true);
     } else if (warp < kTsDequantWarp0) {
         // ------------------------------------------------------------------ epilogue
         tmem = finish_prologue();
-        // the row this thread's lane holds
-        const int row_in_block = WMODE == 1 ? 32 * quarter + lane : 8 * lane_row_group(quarter, lane) + (lane & 7);
-        const int tmem_lane = 32 * quarter + lane;
-        const size_t slot_floats = (size_t)RB * kBlockRows * N_TILE;
-        // exchange launches: where this launch's slabs start (the counter is read after the dependency wait)
-        long long region = 0;
-        if (p.n_peers > 0) region = p.region0 + (long long)((__ldcg(p.epoch) + 1u) & 1u) * p.region_bytes;
-        // 16 tokens (one accumulator piece) of one finished row, scaled: to o, or to every rank's slab
-        auto store_row = [&](const TsGemm &G, int row, int piece, const float (&v)[16], float sc) {
-            if (p.n_peers > 0 && G.slab_off >= 0) {
-                uint32_t h[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const __half2 t = __floats2half2_rn(v[2 * i] * sc, v[2 * i + 1] * sc);
-                    h[i] = *reinterpret_cast<const uint32_t *>(&t);
-                }
-                const long long off = region + G.slab_off + ((long long)row * N_TILE + piece * 16) * 2;
-                for (int pr = 0; pr < p.n_peers; ++pr) {
-                    uint4 *dst = reinterpret_cast<uint4 *>(p.peer[pr] + off);
-                    dst[0] = make_uint4(h[0], h[1], h[2], h[3]);
-                    dst[1] = make_uint4(h[4], h[5], h[6], h[7]);
-                }
-            } else {
-#pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    const int tok = p.tok0 + piece * 16 + i;
-                    if (tok < G.n) G.o[(size_t)tok * G.m + row] = __float2half_rn(v[i] * sc);
-                }
-            }
-        };
+        depend();
         Ring rd;
         TsCursor cur;
         cur.init(L, u_begin, n_units);
@@ -519,21 +582,23 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_w4a16_tstream_kernel(const
             TS_PROF_END(0)
             tc_fence_after();
             TS_PROF_BEGIN
+            const int groups4 = token_groups(G);
             float *my_partial = p.partials + (size_t)(2 * cta + (c0 == 0 ? 1 : 0)) * slot_floats;
             for (int rb = 0; rb < RB; ++rb) {
-                const int row = (tile * RB + rb) * kBlockRows + row_in_block;
+                const int row = (tile * RB + rb) * kBlockRows + row_in_block(quarter);
                 const float sc = (full && row < G.m) ? G.absmax[row] : 0.f;
 #pragma unroll 1
-                for (int piece = 0; piece < N_TILE / 16; ++piece) {
+                for (int piece = 0; 4 * piece < groups4; ++piece) {
                     float v[16];
                     tc_ld_x16(tmem + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(rd.idx * p.acc_cols) + (uint32_t)rb * N_TILE + piece * 16, v);
                     if (full) {
-                        if (row < G.m) store_row(G, row, piece, v, sc);
+                        if (row < G.m) store_row(G, row, 16 * piece, v, sc);
                     } else {
                         // [rb][4-token group][128 lanes] float4: a warp store is 512 contiguous bytes
-                        float4 *dst = reinterpret_cast<float4 *>(my_partial) + ((size_t)rb * (N_TILE / 4) + piece * 4) * kBlockRows + tmem_lane;
+                        float4 *dst = reinterpret_cast<float4 *>(my_partial) + ((size_t)rb * (N_TILE / 4) + piece * 4) * kBlockRows + 32 * quarter + lane;
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) dst[i * kBlockRows] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+                        for (int i = 0; i < 4; ++i)
+                            if (4 * piece + i < groups4) dst[i * kBlockRows] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
                     }
                 }
             }
@@ -541,56 +606,23 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_w4a16_tstream_kernel(const
             __syncwarp();
             if (lane == 0) mbar_arrive(d_empty + 8 * rd.idx);
             if (!full) {
-                // Each epilogue warp finishes its own 32 lanes of the tile alone: it arrives at the
-                // counter of (tile, quarter); the last warp to arrive adds that quarter's partials in
-                // range order and stores the rows.
-                __threadfence();
+                // Each epilogue warp arrives for its own 32 lanes at the counter of (tile, quarter).  Whoever arrives
+                // last has all the partials: in the middle of the range the warp adds them up itself, at its end - where
+                // nearly all the cut tiles are finished, and nothing else is left to do - all warps of the CTA do.
+                // lane 0's atomic releases the warp's partials and acquires the others'
                 __syncwarp();
-                const int cta_first = ts_cta_of_unit(p, G.unit0 + tile * G.chunks);
-                const int cta_last = ts_cta_of_unit(p, G.unit0 + (tile + 1) * G.chunks - 1);
-                const int nseg = cta_last - cta_first + 1;
+                const int first = first_cta(G, tile), nseg = last_cta(G, tile) - first + 1;
                 unsigned int *counter = p.counters + (size_t)(G.tile0 + tile) * 4 + quarter;
                 unsigned int old = 0;
-                if (lane == 0) old = atomicAdd(counter, 1u);
+                if (lane == 0) asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(old) : "l"(counter) : "memory");
                 old = __shfl_sync(0xffffffffu, old, 0);
                 if (old == (unsigned)nseg - 1) {
                     if (lane == 0) *counter = 0;  // leave the counter clean for the next call
-                    __threadfence();
-                    for (int rb = 0; rb < RB; ++rb) {
-                        const int row = (tile * RB + rb) * kBlockRows + row_in_block;
-                        if (row >= G.m) continue;
-                        const float sc = G.absmax[row];
-#pragma unroll 1
-                        for (int piece = 0; piece < N_TILE / 16; ++piece) {
-                            float acc[16];
-#pragma unroll
-                            for (int i = 0; i < 16; ++i) acc[i] = 0.f;
-                            auto seg_ptr = [&](int sgm) {
-                                return reinterpret_cast<const float4 *>(p.partials + (size_t)(2 * (cta_first + sgm) + (sgm == 0 ? 1 : 0)) * slot_floats) +
-                                       ((size_t)rb * (N_TILE / 4) + piece * 4) * kBlockRows + tmem_lane;
-                            };
-                            // the loads of two segments in flight; the adds keep the range order
-                            int sgm = 0;
-                            for (; sgm + 2 <= nseg; sgm += 2) {
-                                float4 a[4], b[4];
-                                const float4 *s0 = seg_ptr(sgm), *s1 = seg_ptr(sgm + 1);
-#pragma unroll
-                                for (int i = 0; i < 4; ++i) { a[i] = __ldcg(s0 + i * kBlockRows); b[i] = __ldcg(s1 + i * kBlockRows); }
-#pragma unroll
-                                for (int i = 0; i < 4; ++i) { acc[4 * i] += a[i].x; acc[4 * i + 1] += a[i].y; acc[4 * i + 2] += a[i].z; acc[4 * i + 3] += a[i].w; }
-#pragma unroll
-                                for (int i = 0; i < 4; ++i) { acc[4 * i] += b[i].x; acc[4 * i + 1] += b[i].y; acc[4 * i + 2] += b[i].z; acc[4 * i + 3] += b[i].w; }
-                            }
-                            if (sgm < nseg) {
-                                const float4 *s0 = seg_ptr(sgm);
-#pragma unroll
-                                for (int i = 0; i < 4; ++i) {
-                                    const float4 a = __ldcg(s0 + i * kBlockRows);
-                                    acc[4 * i] += a.x; acc[4 * i + 1] += a.y; acc[4 * i + 2] += a.z; acc[4 * i + 3] += a.w;
-                                }
-                            }
-                            store_row(G, row, piece, acc, sc);
-                        }
+                    if (u + (c1 - c0) < n_units) finish_tile(G, tile, first, nseg, quarter, 4, [](int) { return true; });
+                    else if (lane == 0) {
+                        s_fix[quarter] = 1;
+                        // the same values from every flagged quarter
+                        s_last[0] = cur.g; s_last[1] = tile; s_last[2] = first; s_last[3] = nseg;
                     }
                 }
             }
@@ -680,6 +712,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_w4a16_tstream_kernel(const
             // producer.  The arrival is a release: it is ordered after this warp's loads.
             __syncwarp();
             if (lane == 0) mbar_arrive(w_empty + 8 * w_idx);
+            if (sl >= A && sl < A + kGroups) depend();  // the first slots whose A-slot has to be emptied first
             TS_PROF_BEGIN
             ok = mbar_wait_warp(a_empty + 8 * a_idx, a_phase ^ 1, abort_flag, p.status, 7);
             TS_PROF_END(0)
@@ -718,6 +751,9 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_w4a16_tstream_kernel(const
     TS_PROF_MARK(2)
     tc_fence_before();
     __syncthreads();
+    if (s_fix[0] | s_fix[1] | s_fix[2] | s_fix[3]) {
+        finish_tile(L.g[s_last[0]], s_last[1], s_last[2], s_last[3], warp, kTsThreads / 32, [&](int q) { return s_fix[q] != 0; });
+    }
     if (warp < kTsDequantWarp0) { TS_PROF_MARK(3) }
     TS_PROF_STORE
     if (warp == 0) {
