@@ -233,12 +233,15 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
             const uint32_t v = __shfl_sync(0xffffffffu, ch, e >> 4) | (__shfl_sync(0xffffffffu, ch, e & 15) << 16);
             asm volatile("st.shared.u32 [%0], %1;" ::"r"(lut_addr + (uint32_t)e * 128 + lane * 4), "r"(v) : "memory");
         }
-        asm volatile("griddepcontrol.wait;" ::: "memory");
         tc_fence_before();
         cluster_sync_all();
         tc_fence_after();
         return s_tmem_base;
     };
+    // Only what reads or writes data of the kernels before this one waits for them (the copies of x, the
+    // epilogue), and whoever is about to make a bounded wait that ends only after that; the weights
+    // are constants, so the dequant warps fill the A slots meanwhile.
+    auto depend = [] { asm volatile("griddepcontrol.wait;" ::: "memory"); };
     uint32_t tmem = 0;
     const uint32_t d_cols = (uint32_t)N;
     const uint32_t a_off = (uint32_t)p.nd * d_cols;  // first A slot
@@ -292,6 +295,7 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
 
     if (warp == 0) {
         tmem = finish_prologue();
+        depend();
         if (rank == 0) {
             // -------------------------------------------------------------- MMA issue
             // The warp stays converged: every lane runs the loop and the waits, one elected lane issues.
@@ -336,7 +340,7 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
     } else if (warp == 1) {
         // ------------------------------------------------------------------ weight producer
         // One elected lane of the converged warp issues the copies.  The weights are constants: the first
-        // ring-full is requested before the dependency wait.
+        // ones are requested before the dependency wait.
         Ring rw;
         int u = 0;
         bool ok = segs.next(p);
@@ -375,10 +379,13 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
         };
         issue_until(min(SW, total));
         tmem = finish_prologue();
+        issue_until(min(SW + S, total));  // the stages the dequant warps empty before the first MMA
+        depend();
         issue_until(total);
     } else if (warp == 2) {
         // ------------------------------------------------------------------ activation producer
         tmem = finish_prologue();
+        depend();
         Ring ru;
         const uint32_t full = rank == 0 ? u_full : x_full;
         bool ok = true;
@@ -405,6 +412,7 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
     } else if (warp < kPairDequantWarp0) {
         // ------------------------------------------------------------------ epilogue
         tmem = finish_prologue();
+        depend();
         const int quarter = warp & 3;
         const uint32_t tmem_q = tmem + ((uint32_t)(32 * quarter) << 16);
         Ring rd;
@@ -471,7 +479,6 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
                     for (int i = 0; i < 4; ++i) dst[(size_t)(t0 / 4 + i) * kBlockRows] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
                 }
                 tc_fence_before();
-                __threadfence();
                 __syncwarp();
                 if (lane == 0) mbar_arrive_cluster(leader_d_empty + 8 * rd.idx);
                 auto pair_of = [&](int unit) {
@@ -481,11 +488,11 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
                 const int nseg = pair_of((segs.tile + 1) * p.chunks - 1) - pair_of(segs.tile * p.chunks) + 1;
                 unsigned int *counter = p.counters + (size_t)(2 * segs.tile + rank) * 4 + quarter;
                 unsigned int old = 0;
-                if (lane == 0) old = atomicAdd(counter, 1u);
+                // releases the warp's partials (the __syncwarp above orders them before it) and acquires the others'
+                if (lane == 0) asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(old) : "l"(counter) : "memory");
                 old = __shfl_sync(0xffffffffu, old, 0);
                 if (old == (unsigned)nseg - 1) {
                     if (lane == 0) *counter = 0;  // leave the counter clean for the next call
-                    __threadfence();
                     // the pair's last segment: all warps of the CTA finish it together, below
                     if (segs.more()) {
                         for (int col = 0; col < cols; col += 16) fix_piece(segs.tile, quarter, col);
@@ -545,6 +552,7 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
             lookups(0);
             __syncwarp();
             if (lane == 0) mbar_arrive(w_empty + 8 * rw.idx);  // all of the stage's loads have returned (they return in order)
+            if (u >= S && u < S + kPairGroups) depend();  // the first stages whose A slot has to be emptied first
             if (!mbar_wait_warp(u_empty + 8 * ru.idx, ru.phase ^ 1, abort_flag, p.status, 108)) break;
             tc_fence_after();
             const uint32_t slot = a_lane + (uint32_t)ru.idx * kSlotCols;
