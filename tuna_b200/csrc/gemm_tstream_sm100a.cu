@@ -51,7 +51,8 @@
 //
 // Work decomposition ("stream-K"): a unit is (tile of 128*row_blocks rows, 128- or 256-column chunk) =
 // row_blocks slots; the units, tile-major, are cut into one contiguous range per CTA so that
-// every SM streams the same number of bytes whatever the shape.  A tile cut across CTAs is finished by whichever CTA arrives last at
+// every SM streams the same number of bytes whatever the shape (a single GEMM may take fewer CTAs, so that its tiles
+// are cut into whole segments: ts_pick_split).  A tile cut across CTAs is finished by whichever CTA arrives last at
 // the tile's counter (per 32-row quarter): it adds the fp32 partials from the workspace in range order, so the
 // result does not depend on arrival order (the reference adds fp16 partials with atomicAdd, kernel.cu:2739-2745).  No
 // floating-point atomics, no zero-filled output.  This tail is what a single small GEMM waits for: at 28672x4096 and 16
@@ -764,9 +765,46 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_w4a16_tstream_kernel(const
 
 // ------------------------------------------------------------------ host side
 
-// Columns of a slot: 256 (16 MMAs per wait and commit of the issuing warp) when the matrix is
-// large enough for 16-KB units to balance across the SMs, else 128.
 static int ts_steps(const tuna_config &c) { return c.k_steps == 4 ? 4 : 8; }
+
+// Row blocks per tile and CTAs of a single GEMM, the free ones of them: the lowest estimate in microseconds.  A
+// 128 x 256 slot takes 0.66 us, less where row blocks share its activations.  What comes on top depends on how the
+// tiles are cut: not at all, into whole segments per tile, or anywhere (every CTA the same number of units); the partial
+// sums of a cut tile cost by tokens and row blocks.  The constants are fitted to launches of 512x512 to
+// 57344x8192 at 1 to 32 tokens; examples (us): 4096x4096 at 16 tokens 128 CTAs 8.8, 148 10.0; 4096x14336 two row blocks
+// and 128 CTAs 15.6, one and 148 17.9; 14336x4096 one row block uncut 16.4, 148 CTAs 17.2; 57344x8192 four, two, one: 62, 65, 72.
+static void ts_pick_split(int m, int n, int k, int sm_count, tuna_config *c)
+{
+    const int chunks = div_up(k, 32 * ts_steps(*c));
+    const int groups = div_up(n < c->tile_tok ? n : c->tile_tok, 4);
+    const int rb_wanted = c->row_blocks, ctas_wanted = c->ctas;
+    double best = -1;
+    for (int rb = 1; rb <= 4; rb *= 2) {
+        if ((rb_wanted && rb != rb_wanted) || (!rb_wanted && rb * c->tile_tok > 64)) continue;
+        const double unit_us = rb == 1 ? 0.66 : (rb == 2 ? 1.15 : 2.13);
+        const long long tiles = div_up(m, kBlockRows * rb), units = tiles * chunks;
+        auto consider = [&](long long ctas) {
+            const long long per = (units + ctas - 1) / ctas;
+            const bool whole = ctas % tiles == 0 && chunks % (ctas / tiles) == 0;
+            double us = per * unit_us;
+            if (whole && ctas == tiles) us = 1.15 * us + 3.6 + 0.2 * groups;  // fewer SMs draw on HBM
+            else if (whole) us += 4.8 + (0.3 + 0.1 * rb) * groups + 0.17 * (ctas / tiles);
+            else us += 6.3 + 0.55 * groups + 0.12 * rb * (groups - 1) + 0.17 * (ctas / tiles);
+            if (best < 0 || us < best) {
+                best = us;
+                c->row_blocks = rb;
+                c->ctas = (int)ctas;
+            }
+        };
+        if (ctas_wanted) {
+            consider(ctas_wanted);
+            continue;
+        }
+        consider(sm_count < units ? sm_count : units);
+        for (long long ctas = tiles; ctas <= sm_count && ctas <= units; ctas += tiles) consider(ctas);
+    }
+    if (ctas_wanted) c->ctas = ctas_wanted;
+}
 
 int gemm_tstream_normalize_config(int m, int n, int k, int sm_count, tuna_config *c)
 {
@@ -780,18 +818,15 @@ int gemm_tstream_normalize_config(int m, int n, int k, int sm_count, tuna_config
         if (c->k_steps == 0) c->k_steps = 4;
         if (c->row_blocks != 1 || c->k_steps != 4) return TUNA_ERR_BAD_CONFIG;
     }
-    // two row blocks share an activation stage when the matrix is tall enough for 32-KB units to balance
-    if (c->row_blocks == 0) c->row_blocks = (m >= 8192 && c->tile_tok <= 32) ? 2 : 1;
-    if ((c->row_blocks != 1 && c->row_blocks != 2 && c->row_blocks != 4) || (c->tile_tok <= 64 && c->row_blocks * c->tile_tok > 64))
-        return TUNA_ERR_BAD_CONFIG;
+    if (c->row_blocks != 0 && c->row_blocks != 1 && c->row_blocks != 2 && c->row_blocks != 4) return TUNA_ERR_BAD_CONFIG;
+    if (c->row_blocks != 0 && c->tile_tok <= 64 && c->row_blocks * c->tile_tok > 64) return TUNA_ERR_BAD_CONFIG;
     if (c->ctas < 0) return TUNA_ERR_BAD_CONFIG;
-    if (c->ctas == 0 || c->ctas > sm_count) c->ctas = sm_count;
-    if (c->k_steps == 0) {
-        // 256-column slots unless they leave fewer than ~12 units per CTA to balance with
-        const long long units256 = (long long)div_up(m, kBlockRows * c->row_blocks) * div_up(k, 256);
-        c->k_steps = units256 >= 12ll * c->ctas ? 8 : 4;
-    }
+    if (c->ctas > sm_count) c->ctas = sm_count;
+    // 256-column slots (16 MMAs per wait and commit of the issuing warp) unless one of 128 holds the whole of K:
+    // 128-column slots measured 10 to 30 % slower even where they balance better over the CTAs
+    if (c->k_steps == 0) c->k_steps = k > 128 ? 8 : 4;
     if (c->k_steps != 4 && c->k_steps != 8) return TUNA_ERR_BAD_CONFIG;
+    if (c->row_blocks == 0 || c->ctas == 0) ts_pick_split(m, n, k, sm_count, c);
     return TUNA_OK;
 }
 
