@@ -42,6 +42,7 @@
 // Every wait is bounded: when one runs out the CTA records where in the device status word, raises its
 // abort flag and unwinds to the common exit, where the pair meets and releases the tensor memory.
 #include <cuda.h>
+#include <algorithm>
 #include <cstring>
 #include <mutex>
 #include "common.cuh"
@@ -599,33 +600,72 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
 
 // ------------------------------------------------------------------ host side
 
-// Clocks per 16 columns of K of a tile of `tok` tokens: the tensor pipe's N/2, or the wavefronts of shared
-// memory (see the head of the file).
-static int pair_step_clocks(int tok) { return tok / 2 > tok / 4 + 61 ? tok / 2 : tok / 4 + 61; }
+// Microseconds per 16 columns of K of a tile of `tok` tokens: the wavefronts of shared memory (see the head of the
+// file) at the 1.7 GHz of a short run, or the tensor pipe's N/2 clocks, and what the dequantisation adds to them, at the
+// clock the power cap leaves it (measured at K = 4096: 14 us a wave of 128-token tiles, 22 of 224, 25 of 256).
+static double pair_step_us(int tok) { return std::max((tok / 4 + 61) / 1700.0, (tok / 2 + 8) / 1420.0); }
 
-// Tokens per tile: the multiple of 32 with the least work over all token tiles (the last one may be narrower).
-static int pair_pick_tile_tok(int n)
+static int pair_kc(int tile_tok) { return tile_tok > 128 ? 64 : 128; }
+
+// How the tiles of a launch are handed out (see the head of the file): sk_tiles of them are cut along K over
+// sk_pairs pairs, the others go out in whole waves.
+struct PairSplit {
+    int sk_tiles, sk_pairs;
+    double us;  // the estimate
+};
+
+// What cutting costs beyond the work itself: partial sums written, an arrival, partial sums read by the finishing
+// CTA.  Measured (us, 2 to 8 segments): 32-token tiles 6 to 7, 64 4 to 8, 128 8 to 11, 256 14 to 20; an uncut launch 0.5 to 4.
+static double pair_cut_us(int tile_tok, int segs) { return 5.0 + 0.025 * tile_tok + 0.05 * std::max(0, tile_tok - 128) + segs * (0.25 + 0.002 * tile_tok); }
+constexpr double kPairUncutUs = 1.5;
+
+static PairSplit pair_split(int m, int n, int k, int tile_tok, int pairs)
 {
-    int best = 256;
-    long long best_cost = -1;
-    for (int t = 256; t >= 32; t -= 32) {
-        const int full = n / t, rest = n - full * t;
-        const long long cost = (long long)full * pair_step_clocks(t) + (rest ? pair_step_clocks((rest + 31) / 32 * 32) : 0);
-        if (best_cost < 0 || cost < best_cost) { best = t; best_cost = cost; }
+    const int row_tiles = div_up(m, kPairRows), full = n / tile_tok, last = n - full * tile_tok;
+    const int tok_tiles = full + (last ? 1 : 0), chunks = div_up(k, pair_kc(tile_tok));
+    const long long tiles = (long long)row_tiles * tok_tiles;
+    const double steps = k / 16.0, last_us = last ? steps * pair_step_us((last + 31) / 32 * 32) : 0.0;
+    const double tile_us = full ? steps * pair_step_us(tile_tok) : last_us;  // of the widest tile
+    const double work_us = row_tiles * (full * tile_us + last_us) / pairs;   // per pair, evenly cut
+    const long long waves = tiles / pairs;
+    const int rest = (int)(tiles - waves * pairs);
+    PairSplit best = {0, 0, kPairUncutUs + (waves == 0 ? tile_us : (waves + (rest ? 1 : 0)) * (work_us * pairs / tiles))};
+    auto consider = [&](int sk_tiles, int sk_pairs, double us) {
+        if (us < best.us) best = {sk_tiles, sk_pairs, us};
+    };
+    if (rest > 0 && waves > 0) consider(pairs + rest, pairs, work_us + pair_cut_us(tile_tok, 2));
+    if (waves == 0) {
+        int s = 2;
+        for (; s * tiles <= pairs && s <= chunks; ++s) consider((int)tiles, s * (int)tiles, tile_us / s + pair_cut_us(tile_tok, s));
+        // all pairs, where whole segments leave more than a tenth of them idle
+        if (s <= chunks && (s - 1) * tiles * 10 < pairs * 9) consider((int)tiles, pairs, work_us + pair_cut_us(tile_tok, s + 1));
     }
     return best;
 }
 
-static int pair_kc(int tile_tok) { return tile_tok > 128 ? 64 : 128; }
+// Tokens per tile: the multiple of 32 with the lowest estimate; the smaller one where two are equal.
+static int pair_pick_tile_tok(int m, int n, int k, int pairs)
+{
+    int best = 32;
+    double best_us = -1;
+    for (int t = 32; t <= 256; t += 32) {
+        const double us = pair_split(m, n, k, t, pairs).us;
+        if (best_us < 0 || us < best_us) { best = t; best_us = us; }
+        if (t >= n) break;
+    }
+    return best;
+}
 
 struct PairPlan {
     int tile_tok, kc, stages, w_stages, nd;
 };
 
-static PairPlan pair_plan(int n, const tuna_config &c)
+static int pair_count(const tuna_config &c) { return c.ctas / 2 > 0 ? c.ctas / 2 : 1; }
+
+static PairPlan pair_plan(int m, int n, int k, const tuna_config &c)
 {
     PairPlan l;
-    l.tile_tok = c.tile_tok ? (c.tile_tok < 32 ? 32 : c.tile_tok) : pair_pick_tile_tok(n);
+    l.tile_tok = c.tile_tok ? (c.tile_tok < 32 ? 32 : c.tile_tok) : pair_pick_tile_tok(m, n, k, pair_count(c));
     l.kc = pair_kc(l.tile_tok);
     const int slot = l.kc / 2;
     // two accumulator buffers (the epilogue of one tile overlaps the MMAs of the next) where they leave four A slots
@@ -660,8 +700,7 @@ int gemm_umma_normalize_config(int m, int n, int k, int sm_count, tuna_config *c
 
 size_t gemm_umma_workspace_bytes(int m, int n, int k, const tuna_config &c, int sm_count)
 {
-    (void)k;
-    const PairPlan l = pair_plan(n, c);
+    const PairPlan l = pair_plan(m, n, k, c);
     const long long tiles = (long long)div_up(m, kPairRows) * div_up(n, l.tile_tok);
     const long long cut = tiles < sm_count ? tiles : sm_count;  // fewer than two waves of tiles are cut along K
     return partial_region_bytes(sm_count) + ((size_t)cut * 32 + 255) / 256 * 256;  // one counter per tile, CTA and TMEM lane quarter
@@ -700,7 +739,7 @@ static int launch_pair(const PairParams &p, const CUtensorMap &mq, const CUtenso
 
 int launch_gemm_umma(const GemmArgs &a, const tuna_config &c)
 {
-    const PairPlan l = pair_plan(a.n, c);
+    const PairPlan l = pair_plan(a.m, a.n, a.k, c);
     PairParams p;
     std::memset(&p, 0, sizeof(p));
     p.code = a.code; p.absmax = a.absmax; p.o = (__half *)a.o;
@@ -720,29 +759,10 @@ int launch_gemm_umma(const GemmArgs &a, const tuna_config &c)
     const long long tiles_ll = (long long)p.row_tiles * p.tok_tiles;
     if (tiles_ll * p.chunks >= (1ll << 30)) return TUNA_ERR_TOO_LARGE;
     const int tiles = (int)tiles_ll;
-    int pairs = c.ctas / 2 > 0 ? c.ctas / 2 : 1;
-    // Whole waves, and what is left over cut along K: `rest` tiles more than whole waves take a wave of their own
-    // (tile_us) or, cut over all pairs together with the last whole wave, rest / pairs of it plus an exchange of partial sums
-    // (a few microseconds: measured 3 to 6).  Below one wave the cut also shortens the critical path, but every further
-    // segment of a tile adds N * 512 bytes that the finishing CTA reads (~0.2 TB/s): s segments cost tile_us / s + s * fix_us.
-    const double tile_us = (double)p.chunks * (l.kc / 16) * pair_step_clocks(l.tile_tok) / 1700.0;
-    const double fix_us = l.tile_tok * 512.0 / 0.2e6;
-    const int waves = tiles / pairs, rest = tiles - waves * pairs;
-    p.sk_tiles = 0;
-    p.sk_pairs = 0;
-    if (rest > 0) {
-        if (waves > 0) {
-            if (tile_us * (pairs - rest) / pairs > 5.0) { p.sk_tiles = pairs + rest; p.sk_pairs = pairs; }
-        } else {
-            int s = 1;
-            while ((s + 1) * rest <= pairs && s + 1 <= p.chunks && tile_us / (s + 1) + (s + 1) * fix_us + (s == 1 ? 3.0 : 0.0) < tile_us / s + (s == 1 ? 0.0 : s * fix_us)) ++s;
-            if (s > 1) {
-                p.sk_tiles = tiles;
-                // whole segments per tile, unless that leaves a tenth of the machine idle that a finer cut would use
-                p.sk_pairs = (s + 1) * rest > pairs && s * rest * 10 < pairs * 9 ? pairs : s * rest;
-            }
-        }
-    }
+    int pairs = pair_count(c);
+    const PairSplit split = pair_split(a.m, a.n, a.k, l.tile_tok, pairs);
+    p.sk_tiles = split.sk_tiles;
+    p.sk_pairs = split.sk_pairs;
     if (p.sk_tiles) {
         const int units = p.sk_tiles * p.chunks;
         if (p.sk_pairs > units) p.sk_pairs = units;
