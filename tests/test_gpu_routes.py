@@ -1,0 +1,21 @@
+"""tuna_matmul without a configuration on both sides of the lines where its kernel, tile and split change: uncut tiles,
+whole segments per tile, tiles cut anywhere; ragged rows and columns."""
+
+import pytest
+
+from oracle import tuna_oracle as orc
+from tests.gpu_util import check_parity, make_case, run_matmul, stream_ptr
+from tuna_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [1, 16, 17, 32, 33, 64, 65, 129])
+@pytest.mark.parametrize("m,k", [(8, 8), (136, 136), (512, 128), (520, 2048), (4104, 1032), (1024, 8192), (18952, 264)])
+def test_default_route_matches_the_oracle(m, k, n):
+    host, dev = make_case(m, n, k, seed=m + n)
+    st, out, holder = run_matmul(dev, m, n, k)
+    assert st == 0
+    assert _lib.load().tuna_check_device_status(stream_ptr()) == 0, "a bounded wait ran out"
+    check_parity(out.cpu().numpy(), orc.matmul_ref(*host, m, n, k), 1e-2)
+    assert holder.guards_intact()

@@ -48,6 +48,8 @@ static int device_sm_count()
     return cached[dev];
 }
 
+constexpr int kStreamTokens = 32;
+
 static int resolve_config(int m, int n, int k, int sm_count, const tuna_config *user, tuna_config *out)
 {
     tuna_config c;
@@ -59,9 +61,10 @@ static int resolve_config(int m, int n, int k, int sm_count, const tuna_config *
         for (int i = 0; i < kTableSize; ++i)
             if (kTable[i].m == m && kTable[i].k == k && kTable[i].n_bucket == b) { c = kTable[i].cfg; break; }
     }
-    // No table entry: the tcgen05 weight-streaming kernel up to one 64-token pass (the regime
-    // bound by HBM), the TMA-staged tcgen05 kernel above it.
-    if (c.path == TUNA_PATH_AUTO) c.path = (n <= 64) ? TUNA_PATH_TSTREAM : TUNA_PATH_UMMA;
+    // No table entry: the tcgen05 weight-streaming kernel up to 32 tokens (the regime bound by HBM), the
+    // kernel on CTA pairs above, which stages half of the tokens per SM (us, weight streaming / pairs: 57344x8192 at 64
+    // tokens 95 / 74, at 32 69 / 69, at 16 62 / 67; 4096x4096 at 43 11.1 / 10.9, at 24 9.3 / 10.0; 11000x4104 at 43 19.9 / 15.4).
+    if (c.path == TUNA_PATH_AUTO) c.path = (n <= kStreamTokens) ? TUNA_PATH_TSTREAM : TUNA_PATH_UMMA;
     int st;
     if (c.path == TUNA_PATH_STREAM) st = gemm_stream_normalize_config(m, n, k, sm_count, &c);
     else if (c.path == TUNA_PATH_UMMA) st = gemm_umma_normalize_config(m, n, k, sm_count, &c);
@@ -96,8 +99,8 @@ static int launch_gemm(const GemmArgs &a, const tuna_config &c)
 }
 
 // Whether equal-shape GEMMs share persistent launches of the sequence kernel: every token count it
-// takes (eight 4096x14336 GEMMs of 16 tokens: 132 us as a launch each, 69 as one).
-static bool batched_as_sequence(const tuna_config &c, int n) { return c.path == TUNA_PATH_TSTREAM && n <= 64; }
+// takes (eight 4096x14336 GEMMs of 16 tokens: 132 us as a launch each, 66 as one).
+static bool batched_as_sequence(const tuna_config &c, int n) { return c.path != TUNA_PATH_STREAM && n <= 64; }
 
 }  // namespace tuna
 
