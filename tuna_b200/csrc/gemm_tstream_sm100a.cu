@@ -665,6 +665,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_w4a16_tstream_kernel(const
         int a_idx = group % A, w_idx = group % WS;  // ring positions of slot `sl`: sl % A, sl % WS
         uint32_t a_phase = (uint32_t)(group / A) & 1u, w_phase = (uint32_t)(group / WS) & 1u;
         bool ok = true;
+        if (MAXG > 1) depend();  // a sequence is too long to gain from a head start
 #ifdef TUNA_TS_PROFILE
         const long long loop_c0 = clock64();
 #endif
@@ -713,7 +714,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_w4a16_tstream_kernel(const
             // producer.  The arrival is a release: it is ordered after this warp's loads.
             __syncwarp();
             if (lane == 0) mbar_arrive(w_empty + 8 * w_idx);
-            if (sl >= A && sl < A + kGroups) depend();  // the first slots whose A-slot has to be emptied first
+            if (MAXG == 1 && sl >= A && sl < A + kGroups) depend();  // the first slots whose A-slot has to be emptied first
             TS_PROF_BEGIN
             ok = mbar_wait_warp(a_empty + 8 * a_idx, a_phase ^ 1, abort_flag, p.status, 7);
             TS_PROF_END(0)
