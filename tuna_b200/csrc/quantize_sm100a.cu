@@ -26,7 +26,7 @@
 // comparison per weight.  The table is exact because a threshold is filed under the bucket the same
 // FMA gives it.  Rows it cannot represent (two thresholds in one bucket, a zero, tiny or
 // non-finite absmax, codes that are equal, closer than fp32 can separate, or not finite) take the
-// literal expression.  28672x4096: 436 -> 84 us (0.68 -> 3.5 TB/s of its 294 MB).
+// literal expression.  28672x4096: 436 -> 80 us (0.68 -> 3.7 TB/s of its 294 MB).
 #include <cuda_fp16.h>
 #include <mutex>
 #include "common.cuh"
@@ -37,7 +37,7 @@ namespace tuna {
 
 constexpr int kQuantThreads = 256;
 constexpr int kQuantShareCols = 4096;      // columns of a CTA's share a cluster is chosen for
-constexpr int kQuantMaxShareCols = 14000;  // what shared memory holds at one CTA per SM
+constexpr int kQuantMaxShareCols = 13936;  // what shared memory holds at one CTA per SM (beside the tables)
 constexpr int kQuantMaxCluster = 8;
 constexpr int kBuckets = 128;
 // The "NormalFloat4" levels the reference's quantizer emits (test.py:19-40); codebooks.py has the same list.
@@ -46,7 +46,11 @@ __constant__ float kNf4[16] = {-1.0f, -0.6961928009986877f, -0.5250730514526367f
                                0.24611230194568634f, 0.33791524171829224f, 0.44070982933044434f, 0.5626170039176941f,
                                0.7229568362236023f, 1.0f};
 
-constexpr int kTableStride = kBuckets + 4;  // words; the skew keeps equal buckets of the 8 rows in different banks
+// The rows' tables lie side by side, bucket by bucket, each row's twice: lane l of a warp (row l % 8) looks up in column
+// l % 16, so that two lanes share a bank at most (rows' tables one after another, where random
+// lookups meet three or four at a time: 84 us against 80 on 28672x4096).
+constexpr int kTableCols = 16;
+constexpr int kThrStride = 17;  // words of a row's thresholds: the eight rows' lie in different banks
 
 // The reference's expression for one weight.
 __device__ __forceinline__ uint32_t nearest_code(float w, float scale, const float *cb)
@@ -88,9 +92,9 @@ __global__ void __launch_bounds__(kQuantThreads) quantize_rows_kernel(const __ha
     __shared__ uint32_t s_row_max[8];  // fp16 bits; read by the other CTAs of the cluster
     __shared__ float s_scale[8];
     __shared__ uint32_t s_bucket_scale[8];  // half2
-    __shared__ uint32_t s_thr[8][16];       // fp16 bits of threshold i | its bucket << 16
+    __shared__ uint32_t s_thr[8][kThrStride];  // fp16 bits of threshold i | its bucket << 16
     __shared__ int s_row_ok[8];
-    __shared__ uint32_t s_table[8 * kTableStride];  // fp16 threshold | codes (below | (below ^ above) << 4) << 16
+    __shared__ uint32_t s_table[kBuckets * kTableCols];  // fp16 threshold | codes (below | (below ^ above) << 4) << 16
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int rg = blockIdx.x / cluster, rank = blockIdx.x - rg * cluster;
@@ -243,26 +247,29 @@ __global__ void __launch_bounds__(kQuantThreads) quantize_rows_kernel(const __ha
     }
     __syncthreads();
 
-    // ---- the rows' tables: warp `warp` fills row `warp`
+    // ---- the rows' tables: lane (row r, l / 8) fills four of the warp's 16 buckets
     {
-        uint32_t below[kBuckets / 32] = {}, hits[kBuckets / 32] = {}, thr[kBuckets / 32];
+        const int row = lane & 7, b0 = warp * (kBuckets / 8) + (lane >> 3);
+        uint32_t below[4] = {}, hits[4] = {}, thr[4];
 #pragma unroll
-        for (int j = 0; j < kBuckets / 32; ++j) thr[j] = 0x7fffu;
+        for (int j = 0; j < 4; ++j) thr[j] = 0x7fffu;
         for (int i = 0; i < 15; ++i) {
-            const uint32_t t = s_thr[warp][i], bt = t >> 16;
+            const uint32_t t = s_thr[row][i], bt = t >> 16;
 #pragma unroll
-            for (int j = 0; j < kBuckets / 32; ++j) {
-                const uint32_t b = (uint32_t)(lane + 32 * j);
+            for (int j = 0; j < 4; ++j) {
+                const uint32_t b = (uint32_t)(b0 + 4 * j);
                 below[j] += bt < b ? 1u : 0u;
                 if (bt == b) { ++hits[j]; thr[j] = t & 0xffffu; }
             }
         }
 #pragma unroll
-        for (int j = 0; j < kBuckets / 32; ++j) {
-            const uint32_t b = (uint32_t)(lane + 32 * j);
+        for (int j = 0; j < 4; ++j) {
+            const uint32_t b = (uint32_t)(b0 + 4 * j);
             const uint32_t lo = s_sorted_idx[below[j]], hi = s_sorted_idx[min(below[j] + 1u, 15u)];
-            s_table[warp * kTableStride + b] = thr[j] | ((lo | ((lo ^ hi) << 4)) << 16);
-            if (b > 0 && hits[j] > 1) s_row_ok[warp] = 0;
+            const uint32_t e = thr[j] | ((lo | ((lo ^ hi) << 4)) << 16);
+            s_table[b * kTableCols + row] = e;
+            s_table[b * kTableCols + 8 + row] = e;
+            if (b > 0 && hits[j] > 1) s_row_ok[row] = 0;
         }
     }
     __syncthreads();
@@ -272,7 +279,7 @@ __global__ void __launch_bounds__(kQuantThreads) quantize_rows_kernel(const __ha
         uint8_t *dst = q + (size_t)rg * row_group_bytes(k) + (size_t)col0 * 4 + r * 4;
         if (s_row_ok[r]) {
             const uint32_t scale2 = s_bucket_scale[r];
-            const uint32_t table = smem_u32(&s_table[r * kTableStride]);
+            const uint32_t table = smem_u32(&s_table[lane & (kTableCols - 1)]);
             for (int kt = 4 * warp + tl; kt < tiles; kt += kTilesPerPass) {
                 const uint4 v = load8(kt);
                 const uint32_t u[4] = {v.x, v.y, v.z, v.w};
@@ -280,8 +287,8 @@ __global__ void __launch_bounds__(kQuantThreads) quantize_rows_kernel(const __ha
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const uint32_t b2 = buckets2(u[i], scale2);
-                    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(e0[i]) : "r"(table + 4u * (b2 & 0xffu)));
-                    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(e1[i]) : "r"(table + 4u * __byte_perm(b2, 0, 0x4442)));
+                    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(e0[i]) : "r"(table + 4u * kTableCols * (b2 & 0xffu)));
+                    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(e1[i]) : "r"(table + 4u * kTableCols * __byte_perm(b2, 0, 0x4442)));
                 }
                 uint32_t word = 0;
 #pragma unroll
@@ -311,7 +318,7 @@ __global__ void __launch_bounds__(kQuantThreads) quantize_rows_kernel(const __ha
     if (cluster > 1) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
 }
 
-// ---- rows too wide for a cluster's shared memory (k > 112000): two passes over memory, the literal expression
+// ---- rows too wide for a cluster's shared memory (k > 111488): two passes over memory, the literal expression
 
 __global__ void __launch_bounds__(256) row_absmax_kernel(const __half *__restrict__ w, float *__restrict__ absmax, int m, int k)
 {
