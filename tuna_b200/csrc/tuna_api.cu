@@ -48,7 +48,7 @@ static int device_sm_count()
     return cached[dev];
 }
 
-constexpr int kStreamTokens = 32;
+constexpr int kStreamTokens = 24;
 
 static int resolve_config(int m, int n, int k, int sm_count, const tuna_config *user, tuna_config *out)
 {
@@ -61,9 +61,10 @@ static int resolve_config(int m, int n, int k, int sm_count, const tuna_config *
         for (int i = 0; i < kTableSize; ++i)
             if (kTable[i].m == m && kTable[i].k == k && kTable[i].n_bucket == b) { c = kTable[i].cfg; break; }
     }
-    // No table entry: the tcgen05 weight-streaming kernel up to 32 tokens (the regime bound by HBM), the
-    // kernel on CTA pairs above, which stages half of the tokens per SM (us, weight streaming / pairs: 57344x8192 at 64
-    // tokens 95 / 74, at 32 69 / 69, at 16 62 / 67; 4096x4096 at 43 11.1 / 10.9, at 24 9.3 / 10.0; 11000x4104 at 43 19.9 / 15.4).
+    // No table entry: the tcgen05 weight-streaming kernel up to 24 tokens (the regime bound by HBM), the
+    // kernel on CTA pairs above, which stages half of the tokens per SM.  Measured (us, weight streaming / pairs):
+    // 57344x8192 at 64 tokens 95 / 74, at 32 69 / 69, at 16 62 / 67; 14336x4096 at 32 17.3 / 15.4, 2048x2048 at 32
+    // 7.2 / 6.2; 4096x4096 at 43 11.1 / 10.9, at 32 10.0 / 10.0, at 24 9.3 / 10.1; 28672x4096 at 32 26.9 / 26.5, at 24 25.3 / 26.5.
     if (c.path == TUNA_PATH_AUTO) c.path = (n <= kStreamTokens) ? TUNA_PATH_TSTREAM : TUNA_PATH_UMMA;
     int st;
     if (c.path == TUNA_PATH_STREAM) st = gemm_stream_normalize_config(m, n, k, sm_count, &c);
