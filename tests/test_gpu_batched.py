@@ -59,9 +59,10 @@ def _batched_abi(xd, qd, sd, cd, out, batch, m, n, k, ws, o_stride=None):
                                    torch.cuda.current_stream().cuda_stream)
 
 
-@pytest.mark.parametrize("batch,m,n,k", [(70, 136, 16, 264), (66, 64, 33, 128)])
+@pytest.mark.parametrize("batch,m,n,k", [(70, 136, 16, 264), (66, 64, 33, 128), (3, 40000, 40, 64)])
 def test_batched_more_matrices_than_one_launch_and_small_workspaces(batch, m, n, k):
-    """Batches beyond one launch's table, and workspaces that hold the counters of one matrix only: the same results."""
+    """Batches beyond one launch's table, and workspaces that hold the counters of one matrix only - in the last case fewer
+    than a shared launch needs for one: the same results."""
     lib = tuna_b200._lib.load()
     per, x, q, s, code = _case(batch, m, n, k, 1200 + n, False)
     xd, qd, sd, cd = (torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (x, q, s, code))

@@ -159,8 +159,11 @@ extern "C" int tuna_matmul_batched(const void *q, const void *x, const void *cod
     }
     const size_t need = workspace_for(m, n, k, c, sms);
     if (workspace == nullptr || workspace_bytes < need) return TUNA_ERR_WORKSPACE;
-    if (batched_as_sequence(c, n) && batch > 1 && o_stride >= (size_t)n * m * 2) {
-        // persistent launches over up to 64 matrices each (as many as the workspace has counters for: at least one).
+    const tuna_gemm_desc one = {q, x, absmax, o, m, n, k, 0};
+    if (batched_as_sequence(c, n) && batch > 1 && o_stride >= (size_t)n * m * 2 &&
+        gemm_tstream_sequence_min_workspace_bytes(&one, 1, sms) <= workspace_bytes) {
+        // persistent launches over up to 64 matrices each: as many as the workspace has counters for.  One that cannot
+        // hold a single matrix's (a launch of its own may need fewer) is served by the launches per matrix below.
         // Launches on a stream follow one another and leave the counters zero, so all use the same ones.
         tuna_gemm_desc d[kSequenceMax];
         for (int first = 0; first < batch;) {
