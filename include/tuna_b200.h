@@ -90,6 +90,12 @@ typedef struct tuna_config {
  * that overlap on the device need separate workspaces.  Alignment: q, x, o,
  * workspace 16 bytes; absmax, code 4 bytes (absmax may be a slice of a larger
  * scale buffer).
+ * Order: x, absmax, o and the workspace follow ordinary stream order.  So do q and code above 64 tokens.
+ * Up to 64 tokens (and in tuna_matmul_batched and the sequences below) q and code count as constants
+ * and are read while the kernel before the call in its stream still drains: a kernel that
+ * writes them right before such a call must not let dependent launches start early
+ * (griddepcontrol.launch_dependents; this library's quantizer does not); behind one that does,
+ * enqueue something that is not a kernel (a copy, a memset) in between, or synchronise.
  */
 int tuna_matmul(const void *q, const void *x, const void *code, const void *absmax, void *o,
                 int m, int n, int k, void *workspace, size_t workspace_bytes, void *stream);

@@ -65,6 +65,11 @@ constexpr int kPairMaxStages = 8;           // unit stages: activations in share
 constexpr int kPairMaxWStages = 8;
 constexpr int kPairSmemDynamic = 226 * 1024;
 constexpr int kPairTokGroup = 8;            // token tiles of a wave's working set
+// Up to here weights and codebook are read ahead of the dependency wait, as the weight-streaming kernels do (the header's
+// contract); more tokens see ordinary stream order.  Reading ahead hides the pipeline's fill: 11000x4104 at 43 tokens
+// 14.7 us against 17.1, 28672x4096 at 64 25.7 / 28.1; what ordinary order costs above: 6144x4096 at 256 16.6 -> 17.6,
+// 28672x4096 at 1024 163.2 -> 164.9 (graph replay).
+constexpr int kPairAheadTokens = 64;
 
 struct PairParams {
     const float *code;
@@ -81,6 +86,7 @@ struct PairParams {
     int stages;       // unit stages
     int w_stages;
     int nd;           // accumulator buffers
+    int ahead;        // weights and codebook are read before the dependency wait
     int q3d;          // the weights' tensor map is the 3-D view (WMODE 0)
     int sk_tiles;     // tiles 0 .. sk_tiles - 1 are cut along K over pairs 0 .. sk_pairs - 1 ...
     int sk_pairs;
@@ -220,13 +226,20 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
     }
     __syncthreads();  // this CTA's barriers are initialised: its weight producer may start
 
+    // What a kernel before this one wrote is there only after this wait: its end alone, or its letting dependents start, is no
+    // promise.  The copies of x and the epilogue always wait; weights and codebook are read ahead of it (the dequant
+    // warps fill the A slots meanwhile) up to kPairAheadTokens only.
+    auto depend = [] { asm volatile("griddepcontrol.wait;" ::: "memory"); };
+    if (!p.ahead) depend();
+
     PairSegs segs;
     segs.init(p, pair, pairs);
     const int total = segs.total_units(p);
 
     // Rest of the prologue, run by every warp inside its own role's branch: the byte -> half2 table (even
-    // column = high nibble in the low half) - the codebook is a constant, so this runs before the dependency
-    // wait - then the wait, then the barrier of the pair, which publishes both CTAs' barriers and tables.
+    // column = high nibble in the low half), then the barrier of the pair, which publishes both CTAs' barriers and tables.
+    // depend() comes after it in every role that needs it, and in whoever is about to make a bounded wait that
+    // ends only after the kernels before this one.
     auto finish_prologue = [&]() -> uint32_t {
         const float cv = p.code[lane & 15];
         const uint32_t ch = (uint32_t)__half_as_ushort(__float2half_rn(cv));
@@ -239,10 +252,6 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
         tc_fence_after();
         return s_tmem_base;
     };
-    // Only what reads or writes data of the kernels before this one waits for them (the copies of x, the
-    // epilogue), and whoever is about to make a bounded wait that ends only after that; the weights
-    // are constants, so the dequant warps fill the A slots meanwhile.
-    auto depend = [] { asm volatile("griddepcontrol.wait;" ::: "memory"); };
     uint32_t tmem = 0;
     const uint32_t d_cols = (uint32_t)N;
     const uint32_t a_off = (uint32_t)p.nd * d_cols;  // first A slot
@@ -340,8 +349,7 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ weight producer
-        // One elected lane of the converged warp issues the copies.  The weights are constants: the first
-        // ones are requested before the dependency wait.
+        // One elected lane of the converged warp issues the copies, the first ones before the rest of the prologue.
         Ring rw;
         int u = 0;
         bool ok = segs.next(p);
@@ -750,6 +758,7 @@ int launch_gemm_umma(const GemmArgs &a, const tuna_config &c)
     p.tok_tiles = div_up(a.n, l.tile_tok);
     p.rot_step = p.chunks * 5 / 8 | 1;
     p.stages = l.stages; p.w_stages = l.w_stages; p.nd = l.nd;
+    p.ahead = a.n <= kPairAheadTokens;
     p.status = device_status_word();
     if (!p.status) return TUNA_ERR_NO_DEVICE;
     if (a.workspace == nullptr || a.workspace_bytes < gemm_umma_workspace_bytes(a.m, a.n, a.k, c, a.sm_count)) return TUNA_ERR_WORKSPACE;
