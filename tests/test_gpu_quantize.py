@@ -1,5 +1,7 @@
 """The device quantizer against the oracle (bit-exact) and the torch-CPU golden fixture."""
 
+import subprocess
+import sys
 from pathlib import Path
 
 import numpy as np
@@ -97,3 +99,27 @@ def test_widest_single_pass_rows():
         q_ref, a_ref, _ = orc.quantize_blockwise_dynamic_4bit(w)
         assert np.array_equal(absmax.cpu().numpy(), a_ref)
         assert np.array_equal(q.cpu().numpy(), q_ref)
+
+
+FIRST_CALL_CAPTURED = """
+import numpy as np, torch, tuna_b200
+from oracle import tuna_oracle as orc
+w = (np.random.default_rng(5).standard_normal((64, 4104)) * 0.05).astype(np.float16)
+wd, code = torch.zeros(w.shape, dtype=torch.float16, device="cuda"), torch.from_numpy(orc.NF4_CODE).cuda()
+g = torch.cuda.CUDAGraph()
+with torch.cuda.graph(g):
+    q, (absmax, c) = tuna_b200.quantize(wd, {codebook})
+wd.copy_(torch.from_numpy(w))
+g.replay()
+q_ref, a_ref, _ = orc.quantize_blockwise_dynamic_4bit(w)
+assert np.array_equal(q.cpu().numpy(), q_ref) and np.array_equal(absmax.cpu().numpy(), a_ref)
+assert np.array_equal(c.cpu().numpy(), orc.NF4_CODE)
+assert tuna_b200._lib.load().tuna_check_device_status(torch.cuda.current_stream().cuda_stream) == 0
+"""
+
+
+@pytest.mark.parametrize("codebook", ["None", "code"])
+def test_first_call_of_a_process_can_be_captured(codebook):
+    r = subprocess.run([sys.executable, "-c", FIRST_CALL_CAPTURED.format(codebook=codebook)], capture_output=True, text=True, timeout=300,
+                       cwd=GOLDEN.parents[1])
+    assert r.returncode == 0, r.stderr[-2000:]

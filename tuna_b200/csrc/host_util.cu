@@ -8,6 +8,9 @@
 
 namespace tuna {
 
+// File scope and not cudaMalloc: the first call on a device may come while a stream is being captured.
+static __device__ __align__(8) DeviceStatus g_device_status;
+
 DeviceStatus *device_status_word()
 {
     static DeviceStatus *ptrs[64] = {nullptr};
@@ -16,10 +19,9 @@ DeviceStatus *device_status_word()
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
     std::lock_guard<std::mutex> lock(mu);
     if (!ptrs[dev]) {
-        DeviceStatus *p = nullptr;
-        if (cudaMalloc(&p, sizeof(DeviceStatus)) != cudaSuccess) return nullptr;
-        cudaMemset(p, 0, sizeof(DeviceStatus));
-        ptrs[dev] = p;
+        void *p = nullptr;
+        if (cudaGetSymbolAddress(&p, g_device_status) != cudaSuccess) return nullptr;
+        ptrs[dev] = (DeviceStatus *)p;
     }
     return ptrs[dev];
 }
