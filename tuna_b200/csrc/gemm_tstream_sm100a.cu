@@ -325,6 +325,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_w4a16_tstream_kernel(const
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
+        __syncwarp();  // lane 0 comes from the branch above, and the allocation wants a converged warp
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem_base)),
                      "r"(kTsTmemCols)
                      : "memory");
@@ -759,6 +760,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_w4a16_tstream_kernel(const
     if (warp < kTsDequantWarp0) { TS_PROF_MARK(3) }
     TS_PROF_STORE
     if (warp == 0) {
+        __syncwarp();  // lanes of rows past the matrix leave finish_tile early
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTsTmemCols) : "memory");
     }

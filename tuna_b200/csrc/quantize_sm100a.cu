@@ -160,6 +160,7 @@ __global__ void __launch_bounds__(kQuantThreads) quantize_rows_kernel(const __ha
         s_row_max[tid] = best;
     }
     if (cluster > 1) {
+        __syncwarp();  // the aligned barriers want converged warps, and lanes take different ways before each of them
         asm volatile("barrier.cluster.arrive.aligned;\n barrier.cluster.wait.aligned;" ::: "memory");
         if (tid < 8) {
             uint32_t best = 0;
@@ -172,6 +173,7 @@ __global__ void __launch_bounds__(kQuantThreads) quantize_rows_kernel(const __ha
             s_warp_max[0][tid] = best;  // not s_row_max: the other CTAs may still be reading it
         }
         // the matching wait stands at the end: no CTA leaves while another may read its maxima
+        __syncwarp();
         asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
     } else if (tid < 8) {
         s_warp_max[0][tid] = s_row_max[tid];
@@ -315,7 +317,10 @@ __global__ void __launch_bounds__(kQuantThreads) quantize_rows_kernel(const __ha
             }
         }
     }
-    if (cluster > 1) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    if (cluster > 1) {
+        __syncwarp();
+        asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    }
 }
 
 // ---- rows too wide for a cluster's shared memory (k > 111488): two passes over memory, the literal expression
