@@ -2,6 +2,8 @@
 
 import random
 
+import pytest
+
 from tuna_b200 import _lib, tuner
 
 
@@ -32,6 +34,21 @@ def test_validity_filter_matches_the_launcher(tuna_lib):
         g = dict(row_blocks=1, stages_w=4, stages_x=4, dequant_warps=16, k_accs=1)
         g.update(bad)
         assert not tuner.is_valid(tuna_lib, 4096, 2048, 4096, tuner.to_config("umma", 64, g))
+
+
+@pytest.mark.parametrize("n,tile_tok,fields,fits", [
+    (2048, 0, dict(row_blocks=4), False),      # 4 x 256 accumulator columns
+    (100, 0, dict(row_blocks=2), True),
+    (1, 0, dict(stages_x=4), False),           # four row blocks of 16 tokens: two accumulators leave three A-slot stages
+    (16, 16, dict(row_blocks=1, stages_x=15), True),
+    (16, 16, dict(row_blocks=1, stages_x=16), False),
+    (256, 256, dict(row_blocks=1, stages_w=4, stages_x=5), True),
+    (256, 256, dict(row_blocks=1, stages_w=9, stages_x=5), False),  # shared memory: 32 + 36 + 160 KB
+    (128, 128, dict(row_blocks=2, stages_w=6, stages_x=4), True),
+    (128, 128, dict(row_blocks=2, stages_w=6, stages_x=5), False),
+])
+def test_umma_fields_that_do_not_fit_one_sm_are_refused(tuna_lib, n, tile_tok, fields, fits):
+    assert tuner.is_valid(tuna_lib, 4096, n, 4096, tuner.to_config("umma", tile_tok, fields)) == fits
 
 
 def test_config_fields_round_trip():

@@ -688,19 +688,33 @@ static PairPlan pair_plan(int m, int n, int k, const tuna_config &c)
     return l;
 }
 
+// The fields of an explicit configuration describe a tile of one SM - `row_blocks` x 128 rows x `tile_tok` tokens in stages
+// of 64 columns - and what does not fit one SM's tensor or shared memory is refused, although this kernel takes no
+// more than the token tile from them.
+static bool umma_fields_fit(int n, const tuna_config &c)
+{
+    constexpr int kSlot = 32, kLut = 32 * 1024, kBlock = 4096, kSmem = 225 * 1024;  // A-slot columns; bytes
+    const int t = c.tile_tok ? c.tile_tok : (n <= 16 ? 16 : n <= 32 ? 32 : n <= 64 ? 64 : n <= 128 ? 128 : 256);
+    const int rb = c.row_blocks ? c.row_blocks : (t <= 32 ? 4 : (t <= 64 ? 2 : 1));
+    if (rb * t + 2 * rb * kSlot > kPairTmemCols) return false;
+    const int bufs = 2 * rb * t + 2 * rb * kSlot <= kPairTmemCols ? 2 : 1;
+    const int sw = c.stages_w ? c.stages_w : (rb == 4 ? 4 : (rb == 2 ? 6 : 8));
+    const int sx = c.stages_x ? c.stages_x : 2;  // left free, as few as it takes
+    return sx <= (kPairTmemCols - bufs * rb * t) / (rb * kSlot) && kLut + sw * rb * kBlock + sx * t * 128 <= kSmem;
+}
+
 int gemm_umma_normalize_config(int m, int n, int k, int sm_count, tuna_config *c)
 {
-    (void)m; (void)n; (void)k;
-    // tile_tok 0 lets the launcher choose per token count; the fields of the earlier one-SM kernel are accepted as far as
-    // that kernel took them (row blocks, stage counts, dequant warps) and no longer steer anything
+    (void)m; (void)k;
+    // tile_tok 0 lets the launcher choose per token count
     const int t = c->tile_tok;
     if (t != 0 && t != 16 && t != 32 && t != 64 && t != 128 && t != 256) return TUNA_ERR_BAD_CONFIG;
     if (c->row_blocks != 0 && c->row_blocks != 1 && c->row_blocks != 2 && c->row_blocks != 4) return TUNA_ERR_BAD_CONFIG;
     if (c->dequant_warps != 0 && c->dequant_warps != 8 && c->dequant_warps != 16) return TUNA_ERR_BAD_CONFIG;
     if (c->k_accs != 0 && c->k_accs != 1) return TUNA_ERR_BAD_CONFIG;
-    if (c->row_blocks * t + 64 * c->row_blocks > kPairTmemCols) return TUNA_ERR_BAD_CONFIG;
     if (c->stages_x != 0 && (c->stages_x < 2 || c->stages_x > 16)) return TUNA_ERR_BAD_CONFIG;
     if (c->stages_w != 0 && (c->stages_w < 4 || c->stages_w > 16)) return TUNA_ERR_BAD_CONFIG;
+    if (!umma_fields_fit(n, *c)) return TUNA_ERR_BAD_CONFIG;
     if (c->ctas < 0) return TUNA_ERR_BAD_CONFIG;
     if (c->ctas == 0 || c->ctas > sm_count) c->ctas = sm_count;
     return TUNA_OK;
