@@ -57,19 +57,20 @@ typedef enum tuna_path {
 typedef struct tuna_config {
     int32_t path;          /* tuna_path                                               */
     int32_t tile_tok;      /* tokens per pass: stream 8|16|32; tstream 16|32|64|128;  *
-                            * umma 16|32|64|128|256 (the largest tile; 0 = by shape)  */
+                            * umma 16 or a multiple of 32 up to 256 (0 = by shape)     */
     int32_t rows_per_warp; /* stream: 32-row blocks per warp (1|2)                    */
     int32_t warps_m;       /* stream: consumer warps along output rows (power of 2)   */
     int32_t warps_k;       /* stream: consumer warps along K (power of 2, m*k <= 16)  */
     int32_t k_steps;       /* stream: 32-column steps per warp per unit (8|16|32|64); *
                             * tstream: 32-column steps per slot (4|8)                 */
     int32_t ctas;          /* persistent CTAs (0 = one per SM)                        */
-    int32_t stages_w;      /* umma: 0, or 4..16 (range-checked; the kernel derives it) */
-    int32_t stages_x;      /* umma: 0, or 2..16 (the same)                            */
-    int32_t dequant_warps; /* umma: 0, 8 or 16 (the same)                             */
-    int32_t row_blocks;    /* tstream: 128-row blocks per CTA tile (1|2|4); umma as above */
+    int32_t stages_w;      /* umma: 0, or 4..16.  This and the next four are checked,  *
+                            * also for what fits one SM, and steer nothing             */
+    int32_t stages_x;      /* umma: 0, or 2..16                                       */
+    int32_t dequant_warps; /* umma: 0, 8 or 16                                        */
+    int32_t row_blocks;    /* 128-row blocks per CTA tile (1|2|4; steers tstream only) */
     int32_t stages_a;      /* ignored                                                 */
-    int32_t k_accs;        /* umma: 0 or 1 (as above)                                 */
+    int32_t k_accs;        /* umma: 0 or 1                                            */
     int32_t reserved[3];
 } tuna_config;
 
@@ -116,7 +117,8 @@ size_t tuna_workspace_scratch_bytes(void);
 
 /* The configuration tuna_matmul would use for (m, n, k) on the current device:
  * exact table entry if param_map.json had one for the shape and token bucket,
- * otherwise a heuristic.  Replaces the 122-arm if-chain of kernel.cu:3022-3155;
+ * otherwise a heuristic.  tuna_matmul_cfg takes what it answers and runs the same
+ * launch.  Replaces the 122-arm if-chain of kernel.cu:3022-3155;
  * unlike it, an unknown shape is never a silent no-op. */
 int tuna_lookup_config(int m, int n, int k, tuna_config *out);
 

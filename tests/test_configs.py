@@ -5,7 +5,7 @@ import json
 
 import pytest
 
-from tuna_b200 import _lib, make_configs
+from tuna_b200 import _lib, make_configs, tuner
 
 BASELINE_SHAPES = [
     (6144, 4096), (4096, 4096), (28672, 4096), (4096, 14336),
@@ -59,6 +59,16 @@ def test_lookup_always_yields_a_runnable_config(tuna_lib, m, k, n):
         assert 1 <= cfg.warps_m * cfg.warps_k <= 16 and cfg.k_steps in (4, 8, 16, 32, 64)
     ws = tuna_lib.tuna_matmul_workspace_bytes(m, n, k)
     assert ws < (1 << 31)
+
+
+@pytest.mark.parametrize("n", [17, 25, 43, 64, 65, 100, 256, 300, 777, 4096])
+@pytest.mark.parametrize("m,k", [(6144, 4096), (512, 512), (11000, 4104), (57344, 8192)])
+def test_lookup_names_the_tile_and_is_accepted_as_a_configuration(tuna_lib, m, k, n):
+    cfg = _lib.TunaConfig()
+    assert tuna_lib.tuna_lookup_config(m, n, k, ctypes.byref(cfg)) == 0
+    assert 16 <= cfg.tile_tok <= 256 and cfg.ctas > 0 and cfg.row_blocks in (1, 2, 4)
+    assert cfg.tile_tok - 31 <= n or cfg.path != _lib.PATH_UMMA  # a tile is not wider than the tokens need
+    assert tuner.is_valid(tuna_lib, m, n, k, cfg)
 
 
 def test_table_size_matches_param_map(tuna_lib):

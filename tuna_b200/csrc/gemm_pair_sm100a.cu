@@ -670,10 +670,11 @@ struct PairPlan {
 
 static int pair_count(const tuna_config &c) { return c.ctas / 2 > 0 ? c.ctas / 2 : 1; }
 
-static PairPlan pair_plan(int m, int n, int k, const tuna_config &c)
+// of a normalized configuration
+static PairPlan pair_plan(const tuna_config &c)
 {
     PairPlan l;
-    l.tile_tok = c.tile_tok ? (c.tile_tok < 32 ? 32 : c.tile_tok) : pair_pick_tile_tok(m, n, k, pair_count(c));
+    l.tile_tok = c.tile_tok < 32 ? 32 : c.tile_tok;
     l.kc = pair_kc(l.tile_tok);
     const int slot = l.kc / 2;
     // two accumulator buffers (the epilogue of one tile overlaps the MMAs of the next) where they leave four A slots
@@ -705,10 +706,8 @@ static bool umma_fields_fit(int n, const tuna_config &c)
 
 int gemm_umma_normalize_config(int m, int n, int k, int sm_count, tuna_config *c)
 {
-    (void)m; (void)k;
-    // tile_tok 0 lets the launcher choose per token count
     const int t = c->tile_tok;
-    if (t != 0 && t != 16 && t != 32 && t != 64 && t != 128 && t != 256) return TUNA_ERR_BAD_CONFIG;
+    if (t < 0 || t > 256 || (t != 16 && t % 32 != 0)) return TUNA_ERR_BAD_CONFIG;
     if (c->row_blocks != 0 && c->row_blocks != 1 && c->row_blocks != 2 && c->row_blocks != 4) return TUNA_ERR_BAD_CONFIG;
     if (c->dequant_warps != 0 && c->dequant_warps != 8 && c->dequant_warps != 16) return TUNA_ERR_BAD_CONFIG;
     if (c->k_accs != 0 && c->k_accs != 1) return TUNA_ERR_BAD_CONFIG;
@@ -717,12 +716,18 @@ int gemm_umma_normalize_config(int m, int n, int k, int sm_count, tuna_config *c
     if (!umma_fields_fit(n, *c)) return TUNA_ERR_BAD_CONFIG;
     if (c->ctas < 0) return TUNA_ERR_BAD_CONFIG;
     if (c->ctas == 0 || c->ctas > sm_count) c->ctas = sm_count;
+    // what the launch takes, for whoever looks it up (stages follow from the token tile and stay 0)
+    if (t == 0) c->tile_tok = pair_pick_tile_tok(m, n, k, pair_count(*c));
+    if (c->row_blocks == 0) c->row_blocks = 1;
+    if (c->dequant_warps == 0) c->dequant_warps = kPairDequantWarps;
+    if (c->k_accs == 0) c->k_accs = 1;
     return TUNA_OK;
 }
 
 size_t gemm_umma_workspace_bytes(int m, int n, int k, const tuna_config &c, int sm_count)
 {
-    const PairPlan l = pair_plan(m, n, k, c);
+    (void)k;
+    const PairPlan l = pair_plan(c);
     const long long tiles = (long long)div_up(m, kPairRows) * div_up(n, l.tile_tok);
     const long long cut = tiles < sm_count ? tiles : sm_count;  // fewer than two waves of tiles are cut along K
     return partial_region_bytes(sm_count) + ((size_t)cut * 32 + 255) / 256 * 256;  // one counter per tile, CTA and TMEM lane quarter
@@ -761,7 +766,7 @@ static int launch_pair(const PairParams &p, const CUtensorMap &mq, const CUtenso
 
 int launch_gemm_umma(const GemmArgs &a, const tuna_config &c)
 {
-    const PairPlan l = pair_plan(a.m, a.n, a.k, c);
+    const PairPlan l = pair_plan(c);
     PairParams p;
     std::memset(&p, 0, sizeof(p));
     p.code = a.code; p.absmax = a.absmax; p.o = (__half *)a.o;
