@@ -5,6 +5,8 @@ import ctypes
 import re
 from pathlib import Path
 
+import pytest
+
 from tuna_b200 import _lib
 
 ROOT = Path(__file__).resolve().parents[1]
@@ -100,3 +102,19 @@ def test_bad_explicit_config_is_rejected(tuna_lib):
     assert call(path=_lib.PATH_UMMA, tile_tok=256, row_blocks=2) == -5                             # TMEM columns
     assert call(path=_lib.PATH_UMMA, tile_tok=16, dequant_warps=6) == -5
     assert call(path=7) == -5
+
+
+def test_the_largest_gemms_are_not_refused_for_their_tiles(tuna_lib):
+    """168000^3 is 127 GB of operands and 2625 chunks of 431 649 tiles: more units than 2^30, 15 million for a pair of SMs."""
+    import torch
+
+    if torch.cuda.is_available():
+        pytest.skip("addresses that only a machine without a GPU may be given")
+    buf = ctypes.create_string_buffer(256)
+    p = ctypes.c_void_p((ctypes.addressof(buf) + 63) & ~63)
+
+    def status(m, n, k):
+        return tuna_lib.tuna_matmul(p, p, p, p, p, m, n, k, p, 1 << 40, None)
+
+    assert status(168000, 168000, 168000) == -7  # no device: everything else is in order
+    assert status(1 << 20, 1 << 30, 1 << 20) == -9

@@ -778,17 +778,19 @@ int launch_gemm_umma(const GemmArgs &a, const tuna_config &c)
     p.rot_step = p.chunks * 5 / 8 | 1;
     p.stages = l.stages; p.w_stages = l.w_stages; p.nd = l.nd;
     p.ahead = a.n <= kPairAheadTokens;
-    p.status = device_status_word();
-    if (!p.status) return TUNA_ERR_NO_DEVICE;
     if (a.workspace == nullptr || a.workspace_bytes < gemm_umma_workspace_bytes(a.m, a.n, a.k, c, a.sm_count)) return TUNA_ERR_WORKSPACE;
     p.partials = (float *)a.workspace;
     p.counters = (unsigned int *)((uint8_t *)a.workspace + partial_region_bytes(a.sm_count));
 
-    const long long tiles_ll = (long long)p.row_tiles * p.tok_tiles;
-    if (tiles_ll * p.chunks >= (1ll << 30)) return TUNA_ERR_TOO_LARGE;
-    const int tiles = (int)tiles_ll;
     int pairs = pair_count(c);
     const PairSplit split = pair_split(a.m, a.n, a.k, l.tile_tok, pairs);
+    const long long tiles_ll = (long long)p.row_tiles * p.tok_tiles;
+    // the kernel numbers tiles, the units (tile, chunk) of cut tiles and a pair's units in 32 bits
+    constexpr long long kLimit = 1ll << 30;
+    if (tiles_ll >= kLimit || (long long)split.sk_tiles * p.chunks >= kLimit || (tiles_ll / pairs + 2) * p.chunks >= kLimit) return TUNA_ERR_TOO_LARGE;
+    p.status = device_status_word();
+    if (!p.status) return TUNA_ERR_NO_DEVICE;
+    const int tiles = (int)tiles_ll;
     p.sk_tiles = split.sk_tiles;
     p.sk_pairs = split.sk_pairs;
     if (p.sk_tiles) {
