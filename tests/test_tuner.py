@@ -1,10 +1,11 @@
 """Host logic of the tuner: genome handling and configuration validity, no GPU needed."""
 
+import ctypes
 import random
 
 import pytest
 
-from tuna_b200 import _lib, tuner
+from tuna_b200 import _lib, make_configs, tuner
 
 
 def test_genomes_stay_inside_the_search_space():
@@ -65,6 +66,29 @@ def test_path_is_part_of_the_search():
     assert tuner.tile_tok_for("tstream", 9) == 16 and tuner.tile_tok_for("tstream", 40) == 64
     assert tuner.tile_tok_for("tstream", 65) == 128 and tuner.tile_tok_for("tstream", 2048) == 128
     assert tuner.tile_tok_for("stream", 8) == 8 and tuner.tile_tok_for("umma", 2048) == 256
+
+
+def test_the_default_kernel_is_always_among_the_candidates(tuna_lib):
+    """What the library chooses by shape can be found by a search, with the tile it chooses itself."""
+    names = {v: k for k, v in tuner.PATH_IDS.items()}
+    for m, k in ((4096, 4096), (57344, 8192), (512, 512)):
+        for n in (1, 9, 16, 17, 24, 25, 32, 33, 64, 65, 256, 300, 2048):
+            chosen = _lib.TunaConfig()
+            assert tuna_lib.tuna_lookup_config(m, n, k, ctypes.byref(chosen)) == 0
+            assert names[chosen.path] in tuner.candidate_paths(n), n
+    genome = tuner.random_genome(random.Random(1), "umma")
+    assert tuner.to_config("umma", tuner.tile_tok_for("umma", 256), genome).tile_tok == 0
+
+
+def test_only_a_faster_configuration_becomes_an_entry():
+    umma = tuner.random_genome(random.Random(1), "umma")
+    results = [(12.0, "tstream", {"row_blocks": 1, "k_steps": 8}), (10.0, "umma", umma)]
+    entry = tuner.table_entry(32, results, 11.0)
+    assert entry["path"] == "umma" and entry["tile_tok"] == 0 and entry["us"] == 10.0
+    make_configs.validate({"4096_32_4096": entry})
+    assert tuner.table_entry(32, results, 10.0) is None  # the default is as fast
+    assert tuner.table_entry(32, results, 10.05) is None
+    assert tuner.table_entry(32, results, None)["path"] == "umma"  # the default could not be timed
 
 
 def test_tstream_validity(tuna_lib):

@@ -41,8 +41,10 @@ TSTREAM_SPACE = {
     "k_steps": (4, 8),
 }
 # The kernel for large token counts derives its tile, stages and work split from the shape
-# (gemm_pair_sm100a.cu): there is nothing to search, 0 = its own choice.
+# (gemm_pair_sm100a.cu): there is nothing to search, 0 = its own choice (the token tile too: a
+# genome's `tile_tok` takes precedence over `tile_tok_for`).
 UMMA_SPACE = {
+    "tile_tok": (0,),
     "row_blocks": (0,),
     "stages_w": (0,),
     "stages_x": (0,),
@@ -61,8 +63,10 @@ def space_for(path: str) -> dict:
 def candidate_paths(n: int) -> tuple:
     """Kernel families worth measuring for a token count: the path is part of what is tuned
     (the reference's table has one kernel and tunes its tile per bucket, kernel.cu:3022-3155)."""
-    if n <= 32:
+    if n <= 16:
         return ("tstream", "stream")
+    if n <= 32:  # the call without a configuration changes kernels inside this bucket
+        return ("tstream", "stream", "umma")
     return ("tstream", "umma")  # above 64 tokens the streaming kernel runs passes of 128 tokens
 
 
@@ -207,6 +211,19 @@ def tune_shape(m: int, n: int, k: int, path: str, generations: int, population: 
     return pop[0], fitness(pop[0])
 
 
+def table_entry(n: int, results: list, default_us: float | None) -> dict | None:
+    """The table entry of the fastest of `results` = [(us, path, genome), ...], or None where it is not
+    1 % (more than two such medians differ by) faster than the call without a configuration: an
+    entry overrides what the library chooses by shape, so it has to earn its place."""
+    us, path, best = min(results, key=lambda r: r[0])
+    if default_us is not None and us > 0.99 * default_us:
+        return None
+    note = ", ".join(f"{p_} {u:.2f} us" for u, p_, _ in sorted(results, key=lambda r: r[0]))
+    if default_us is not None:
+        note += f", without an entry {default_us:.2f} us"
+    return {"path": path, "tile_tok": tile_tok_for(path, n), **best, "us": round(us, 2), "note": note}
+
+
 def main(argv=None):
     ap = argparse.ArgumentParser(description=__doc__.split("\n")[0])
     ap.add_argument("--shapes", nargs="+", required=True, help="MxK pairs, e.g. 28672x4096")
@@ -233,11 +250,15 @@ def main(argv=None):
             if not results:
                 print(f"{m}x{k} n={n}: no valid configuration found")
                 continue
-            us, path, best = min(results, key=lambda r: r[0])
-            note = ", ".join(f"{p_} {u:.2f} us" for u, p_, _ in sorted(results, key=lambda r: r[0]))
-            pm[f"{m}_{make_configs.token_bucket(n)}_{k}"] = {"path": path, "tile_tok": tile_tok_for(path, n), **best, "us": round(us, 2),
-                                                             "note": note}
-            print(f"{m}x{k} n={n}: {path} {us:.2f} us {best}   [{note}]", flush=True)
+            default_us = bench.time_us(_lib.TunaConfig())  # all fields 0: by shape, whatever the table says
+            key = f"{m}_{make_configs.token_bucket(n)}_{k}"
+            entry = table_entry(n, results, default_us)
+            if entry is None:
+                pm.pop(key, None)
+                print(f"{m}x{k} n={n}: no entry, {min(results)[0]:.2f} us against {default_us:.2f} without", flush=True)
+            else:
+                pm[key] = entry
+                print(f"{m}x{k} n={n}: {entry['path']}   [{entry['note']}]", flush=True)
             args.param_map.write_text(json.dumps(pm, indent=1, sort_keys=True))
     make_configs.generate(args.param_map)
 
