@@ -91,6 +91,18 @@ def test_only_a_faster_configuration_becomes_an_entry():
     assert tuner.table_entry(32, results, None)["path"] == "umma"  # the default could not be timed
 
 
+def test_token_counts_of_one_bucket_are_measured_apart(tuna_lib, tmp_path):
+    class FakeBench:
+        def __init__(self, us):
+            self.us = us
+
+        def time_us(self, cfg):
+            return self.us
+
+    for n, us in ((24, 10.0), (32, 12.0)):
+        assert tuner.tune_shape(4096, n, 4096, "umma", 1, 4, 0, tmp_path / "state.json", log=lambda s: None, bench=FakeBench(us))[1] == us
+
+
 def test_tstream_validity(tuna_lib):
     ok = tuner.to_config("tstream", 16, dict(row_blocks=2, k_steps=8))
     assert tuner.is_valid(tuna_lib, 4096, 16, 4096, ok)

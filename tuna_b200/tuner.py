@@ -169,7 +169,7 @@ def tune_shape(m: int, n: int, k: int, path: str, generations: int, population: 
     lib = _lib.load()
     rng = random.Random(seed * 1000003 + m * 31 + k * 17 + n)
     tile_tok = tile_tok_for(path, n)
-    key = f"{m}_{make_configs.token_bucket(n)}_{k}"
+    key = f"{m}_{n}_{k}"  # the times of these tokens, not of another count in their bucket
     state = json.loads(state_path.read_text()) if state_path.exists() else {}
     entry = state.setdefault(f"{key}/{path}", {"measured": {}, "generation": 0, "population": []})
     bench = bench or Bench(m, n, k, seed)
