@@ -55,3 +55,91 @@ def test_weights_and_codebook_of_the_kernel_before(m, k, n, graph):
         assert torch.equal(out, ref)
     assert _lib.load().tuna_check_device_status(stream_ptr()) == 0
     assert np.isfinite(ref.float().cpu().numpy()).all()
+
+
+# (m, n, k) of GEMMs that each read their activations from the output before: both sides of every change of kernel, tiles cut
+# along K and uncut ones
+CHAIN = [(2048, 300, 512), (4096, 16, 4096), (11000, 43, 1024), (768, 16, 4096), (520, 8, 1536), (4096, 1, 4096), (8192, 100, 40), (1032, 65, 8192),
+         (4096, 24, 2048), (2048, 25, 3072), (512, 129, 264)]
+
+
+class Chain:
+    def __init__(self):
+        lib = _lib.load()
+        self.steps = []
+        need = 0
+        gen = torch.Generator(device="cuda").manual_seed(11)
+        for i, (m, n, k) in enumerate(CHAIN):
+            _, (x, q, s, c) = make_case(m, n, k, seed=40 + i)
+            s = s * (8.0 / k ** 0.5) / s.mean() / 4  # outputs of the size of the inputs
+            self.steps.append((m, n, k, q, s.contiguous(), c, torch.empty((n, m), dtype=torch.float16, device="cuda")))
+            self.x = x if i == 0 else self.x
+            need = max(need, lib.tuna_matmul_workspace_bytes(m, n, k))
+        last = self.steps[-1][-1]
+        self.w = torch.randn((1024, 2048), device="cuda", generator=gen).half() * 2048 ** -0.5
+        self.o_quantized = torch.empty((32, 1024), dtype=torch.float16, device="cuda")
+        self.x_quantized = last.view(-1)[:32 * 2048].view(32, 2048)
+        m, n, k = 256, 16, 512
+        per = [make_case(m, n, k, seed=70 + i)[1] for i in range(4)]
+        self.q4, self.s4 = torch.stack([p[1] for p in per]), torch.stack([p[2] for p in per])
+        self.o4 = torch.empty((4, n, m), dtype=torch.float16, device="cuda")
+        self.x4 = self.o_quantized.view(-1)[:4 * n * k].view(4, n, k)
+        self.code = per[0][3]
+        self.seq_out = [torch.empty((t, 512), dtype=torch.float16, device="cuda") for t in (9, 70, 33)]
+        weights = [make_case(512, 16, 64, seed=90 + i)[1] for i in range(3)]
+        flat, first, gemms = self.o4.view(-1), 0, []
+        for out, (_, q, s, c) in zip(self.seq_out, weights):
+            t = out.shape[0]
+            gemms.append((flat[first:first + t * 64].view(t, 64), q, s, out, 512, t, 64))
+            first += t * 64
+        self.ws = torch.zeros(max(need, 64 << 20), dtype=torch.uint8, device="cuda")  # one workspace for all of them
+        self.seq = tuna_b200.MatmulSequence(gemms, self.code, workspace=self.ws)
+
+    def outputs(self):
+        return [st[-1] for st in self.steps] + [self.o_quantized, self.o4] + self.seq_out
+
+    def run(self, between=lambda: None):
+        x = self.x
+        for m, n, k, q, s, c, o in self.steps:
+            tuna_b200.matmul(x.view(-1)[:n * k].view(n, k), q, s, c, o, m, n, k, workspace=self.ws)
+            between()
+            x = o
+        q, (absmax, code) = tuna_b200.quantize(self.w)  # weights, scales and codebook of the next call
+        between()
+        tuna_b200.matmul(self.x_quantized, q, absmax, code, self.o_quantized, 1024, 32, 2048, workspace=self.ws)
+        between()
+        tuna_b200.matmul_batched(self.x4, self.q4, self.s4, self.code, self.o4, 256, 16, 512, workspace=self.ws)
+        between()
+        self.seq.run()
+        between()
+
+
+def test_chain_of_dependent_calls_on_one_workspace():
+    """Calls that follow one another without a synchronisation, each reading what the one before wrote: the same bits as with one."""
+    chain = Chain()
+    for m, n, k in CHAIN[1:]:
+        i = CHAIN.index((m, n, k))
+        assert n * k <= CHAIN[i - 1][0] * CHAIN[i - 1][1]  # the output before holds that many activations
+    chain.run(torch.cuda.synchronize)
+    ref = [o.clone() for o in chain.outputs()]
+    for o in ref:
+        assert torch.isfinite(o).all() and float(o.float().std()) > 1e-3
+
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=side):
+            chain.run()
+            chain.run()
+    for run in (chain.run, lambda: (chain.run(), chain.run()), g.replay):
+        for _ in range(5):
+            torch.cuda.synchronize()
+            for o in chain.outputs():
+                o.fill_(float("nan"))
+            run()
+            torch.cuda.synchronize()
+            for o, r in zip(chain.outputs(), ref):
+                assert torch.equal(o, r)
+    assert _lib.load().tuna_check_device_status(stream_ptr()) == 0
+    assert int(chain.ws[_lib.load().tuna_workspace_scratch_bytes():].sum()) == 0
