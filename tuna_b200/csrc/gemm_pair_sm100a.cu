@@ -71,6 +71,8 @@ constexpr int kPairTokGroup = 8;            // token tiles of a wave's working s
 // 28672x4096 at 1024 163.2 -> 164.9 (graph replay).
 constexpr int kPairAheadTokens = 64;
 
+static_assert((size_t)kBlockRows * 256 * 4 <= kMaxPartialSlotBytes, "partial sums of the widest tile");
+
 struct PairParams {
     const float *code;
     const float *absmax;

@@ -882,23 +882,28 @@ static int launch_ts(const TsLaunch<MAXG> &L, int ctas, cudaStream_t stream)
 template <int MAXG>
 static int launch_ts_dispatch(const TsLaunch<MAXG> &L, int tile_tok, int steps, int ctas, cudaStream_t stream)
 {
+    // sequences: 256-column slots and up to 64 tokens only
     switch (tile_tok * 100 + steps * 10 + L.c.w_mode) {
-        case 1640: return launch_ts<16, 4, MAXG, 0>(L, ctas, stream);
-        case 1641: return launch_ts<16, 4, MAXG, 1>(L, ctas, stream);
         case 1680: return launch_ts<16, 8, MAXG, 0>(L, ctas, stream);
         case 1681: return launch_ts<16, 8, MAXG, 1>(L, ctas, stream);
-        case 3240: return launch_ts<32, 4, MAXG, 0>(L, ctas, stream);
-        case 3241: return launch_ts<32, 4, MAXG, 1>(L, ctas, stream);
         case 3280: return launch_ts<32, 8, MAXG, 0>(L, ctas, stream);
         case 3281: return launch_ts<32, 8, MAXG, 1>(L, ctas, stream);
-        case 6440: return launch_ts<64, 4, MAXG, 0>(L, ctas, stream);
-        case 6441: return launch_ts<64, 4, MAXG, 1>(L, ctas, stream);
         case 6480: return launch_ts<64, 8, MAXG, 0>(L, ctas, stream);
         case 6481: return launch_ts<64, 8, MAXG, 1>(L, ctas, stream);
-        case 12840: return launch_ts<128, 4, MAXG, 0>(L, ctas, stream);
-        case 12841: return launch_ts<128, 4, MAXG, 1>(L, ctas, stream);
-        default: return TUNA_ERR_BAD_CONFIG;
     }
+    if constexpr (MAXG == 1) {
+        switch (tile_tok * 100 + steps * 10 + L.c.w_mode) {
+            case 1640: return launch_ts<16, 4, MAXG, 0>(L, ctas, stream);
+            case 1641: return launch_ts<16, 4, MAXG, 1>(L, ctas, stream);
+            case 3240: return launch_ts<32, 4, MAXG, 0>(L, ctas, stream);
+            case 3241: return launch_ts<32, 4, MAXG, 1>(L, ctas, stream);
+            case 6440: return launch_ts<64, 4, MAXG, 0>(L, ctas, stream);
+            case 6441: return launch_ts<64, 4, MAXG, 1>(L, ctas, stream);
+            case 12840: return launch_ts<128, 4, MAXG, 0>(L, ctas, stream);
+            case 12841: return launch_ts<128, 4, MAXG, 1>(L, ctas, stream);
+        }
+    }
+    return TUNA_ERR_BAD_CONFIG;
 }
 
 // Fills the table entry of one GEMM (tensor maps, geometry); `unit0` / `tile0` are where its units

@@ -24,13 +24,15 @@ struct GemmArgs {
     size_t q_stride = 0, x_stride = 0, absmax_stride = 0, o_stride = 0;
 };
 
-// Workspace layout shared by both GEMM kernels: [split-K partial tiles: a region of fixed size]
+// Workspace layout shared by the GEMM kernels: [split-K partial tiles: a region of fixed size]
 // [arrival counters].  The partial region has the same size for every shape and configuration
-// (two slots per CTA, a slot as large as the largest tile either kernel can be configured with),
+// (two slots per CTA, a slot no smaller than the largest tile any kernel can be configured with),
 // so the counters of any call lie beyond every byte an earlier call may have written partials
 // to: one zero-initialised workspace can be shared by calls of any shapes, the counters being
 // the only part that must be zero and every call leaving them zero.
-constexpr size_t kMaxPartialSlotBytes = 192 * 1024;  // tcgen05 kernel: 128 rows x 384 accumulator columns x 4 bytes
+// A slot is 192 KB.  The largest a kernel fills is 128 KB (the pair kernel's 128 rows x 256 tokens), but the counters' place
+// behind the slots is part of the layout that callers know.
+constexpr size_t kMaxPartialSlotBytes = 192 * 1024;
 inline size_t partial_region_bytes(int sm_count) { return 2 * (size_t)sm_count * kMaxPartialSlotBytes; }
 
 struct DeviceStatus;
