@@ -66,8 +66,8 @@ def test_rejects_bad_arguments():
         tuna_b200.quantize(torch.zeros((12, 8), dtype=torch.float16, device="cuda"))
 
 
-# one CTA per row group up to 4096 columns, clusters above, the two-pass kernels beyond 112000; rows of every kind
-@pytest.mark.parametrize("m,k", [(16, 8), (32, 4088), (16, 4096), (16, 4104), (48, 10008), (8, 28672), (16, 32776), (8, 112000), (16, 112008)])
+# one CTA per row group up to 4096 columns, clusters above, the two-pass kernels beyond 111488; rows of every kind
+@pytest.mark.parametrize("m,k", [(16, 8), (32, 4088), (16, 4096), (16, 4104), (48, 10008), (8, 28672), (16, 32776), (16, 111488), (16, 111496), (8, 112000), (16, 112008)])
 @pytest.mark.parametrize("book", ["nf4", "unsorted", "close", "duplicate"])
 def test_every_share_and_codebook_is_bit_exact(m, k, book):
     rng = np.random.default_rng(m + k)

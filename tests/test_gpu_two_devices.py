@@ -11,7 +11,7 @@ from tests.gpu_util import check_parity, make_case, run_matmul, stream_ptr
 pytestmark = [pytest.mark.gpu, pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs two GPUs")]
 
 
-@pytest.mark.parametrize("n", [16, 64, 300])  # weight-streaming tcgen05 kernel, its 64-token tile, the TMA-staged kernel
+@pytest.mark.parametrize("n", [16, 64, 300])  # weight-streaming tcgen05 kernel, the pair kernel below and above 64 tokens
 def test_same_process_second_device(n):
     m, k = 1024, 2048
     for dev in (0, 1, 0):

@@ -1,4 +1,5 @@
-"""The tcgen05/TMEM kernel against the oracle, through the C ABI, with explicit configurations."""
+"""The tcgen05 kernel for large token counts against the oracle, through the C ABI, with explicit configurations.  Of their
+fields the token tile and the CTA count steer it; row blocks are accepted and run the same launch."""
 
 import ctypes
 

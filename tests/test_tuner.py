@@ -56,7 +56,7 @@ def test_config_fields_round_trip():
     cfg = tuner.to_config("umma", 64, dict(row_blocks=2, stages_w=6, stages_x=4, stages_a=8, dequant_warps=8, k_accs=1))
     d = cfg.as_dict()
     assert d["path"] == _lib.PATH_UMMA and d["tile_tok"] == 64 and d["row_blocks"] == 2 and d["k_accs"] == 1
-    assert all(v == (0,) for v in tuner.UMMA_SPACE.values())  # the TMA-staged kernel: defaults only
+    assert all(v == (0,) for v in tuner.UMMA_SPACE.values())  # the pair kernel: its own choices only
 
 
 def test_path_is_part_of_the_search():

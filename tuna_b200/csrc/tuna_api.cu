@@ -100,7 +100,8 @@ static int launch_gemm(const GemmArgs &a, const tuna_config &c)
 }
 
 // Whether equal-shape GEMMs share persistent launches of the sequence kernel: every token count it
-// takes (eight 4096x14336 GEMMs of 16 tokens: 132 us as a launch each, 66 as one).
+// takes (us as launches of the sequence kernel / as calls on the kernel each would take alone: eight 4096x14336 of 16
+// tokens 61 / 129, of 64 91 / 157; eight 28672x4096 of 64 170 / 199; two 57344x8192 of 16 110 / 127, but of 64 168 / 148).
 static bool batched_as_sequence(const tuna_config &c, int n) { return c.path != TUNA_PATH_STREAM && n <= 64; }
 
 }  // namespace tuna

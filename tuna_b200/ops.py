@@ -112,7 +112,7 @@ def matmul(x, q, s, c, o, m: int, n: int, k: int, *, config: TunaConfig | None =
 
 
 def matmul_batched(x, q, s, c, o, m: int, n: int, k: int, *, workspace=None) -> None:
-    """`batch` independent GEMMs of one shape in one call (one launch for n <= 32):
+    """`batch` independent GEMMs of one shape in one call (one launch per 64 matrices for n <= 64):
     `q` uint8 `[batch, m/8, k/8, 32]`, `s` fp32 `[batch, m]`, `o` fp16 `[batch, n, m]`, and `x` fp16
     either `[batch, n, k]` (per-matrix activations, e.g. one token list per expert) or `[n, k]`
     (shared: the reference's "combined" Mixtral GEMM, make_configs.py:105-106)."""
