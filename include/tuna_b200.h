@@ -53,7 +53,8 @@ typedef enum tuna_path {
 
 /* Launch configuration, the Blackwell counterpart of the reference's
  * KernelConfig (configs.cu:12-54).  Produced by the shape table generated from
- * param_map.json, or filled by hand (tuner, tests).  Zero means "default". */
+ * param_map.json, or filled by hand (tuner, tests).  Zero means "default": all zero is
+ * tuna_matmul's choice by shape; fields without a path are tstream's up to 64 tokens, umma's above. */
 typedef struct tuna_config {
     int32_t path;          /* tuna_path                                               */
     int32_t tile_tok;      /* tokens per pass: stream 8|16|32; tstream 16|32|64|128;  *

@@ -52,6 +52,15 @@ def test_umma_fields_that_do_not_fit_one_sm_are_refused(tuna_lib, n, tile_tok, f
     assert tuner.is_valid(tuna_lib, 4096, n, 4096, tuner.to_config("umma", tile_tok, fields)) == fits
 
 
+@pytest.mark.parametrize("n", [16, 25, 40, 64])
+def test_fields_without_a_kernel_mean_the_weight_streaming_one(tuna_lib, n):
+    """Up to 64 tokens: its own fields steer it, those of the other kernels do not count."""
+    for fields, fits in ((dict(row_blocks=1, k_steps=8), True), (dict(row_blocks=1, k_steps=16), False), (dict(row_blocks=4, tile_tok=32), False),
+                         (dict(row_blocks=1, k_accs=2), True), (dict(dequant_warps=4), True), (dict(stages_w=3), True)):
+        assert tuner.is_valid(tuna_lib, 4096, n, 4096, _lib.TunaConfig(**fields)) == fits, fields
+    assert tuner.is_valid(tuna_lib, 4096, n, 4096, _lib.TunaConfig())
+
+
 def test_config_fields_round_trip():
     cfg = tuner.to_config("umma", 64, dict(row_blocks=2, stages_w=6, stages_x=4, stages_a=8, dequant_warps=8, k_accs=1))
     d = cfg.as_dict()

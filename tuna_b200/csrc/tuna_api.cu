@@ -49,6 +49,7 @@ static int device_sm_count()
 }
 
 constexpr int kStreamTokens = 24;
+constexpr int kStreamPassTokens = 64;  // where a configuration that names fields but no kernel changes kernels: its fields are that kernel's
 
 static int resolve_config(int m, int n, int k, int sm_count, const tuna_config *user, tuna_config *out)
 {
@@ -65,7 +66,11 @@ static int resolve_config(int m, int n, int k, int sm_count, const tuna_config *
     // kernel on CTA pairs above, which stages half of the tokens per SM.  Measured (us, weight streaming / pairs):
     // 57344x8192 at 64 tokens 95 / 74, at 32 69 / 69, at 16 62 / 67; 14336x4096 at 32 17.3 / 15.4, 2048x2048 at 32
     // 7.2 / 6.2; 4096x4096 at 43 11.1 / 10.9, at 32 10.0 / 10.0, at 24 9.3 / 10.1; 28672x4096 at 32 26.9 / 26.5, at 24 25.3 / 26.5.
-    if (c.path == TUNA_PATH_AUTO) c.path = (n <= kStreamTokens) ? TUNA_PATH_TSTREAM : TUNA_PATH_UMMA;
+    if (c.path == TUNA_PATH_AUTO) {
+        const tuna_config none = {};
+        const bool by_shape = !user || std::memcmp(user, &none, sizeof(none)) == 0;
+        c.path = n <= (by_shape ? kStreamTokens : kStreamPassTokens) ? TUNA_PATH_TSTREAM : TUNA_PATH_UMMA;
+    }
     int st;
     if (c.path == TUNA_PATH_STREAM) st = gemm_stream_normalize_config(m, n, k, sm_count, &c);
     else if (c.path == TUNA_PATH_UMMA) st = gemm_umma_normalize_config(m, n, k, sm_count, &c);
