@@ -386,8 +386,21 @@ __global__ void __launch_bounds__(256) quantize_pack_kernel(const __half *__rest
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const __half2 h = *reinterpret_cast<const __half2 *>(&u[i]);
-            // even column in the high nibble
-            word |= ((nearest_code(__low2float(h), scale, cb) << 4) | nearest_code(__high2float(h), scale, cb)) << (8 * i);
+            // nearest_code of both columns side by side: 32 registers; by two calls of it 41 (1024x120000: 503 us against 650)
+            const float x[2] = {__fdiv_rn(__low2float(h), scale), __fdiv_rn(__high2float(h), scale)};
+            uint32_t nib[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                float best = fabsf(x[e] - cb[0]);
+                uint32_t idx = 0;
+#pragma unroll
+                for (int c = 1; c < 16; ++c) {
+                    const float d = fabsf(x[e] - cb[c]);
+                    if (d < best) { best = d; idx = c; }
+                }
+                nib[e] = idx;
+            }
+            word |= ((nib[0] << 4) | nib[1]) << (8 * i);  // even column in the high nibble
         }
         *reinterpret_cast<uint32_t *>(q + (size_t)rg * row_group_bytes(k) + (size_t)kt * 32 + r * 4) = word;
     }
