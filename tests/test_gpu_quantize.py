@@ -91,6 +91,22 @@ def test_every_share_and_codebook_is_bit_exact(m, k, book):
     assert np.array_equal(q.cpu().numpy(), q_ref)
 
 
+@pytest.mark.parametrize("m,k", [(2048, 8), (4096, 8), (4096, 64), (4096, 136), (8192, 128), (8192, 256)])
+@pytest.mark.parametrize("book", ["nf4", "unsorted"])
+def test_narrow_rows_on_both_sides_of_the_two_pass_line(m, k, book):
+    rng = np.random.default_rng(m + k)
+    w = (rng.standard_normal((m, k)) * 0.05).astype(np.float16)
+    w[1] = 0
+    w[2] *= np.float16(1e-3)
+    w[3] = rng.integers(-8, 9, k) / 8
+    code = orc.NF4_CODE if book == "nf4" else np.ascontiguousarray(np.roll(orc.NF4_CODE, 5))
+    q, (absmax, c) = tuna_b200.quantize(torch.from_numpy(w).cuda(), None if book == "nf4" else torch.from_numpy(code).cuda())
+    q_ref, a_ref, _ = orc.quantize_blockwise_dynamic_4bit(w, code)
+    assert np.array_equal(c.cpu().numpy(), code)
+    assert np.array_equal(absmax.cpu().numpy(), a_ref)
+    assert np.array_equal(q.cpu().numpy(), q_ref)
+
+
 def test_widest_single_pass_rows():
     """The widest rows whose staged share and tables fit a CTA of the largest cluster; 8 columns more take two passes."""
     for k in (111488, 111496):

@@ -323,7 +323,8 @@ __global__ void __launch_bounds__(kQuantThreads) quantize_rows_kernel(const __ha
     }
 }
 
-// ---- rows too wide for a cluster's shared memory (k > 111488): two passes over memory, the literal expression
+// ---- rows too wide for a cluster's shared memory (k > 111488), and many narrow rows (quantize_in_two_passes): two passes
+// over memory, the literal expression
 
 __global__ void __launch_bounds__(256) row_absmax_kernel(const __half *__restrict__ w, float *__restrict__ absmax, int m, int k)
 {
@@ -386,7 +387,7 @@ __global__ void __launch_bounds__(256) quantize_pack_kernel(const __half *__rest
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const __half2 h = *reinterpret_cast<const __half2 *>(&u[i]);
-            // nearest_code of both columns side by side: 32 registers; by two calls of it 41 (1024x120000: 503 us against 650)
+            // nearest_code of both columns side by side: 32 registers; by two calls of it 41 (1024x120000: 503 us against 609)
             const float x[2] = {__fdiv_rn(__low2float(h), scale), __fdiv_rn(__high2float(h), scale)};
             uint32_t nib[2];
 #pragma unroll
@@ -406,13 +407,23 @@ __global__ void __launch_bounds__(256) quantize_pack_kernel(const __half *__rest
     }
 }
 
+// Whether two passes are the faster way.  A CTA of the single pass spends ~3 us on its row group before the first code,
+// whatever the width; on narrow rows the literal expression is done with them sooner.  The estimates (us) are fitted to 8 to
+// 229376 rows of 8 to 512 columns; two passes / one: 57344x8 17.7 / 51.0, 57344x128 33.3 / 52.3, 57344x256 55.0 / 55.3, 8192x64
+// 7.2 / 9.5, 4096x128 6.6 / 6.2, 2048x64 4.7 / 4.6.
+static bool quantize_in_two_passes(int m, int k, int sm_count)
+{
+    const double groups_per_sm = (m / 8) / (double)sm_count;
+    return 4.6 + groups_per_sm * (0.15 + 0.00355 * k) < 2.6 + groups_per_sm / 3 * (3.0 + 0.001 * k);
+}
+
 cudaError_t launch_quantize(const void *w, const void *code, void *code_out, void *q, void *absmax, int m, int k, int sm_count,
                             cudaStream_t stream)
 {
     const int want = div_up(k, kQuantShareCols);
     const int cluster0 = want < kQuantMaxCluster ? want : kQuantMaxCluster;
     const int share = div_up(k / 8, cluster0) * 8;
-    if (share > kQuantMaxShareCols) {
+    if (share > kQuantMaxShareCols || quantize_in_two_passes(m, k, sm_count)) {
         const int blocks = sm_count * 8;
         row_absmax_kernel<<<blocks, 256, 0, stream>>>((const __half *)w, (float *)absmax, m, k);
         quantize_pack_kernel<<<blocks, 256, 0, stream>>>((const __half *)w, (const float *)code, (float *)code_out,
