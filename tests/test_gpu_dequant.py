@@ -1,5 +1,5 @@
 """tuna_dequant where its work split can go wrong: row groups cut across warps, warps that walk several row groups,
-passes that end inside a row."""
+passes that end inside a row; small matrices and narrow rows."""
 
 import numpy as np
 import pytest
@@ -12,7 +12,9 @@ from tuna_b200 import _lib
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("m,k", [(40000, 264), (8, 40008), (32, 8200), (33328, 256), (30016, 520)])
+@pytest.mark.parametrize("m,k", [(40000, 264), (8, 40008), (32, 8200), (33328, 256), (30016, 520),
+                                 # both sides of the line between the two kernels, and the smallest and narrowest
+                                 (8, 131072), (8, 131080), (32, 40008), (4096, 256), (4104, 256), (57344, 128), (57344, 136), (57344, 8), (8, 8), (520, 136)])
 def test_dequant_work_split_is_exact(m, k):
     lib = _lib.load()
     (x, q, absmax, code), (xd, qd, sd, cd) = make_case(m, 1, k, seed=m + k)

@@ -87,9 +87,58 @@ dequant_w4_kernel(const uint8_t *__restrict__ q, const float *__restrict__ absma
     }
 }
 
+// Small matrices and narrow rows, where a warp has hardly more to do than to build its tables: they stay in shared memory,
+// one entry looked up per weight, and a warp's share is as little as 128 columns of one row group.
+__global__ void __launch_bounds__(kDqWarps * 32)
+dequant_lookup_kernel(const uint8_t *__restrict__ q, const float *__restrict__ absmax, const float *__restrict__ code,
+                      __half *__restrict__ out, int m, int k, int tiles_per_warp)
+{
+    __shared__ __align__(16) __half lut[kDqWarps][8][kCodeSize];
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rg = blockIdx.x * kDqWarps + warp;
+    if (rg >= (m >> 3)) return;
+    for (int e = lane; e < 8 * kCodeSize; e += 32)
+        lut[warp][e >> 4][e & 15] = __float2half_rn(code[e & 15] * absmax[rg * 8 + (e >> 4)]);
+    __syncwarp();
+
+    const int kt_end = min(k >> 3, ((int)blockIdx.y + 1) * tiles_per_warp);
+    const int half_sel = lane & 1;  // which 4 rows of the tile this lane holds
+    const uint8_t *src = q + (size_t)rg * row_group_bytes(k) + half_sel * 16;
+    const __half(*table)[kCodeSize] = &lut[warp][half_sel * 4];
+    __half *dst_rows = out + (size_t)(rg * 8 + half_sel * 4) * k;
+    for (int kt = (int)blockIdx.y * tiles_per_warp + (lane >> 1); kt < kt_end; kt += 16) {
+        const uint4 v = ldg_stream_u4(src + (size_t)kt * 32);
+        const uint32_t words[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            uint32_t o[4];
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {  // even column: high nibble
+                const uint32_t byte = (words[i] >> (8 * b)) & 0xffu;
+                o[b] = (uint32_t)__half_as_ushort(table[i][byte >> 4]) | ((uint32_t)__half_as_ushort(table[i][byte & 15]) << 16);
+            }
+            *reinterpret_cast<uint4 *>(dst_rows + (size_t)i * k + (size_t)kt * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+        }
+    }
+}
+
+// Measured (graph replay, us, lookups in shared memory / tables in registers): 57344x8 4.0 / 5.5, 57344x128 5.2 / 5.6, 57344x160 7.4 / 7.1;
+// 8x4096 2.1 / 2.6, 512x512 2.3 / 2.5, 4096x256 2.3 / 2.5, 4096x384 2.8 / 2.5, 6144x160 2.7 / 2.5.
+static bool dequant_by_lookup(int m, int k) { return k <= 128 || (m <= 4096 && (long long)m * k <= 1 << 20); }
+
 cudaError_t launch_dequant(const void *q, const void *absmax, const void *code, void *o, int m,
                            int k, int sm_count, cudaStream_t stream)
 {
+    if (dequant_by_lookup(m, k)) {
+        const int tiles = k / 8, gx = div_up(m / 8, kDqWarps);
+        // eight CTAs per SM if the columns give as many, a whole number of warp passes (16 tiles) each
+        const int wanted = std::max(1, std::min(div_up(sm_count * 8, gx), div_up(tiles, 16)));
+        const int per_warp = div_up(div_up(tiles, wanted), 16) * 16;
+        dequant_lookup_kernel<<<dim3(gx, div_up(tiles, per_warp)), kDqWarps * 32, 0, stream>>>(
+            (const uint8_t *)q, (const float *)absmax, (const float *)code, (__half *)o, m, k, per_warp);
+        return cudaGetLastError();
+    }
     const int items = (m / 8) * div_up(k / 8, 16 * kDqUnroll);  // below 2^31: m * k <= 2^41
     const int grid = std::min(sm_count * kDqCtasPerSm * kDqWaves, div_up(items, kDqWarps));
     const int warps = grid * kDqWarps;
