@@ -143,3 +143,64 @@ def test_chain_of_dependent_calls_on_one_workspace():
                 assert torch.equal(o, r)
     assert _lib.load().tuna_check_device_status(stream_ptr()) == 0
     assert int(chain.ws[_lib.load().tuna_workspace_scratch_bytes():].sum()) == 0
+
+
+# Takes SMs away for a while: its shared memory leaves no room for another CTA beside it.
+OCCUPIER = """
+extern "C" __global__ void occupier(long long *out, int clocks)
+{
+    extern __shared__ unsigned char smem[];
+    const long long t0 = clock64();
+    while (clock64() - t0 < clocks) { }
+    if (threadIdx.x == 0) { smem[0] = 1; out[blockIdx.x] = clock64() - t0 + smem[0]; }
+}
+"""
+
+
+def _late_start_calls(kind):
+    if kind == "sequence" or kind == "reduce":
+        shapes = [(1032, 8, 520), (520, 16, 2048), (264, 5, 1000), (1024, 16, 512)] * 6
+    else:
+        shapes = [(4096, 16, 4096), (520, 3, 8192), (1024, 24, 2048), (2048, 50, 1024), (512, 200, 4096)]
+    gemms = []
+    for i, (m, n, k) in enumerate(shapes):
+        _, (x, q, s, c) = make_case(m, n, k, seed=200 + i)
+        gemms.append((x, q, s, torch.empty((n, m), dtype=torch.float16, device="cuda"), m, n, k))
+    if kind == "matmul":
+        def run():
+            for x, q, s, o, m, n, k in gemms:
+                tuna_b200.matmul(x, q, s, c, o, m, n, k)
+    elif kind == "sequence":
+        run = tuna_b200.MatmulSequence(gemms, c).run
+    else:
+        exchange = tuna_b200.Exchange(tuna_b200.ReduceSequence.exchange_bytes([g[4:] for g in gemms], 1), "cuda:0")
+        run = tuna_b200.ReduceSequence(gemms, c, exchange).run
+    return run, [g[3] for g in gemms]
+
+
+@pytest.mark.parametrize("kind", ["matmul", "sequence", "reduce"])
+def test_ctas_that_start_late(kind):
+    """With all but a few SMs taken, CTAs that share a tile run one after another instead of side by side, so the one that
+    arrives last - and adds the partial sums up - is another one than usual: the same bits."""
+    occupier = torch.cuda._compile_kernel(OCCUPIER, "occupier")
+    occupier.set_shared_memory_config(200 << 10)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    times = torch.zeros(sms, dtype=torch.int64, device="cuda")
+    work, side = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(work):
+        run, outs = _late_start_calls(kind)
+        run()
+        torch.cuda.synchronize()
+        ref = [o.clone() for o in outs]
+        for free in (2, 10, 74):
+            for o in outs:
+                o.fill_(float("nan"))
+            torch.cuda.synchronize()
+            with torch.cuda.stream(side):
+                occupier(grid=(sms - free, 1, 1), block=(32, 1, 1), args=[times, 1000000], shared_mem=200 << 10)
+            run()
+            torch.cuda.synchronize()
+            for o, r in zip(outs, ref):
+                assert torch.equal(o, r)
+        assert _lib.load().tuna_check_device_status(work.cuda_stream) == 0

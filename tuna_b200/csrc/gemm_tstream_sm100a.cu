@@ -268,8 +268,9 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_w4a16_tstream_kernel(const
     __shared__ __align__(8) uint64_t bars[2 * kTsMaxASlots + 2 * kTsMaxXStages + 4 + 2 * kTsMaxWStages];
     __shared__ uint32_t s_tmem_base;
     __shared__ int s_abort;
-    __shared__ int s_fix[4];   // quarters of the CTA's last tile that this CTA finishes
-    __shared__ int s_last[4];  // its GEMM, tile, first CTA and segments
+    // The cut tiles of the CTA's range, at most its first [0] and its last [1], that this CTA finishes at its end
+    __shared__ int s_fix[2][4];   // by quarter
+    __shared__ int s_tile[2][4];  // GEMM, tile, first CTA and segments
 
     TS_PROF_DECL
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
@@ -317,7 +318,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_w4a16_tstream_kernel(const
 
     if (threadIdx.x == 0) {
         s_abort = 0;
-        s_fix[0] = s_fix[1] = s_fix[2] = s_fix[3] = 0;
+        for (int i = 0; i < 8; ++i) s_fix[i >> 2][i & 3] = 0;
         for (int i = 0; i < kTsMaxASlots; ++i) { mbar_init(a_full + 8 * i, 4 * kHalves); mbar_init(a_empty + 8 * i, 1); }
         for (int i = 0; i < kTsMaxXStages; ++i) { mbar_init(x_full + 8 * i, 1); mbar_init(x_empty + 8 * i, 1); }
         for (int i = 0; i < 2; ++i) { mbar_init(d_full + 8 * i, 1); mbar_init(d_empty + 8 * i, 4); }
@@ -423,12 +424,12 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_w4a16_tstream_kernel(const
     // The flagged quarters of a tile whose partials are all there, shared out over warps `w0`, w0 + step, ... : a warp
     // takes four tokens of 32 rows at a time (small code: it runs once per CTA, out of a cold instruction cache),
     // in exchange launches 16, whole sectors of a peer's slab.
-    auto finish_tile = [&](const TsGemm &G, int tile, int first, int nseg, int w0, int step, auto flagged) __attribute__((always_inline)) {
+    auto finish_tile = [&](const TsGemm &G, int tile, int first, int nseg, const int *flagged, int w0, int step) __attribute__((always_inline)) {
         const int groups4 = token_groups(G), per = p.n_peers > 0 ? 4 : 1, rb_shift = RB >> 1;
         for (int item = w0; item * per < 4 * RB * groups4; item += step) {
             const int q = item & 3, rest = item >> 2;
             const int g = rest >> rb_shift, rb = rest & (RB - 1);  // RB is 1, 2 or 4
-            if (!flagged(q)) continue;
+            if (!flagged[q]) continue;
             if (per == 1) add_partials(Int<1>(), Int<4>(), G, tile, first, nseg, q, rb, g);
             else add_partials(Int<4>(), Int<2>(), G, tile, first, nseg, q, rb, 4 * g);
         }
@@ -609,8 +610,8 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_w4a16_tstream_kernel(const
             if (lane == 0) mbar_arrive(d_empty + 8 * rd.idx);
             if (!full) {
                 // Each epilogue warp arrives for its own 32 lanes at the counter of (tile, quarter).  Whoever arrives
-                // last has all the partials: in the middle of the range the warp adds them up itself, at its end - where
-                // nearly all the cut tiles are finished, and nothing else is left to do - all warps of the CTA do.
+                // last has all the partials; its CTA adds them up at the end of its range, with all its warps.  That is
+                // the CTA whose range ends with the tile, unless the tile's other CTA started late.
                 // lane 0's atomic releases the warp's partials and acquires the others'
                 __syncwarp();
                 const int first = first_cta(G, tile), nseg = last_cta(G, tile) - first + 1;
@@ -620,11 +621,11 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_w4a16_tstream_kernel(const
                 old = __shfl_sync(0xffffffffu, old, 0);
                 if (old == (unsigned)nseg - 1) {
                     if (lane == 0) *counter = 0;  // leave the counter clean for the next call
-                    if (u + (c1 - c0) < n_units) finish_tile(G, tile, first, nseg, quarter, 4, [](int) { return true; });
-                    else if (lane == 0) {
-                        s_fix[quarter] = 1;
+                    if (lane == 0) {
+                        const int e = u + (c1 - c0) < n_units ? 0 : 1;
+                        s_fix[e][quarter] = 1;
                         // the same values from every flagged quarter
-                        s_last[0] = cur.g; s_last[1] = tile; s_last[2] = first; s_last[3] = nseg;
+                        s_tile[e][0] = cur.g; s_tile[e][1] = tile; s_tile[e][2] = first; s_tile[e][3] = nseg;
                     }
                 }
             }
@@ -754,8 +755,15 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_w4a16_tstream_kernel(const
     TS_PROF_MARK(2)
     tc_fence_before();
     __syncthreads();
-    if (s_fix[0] | s_fix[1] | s_fix[2] | s_fix[3]) {
-        finish_tile(L.g[s_last[0]], s_last[1], s_last[2], s_last[3], warp, kTsThreads / 32, [&](int q) { return s_fix[q] != 0; });
+    {
+        // One copy of that code, outside any loop: half of the warps take the first tile where there is one.  A second copy in the
+        // epilogue, for first tiles, or a loop over the two here took registers and instruction cache from the roles above
+        // (us with the copy / the loop / as it is: 28672x4096 at 16 tokens 22.6 / 20.2 / 20.0, 57344x64 at 5 8.0 / 6.7 / 6.7,
+        // 64 GEMMs of 1032x520 at 8 23.9 / 27.1 / 22.4, 47 of 4096x4096 at 16 95 / 83 / 82).
+        const bool first = (s_fix[0][0] | s_fix[0][1] | s_fix[0][2] | s_fix[0][3]) != 0;
+        const int e = first ? warp & 1 : 1;
+        if (s_fix[e][0] | s_fix[e][1] | s_fix[e][2] | s_fix[e][3])
+            finish_tile(L.g[s_tile[e][0]], s_tile[e][1], s_tile[e][2], s_tile[e][3], s_fix[e], first ? warp >> 1 : warp, first ? kTsThreads / 64 : kTsThreads / 32);
     }
     if (warp < kTsDequantWarp0) { TS_PROF_MARK(3) }
     TS_PROF_STORE
