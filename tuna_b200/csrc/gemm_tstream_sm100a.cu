@@ -59,7 +59,8 @@
 // tokens the last MMA was done at 16.7 us of 24.1.  Hence only token groups that exist are exchanged, one
 // acquire-release atomic per warp replaces two fences, and at the end of the range all 24 warps add up the tile, four
 // tokens of 32 rows each, instead of four warps 16 tokens at a time (graph replay, 16 tokens unless said, us):
-// 4096x4096 10.3 -> 9.9, 57344x8192 67.0 -> 65.2, 4096x4096 at 64 tokens 20.1 -> 14.2, 768x4096 at 64 49.7 -> 12.9.
+// 4096x4096 10.3 -> 9.9, 57344x8192 67.0 -> 65.2, 4096x4096 at 64 tokens 20.1 -> 14.2, 768x4096 at 64 49.7 -> 12.9; with that
+// code in one place only, outside the roles, 4096x4096 7.8, 57344x8192 53.5, 4096x4096 at 64 10.9.
 //
 // Programmatic dependent launch: the kernel lets its successor start as SMs free up and itself waits for its predecessors
 // only before it touches what they may have written (activations, workspace, output); the weights and the
@@ -782,8 +783,9 @@ static int ts_steps(const tuna_config &c) { return c.k_steps == 4 ? 4 : 8; }
 // 128 x 256 slot takes 0.66 us, less where row blocks share its activations.  What comes on top depends on how the
 // tiles are cut: not at all, into whole segments per tile, or anywhere (every CTA the same number of units); the partial
 // sums of a cut tile cost by tokens and row blocks.  The constants are fitted to launches of 512x512 to
-// 57344x8192 at 1 to 32 tokens; examples (us): 4096x4096 at 16 tokens 128 CTAs 8.8, 148 10.0; 4096x14336 two row blocks
-// and 128 CTAs 15.6, one and 148 17.9; 14336x4096 one row block uncut 16.4, 148 CTAs 17.2; 57344x8192 four, two, one: 62, 65, 72.
+// 57344x8192 at 1 to 32 tokens; examples (us) at 16 tokens: 4096x4096 128 CTAs 7.8, 148 8.7; 4096x14336 two row blocks
+// and 128 CTAs 13.8, two and 148 15.9, one and 148 14.5; 28672x4096 two row blocks and 148 CTAs 19.8, two and 112 21.0, one and
+// 148 20.6; 57344x8192 four, two, one on 148 CTAs: 52.4, 52.1, 59.9.
 static void ts_pick_split(int m, int n, int k, int sm_count, tuna_config *c)
 {
     const int chunks = div_up(k, 32 * ts_steps(*c));

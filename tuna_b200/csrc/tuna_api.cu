@@ -64,8 +64,10 @@ static int resolve_config(int m, int n, int k, int sm_count, const tuna_config *
     }
     // No table entry: the tcgen05 weight-streaming kernel up to 24 tokens (the regime bound by HBM), the
     // kernel on CTA pairs above, which stages half of the tokens per SM.  Measured (us, weight streaming / pairs):
-    // 57344x8192 at 64 tokens 95 / 74, at 32 69 / 69, at 16 62 / 67; 14336x4096 at 32 17.3 / 15.4, 2048x2048 at 32
-    // 7.2 / 6.2; 4096x4096 at 43 11.1 / 10.9, at 32 10.0 / 10.0, at 24 9.3 / 10.1; 28672x4096 at 32 26.9 / 26.5, at 24 25.3 / 26.5.
+    // 57344x8192 at 64 tokens 83 / 73, at 32 57 / 67, at 16 54 / 66; 28672x4096 at 64 28.0 / 25.3, at 32 23.2 / 24.8, at 24 21.0 / 24.5;
+    // 4096x4096 at 64 10.9 / 10.7, at 32 8.9 / 9.8; 14336x4096 at 32 15.2 / 14.7, at 24 14.5 / 14.7; 11000x4104 at 32 15.1 / 13.9,
+    // at 24 13.5 / 13.9; 2048x2048 at 32 6.5 / 6.2; 512x512 at 32 4.0 / 3.5, at 24 4.0 / 3.5.  Between 25 and 32 tokens either
+    // leads by up to 15 %, by the shape: the line is where nothing that ran on the pair kernel gets slower.
     if (c.path == TUNA_PATH_AUTO) {
         const tuna_config none = {};
         const bool by_shape = !user || std::memcmp(user, &none, sizeof(none)) == 0;
@@ -106,7 +108,7 @@ static int launch_gemm(const GemmArgs &a, const tuna_config &c)
 
 // Whether equal-shape GEMMs share persistent launches of the sequence kernel: every token count it
 // takes (us as launches of the sequence kernel / as calls on the kernel each would take alone: eight 4096x14336 of 16
-// tokens 61 / 129, of 64 91 / 157; eight 28672x4096 of 64 170 / 199; two 57344x8192 of 16 110 / 127, but of 64 168 / 148).
+// tokens 53 / 115, of 64 83 / 152; eight 28672x4096 of 64 164 / 197; two 57344x8192 of 16 94 / 112, but of 64 161 / 147).
 static bool batched_as_sequence(const tuna_config &c, int n) { return c.path != TUNA_PATH_STREAM && n <= 64; }
 
 }  // namespace tuna
