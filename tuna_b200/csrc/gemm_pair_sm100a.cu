@@ -67,10 +67,11 @@ constexpr int kPairMaxStages = 8;           // unit stages: activations in share
 constexpr int kPairMaxWStages = 8;
 constexpr int kPairSmemDynamic = 226 * 1024;
 constexpr int kPairTokGroup = 8;            // token tiles of a wave's working set
-// Up to here weights and codebook are read ahead of the dependency wait, as the weight-streaming kernels do (the header's
-// contract); more tokens see ordinary stream order.  Reading ahead hides the pipeline's fill: 11000x4104 at 43 tokens
-// 14.7 us against 17.1, 28672x4096 at 64 25.7 / 28.1; what ordinary order costs above: 6144x4096 at 256 16.6 -> 17.6,
-// 28672x4096 at 1024 163.2 -> 164.9 (graph replay).
+// Up to here weights and codebook are taken from ahead of the dependency wait, as the weight-streaming kernels do (the
+// header's contract); more tokens see ordinary stream order.  There the weights are read after the wait, and the lookup table
+// is still built before it, from a copy of the codebook that is compared with the codebook after it.  Graph replay, us,
+// all ahead / so / all after the wait: 512x512 at 100 tokens 3.4 / 3.9 / 5.5, 6144x4096 at 256 16.4 / 16.1 / 17.4, 28672x4096 at
+// 1024 167 / 167 / 168; below the line 2048x2048 at 48 6.1 / 7.8, 28672x4096 at 64 25.4 / 25.7.
 constexpr int kPairAheadTokens = 64;
 
 static_assert((size_t)kBlockRows * 256 * 4 <= kMaxPartialSlotBytes, "partial sums of the widest tile");
@@ -90,7 +91,7 @@ struct PairParams {
     int stages;       // unit stages
     int w_stages;
     int nd;           // accumulator buffers
-    int ahead;        // weights and codebook are read before the dependency wait
+    int ahead;        // weights and codebook are taken from before the dependency wait
     int q3d;          // the weights' tensor map is the 3-D view (WMODE 0)
     int sk_tiles;     // tiles 0 .. sk_tiles - 1 are cut along K over pairs 0 .. sk_pairs - 1 ...
     int sk_pairs;
@@ -188,6 +189,7 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
     __shared__ __align__(8) uint64_t bars[3 * kPairMaxStages + 2 * kPairMaxWStages + 4];
     __shared__ uint32_t s_tmem_base;
     __shared__ int s_abort;
+    __shared__ float s_code[16];  // the codebook as it was before the dependency wait
     __shared__ int s_fix[4];   // quarters this CTA finishes with all its warps at the end
 
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
@@ -228,29 +230,32 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
+    if (!p.ahead && threadIdx.x >= 64 && threadIdx.x < 80) s_code[threadIdx.x - 64] = p.code[threadIdx.x - 64];
     __syncthreads();  // this CTA's barriers are initialised: its weight producer may start
 
     // What a kernel before this one wrote is there only after this wait: its end alone, or its letting dependents start, is no
-    // promise.  The copies of x and the epilogue always wait; weights and codebook are read ahead of it (the dequant
-    // warps fill the A slots meanwhile) up to kPairAheadTokens only.
+    // promise.  The copies of x and the epilogue always wait; up to kPairAheadTokens the weights are copied ahead of it, and
+    // the dequant warps fill the A slots meanwhile.
     auto depend = [] { asm volatile("griddepcontrol.wait;" ::: "memory"); };
-    if (!p.ahead) depend();
 
     PairSegs segs;
     segs.init(p, pair, pairs);
     const int total = segs.total_units(p);
 
-    // Rest of the prologue, run by every warp inside its own role's branch: the byte -> half2 table (even
-    // column = high nibble in the low half), then the barrier of the pair, which publishes both CTAs' barriers and tables.
-    // depend() comes after it in every role that needs it, and in whoever is about to make a bounded wait that
-    // ends only after the kernels before this one.
-    auto finish_prologue = [&]() -> uint32_t {
-        const float cv = p.code[lane & 15];
+    // The byte -> half2 table (even column = high nibble in the low half), its entries shared out over `step` warps.
+    auto build_table = [&](float cv, int first, int step) {
         const uint32_t ch = (uint32_t)__half_as_ushort(__float2half_rn(cv));
-        for (int e = warp; e < 256; e += kPairWarps) {
+        for (int e = first; e < 256; e += step) {
             const uint32_t v = __shfl_sync(0xffffffffu, ch, e >> 4) | (__shfl_sync(0xffffffffu, ch, e & 15) << 16);
             asm volatile("st.shared.u32 [%0], %1;" ::"r"(lut_addr + (uint32_t)e * 128 + lane * 4), "r"(v) : "memory");
         }
+    };
+    // Rest of the prologue, run by every warp inside its own role's branch: the table, then the barrier of the
+    // pair, which publishes both CTAs' barriers and tables.
+    // depend() comes after it in every role that needs it, and in whoever is about to make a bounded wait that
+    // ends only after the kernels before this one.
+    auto finish_prologue = [&]() -> uint32_t {
+        build_table(p.ahead ? p.code[lane & 15] : s_code[lane & 15], warp, kPairWarps);
         tc_fence_before();
         cluster_sync_all();
         tc_fence_after();
@@ -390,9 +395,9 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
                 }
             }
         };
-        issue_until(min(SW, total));
+        if (p.ahead) issue_until(min(SW, total));
         tmem = finish_prologue();
-        issue_until(min(SW + S, total));  // the stages the dequant warps empty before the first MMA
+        if (p.ahead) issue_until(min(SW + S, total));  // the stages the dequant warps empty before the first MMA
         depend();
         issue_until(total);
     } else if (warp == 2) {
@@ -520,6 +525,16 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
     } else {
         // ------------------------------------------------------------------ dequant
         tmem = finish_prologue();
+        if (!p.ahead) {
+            depend();
+            const float cv = __ldcg(p.code + (lane & 15));
+            // the kernel before has written another codebook: all the dequant warps see it, and nobody has looked anything up yet
+            if (__any_sync(0xffffffffu, __float_as_uint(cv) != __float_as_uint(s_code[lane & 15]))) {
+                asm volatile("bar.sync 2, %0;" ::"n"(32 * kPairDequantWarps) : "memory");
+                build_table(cv, warp - kPairDequantWarp0, kPairDequantWarps);
+                asm volatile("bar.sync 2, %0;" ::"n"(32 * kPairDequantWarps) : "memory");
+            }
+        }
         const int quarter = warp & 3, group = (warp - kPairDequantWarp0) >> 2;
         const uint32_t lane_base = lut_addr + (uint32_t)lane * 4u;
         const uint32_t a_lane = tmem + ((uint32_t)(32 * quarter) << 16) + a_off;
