@@ -29,6 +29,13 @@ def test_token_counts(n):
     _run(384, n, 320, seed=n)
 
 
+# every token tile, two full ones and a remainder: 16 dequant warps and the wide table up to 192 tokens, 8 and the compact one above
+@pytest.mark.parametrize("tile_tok", [32, 64, 96, 128, 160, 192, 224, 256])
+@pytest.mark.parametrize("m,k", [(512, 576), (264, 1000)])
+def test_token_tiles(tile_tok, m, k):
+    _run(m, 2 * tile_tok + 7, k, seed=tile_tok, tile_tok=tile_tok)
+
+
 # m and k of every weight view: 5-D runs, 3-D boxes (k % 32 == 0), 2-D boxes (any k); fewer rows than a tile, row remainders
 @pytest.mark.parametrize("m,k", [(8, 8), (256, 64), (264, 96), (520, 136), (1032, 1000), (2048, 2112)])
 @pytest.mark.parametrize("n", [70, 250])

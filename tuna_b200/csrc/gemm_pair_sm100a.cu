@@ -14,7 +14,7 @@
 // pipe active for 87 % of the SMs' active clocks (the one-SM kernel: 49 % of the launch, this one 82 %).
 //
 // One persistent CTA pair per two SMs; each CTA dequantizes its own 128 rows into its own tensor
-// memory, the leader (rank 0) issues the MMAs for both.  16 warps per CTA:
+// memory, the leader (rank 0) issues the MMAs for both.  16 or 24 warps per CTA:
 //   warp 0      leader: MMA issue (M = 256, N = the tile's tokens, K = 16, fp32 accumulate): A from
 //               tensor memory, B through a shared-memory descriptor, D in tensor memory.
 //               follower: tells the leader which of its activation stages have landed
@@ -23,7 +23,7 @@
 //   warp 3      tensor-memory allocation
 //   warps 4-7   epilogue: tensor memory -> registers -> scale by absmax -> fp16 -> stmatrix into a
 //               staging tile -> TMA store; split-K partials and fix-up
-//   warps 8-15  dequant: packed bytes (shared memory) -> byte->half2 table lookups -> tcgen05.st.  A
+//   warps 8 on   dequant (8 or 16, pair_dequant_warps): packed bytes (shared memory) -> byte->half2 table lookups -> tcgen05.st.  A
 //               thread owns one weight row (= one TMEM lane): a 32-bit word of the packed layout is
 //               8 consecutive columns of one row (test.py:58-65), i.e. four TMEM columns in K order
 // The dequantised fp16 weights never touch shared or global memory.  The scale is constant along K
@@ -57,14 +57,12 @@ namespace tuna {
 constexpr int kPairRows = 2 * kBlockRows;   // rows of a tile
 constexpr int kPairEpilogueWarp0 = 4;
 constexpr int kPairDequantWarp0 = 8;
-constexpr int kPairDequantWarps = 8;
-constexpr int kPairWarps = kPairDequantWarp0 + kPairDequantWarps;
-constexpr int kPairThreads = 32 * kPairWarps;
-constexpr int kPairGroups = kPairDequantWarps / 4;  // a group of four warps (one per 32-lane quarter) converts every kPairGroups-th stage
 constexpr int kPairTmemCols = 512;
 constexpr int kPairLutBytes = 256 * 128;    // byte -> half2 table: 256 entries, one copy per bank
+constexpr int kPairLutWide = 4096, kPairLutWideBytes = 256 * 256;  // its place and size with 256 bytes per entry (pair_lookup)
 constexpr int kPairMaxStages = 8;           // unit stages: activations in shared memory + an A slot in tensor memory
 constexpr int kPairMaxWStages = 8;
+constexpr int kPairBars = 3 * kPairMaxStages + 2 * kPairMaxWStages + 4;
 constexpr int kPairSmemDynamic = 226 * 1024;
 constexpr int kPairTokGroup = 8;            // token tiles of a wave's working set
 // Up to here weights and codebook are taken from ahead of the dependency wait, as the weight-streaming kernels do (the
@@ -163,12 +161,22 @@ __device__ __forceinline__ int pair_tile_cols(const PairParams &p, int tt)
     return min(p.tile_tok, (p.n - tt * p.tile_tok + 31) & ~31);
 }
 
-__device__ __forceinline__ uint32_t pair_lookup(uint32_t w, uint32_t lane_base, uint32_t selector)
+// Table lookup: byte C of w (two 4-bit codes) -> half2 of the two code values, from this lane's copy of the table.
+//   WIDE: the table lies kPairLutWide into the shared window with 256 bytes per entry (half of them unused), so that ONE prmt
+//   builds the address (window | byte << 8 | lane * 4, `lane_key` = window | lane * 4) and the offset is the load's immediate;
+//   otherwise 128 bytes per entry at `lane_key` - lane * 4, one multiply-add more per lookup.
+template <bool WIDE, int C>
+__device__ __forceinline__ uint32_t pair_lookup(uint32_t w, uint32_t lane_key)
 {
-    uint32_t b, v;
-    asm("prmt.b32 %0, %1, 0, %2;" : "=r"(b) : "r"(w), "r"(selector));
+    uint32_t a, v;
     // not volatile: the table is constant once built, so the compiler may schedule lookups freely
-    asm("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(lane_base + (b << 7)));
+    if (WIDE) {
+        asm("prmt.b32 %0, %1, %2, %3;" : "=r"(a) : "r"(w), "r"(lane_key), "n"(0x7604 | (C << 4)));
+        asm("ld.shared.u32 %0, [%1 + %2];" : "=r"(v) : "r"(a), "n"(kPairLutWide));
+    } else {
+        asm("prmt.b32 %0, %1, 0, %2;" : "=r"(a) : "r"(w), "n"(0x4440 | C));
+        asm("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(lane_key + (a << 7)));
+    }
     return v;
 }
 
@@ -177,16 +185,20 @@ __device__ __forceinline__ uint32_t pair_lookup(uint32_t w, uint32_t lane_base, 
 //      that reads global memory in runs of 256 bytes (m % 32 == 0 and k % 64 == 0); TMEM lane l holds row l;
 //   0  [step][row group][128 bytes]: one 3-D box per stage (k % 32 == 0) or one 2-D box per step; rows
 //      assigned to lanes by lane_row_group().
-template <int KC, int WMODE>
-__global__ void __launch_bounds__(kPairThreads, 1)
+// DW: dequant warps, 8 or 16 (pair_dequant_warps).
+template <int KC, int WMODE, int DW>
+__global__ void __launch_bounds__(32 * (kPairDequantWarp0 + DW), 1)
 gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_constant__ CUtensorMap tmap_q,
                        const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_o)
 {
     constexpr int STEPS = KC / 32;
+    constexpr int kPairWarps = kPairDequantWarp0 + DW;
+    constexpr int kPairGroups = DW / 4;  // a group of four warps (one per 32-lane quarter) converts every kPairGroups-th stage
+    constexpr bool kWide = DW == 16;
     constexpr int kSlotCols = KC / 2;
     constexpr uint32_t kWBytes = kBlockRows * KC / 2;
     extern __shared__ __align__(1024) uint8_t smem[];
-    __shared__ __align__(8) uint64_t bars[3 * kPairMaxStages + 2 * kPairMaxWStages + 4];
+    __shared__ __align__(8) uint64_t bars[kPairBars];
     __shared__ uint32_t s_tmem_base;
     __shared__ int s_abort;
     __shared__ float s_code[16];  // the codebook as it was before the dependency wait
@@ -201,8 +213,9 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
 
     const uint32_t x_tile_bytes = (uint32_t)N * 64;             // N/2 tokens x 64 columns
     const uint32_t x_stage_bytes = x_tile_bytes * (KC / 64);
-    const uint32_t lut_addr = smem_u32(smem);
-    const uint32_t staging = lut_addr + kPairLutBytes;          // [2 halves of 64 rows][N tokens][128 bytes], 128-byte swizzle
+    const uint32_t window = smem_u32(smem) & 0xFFFF0000u;       // in a cluster a CTA's shared addresses carry its rank in their upper bits
+    const uint32_t lut_addr = kWide ? window + kPairLutWide : smem_u32(smem);
+    const uint32_t staging = lut_addr + (kWide ? kPairLutWideBytes : kPairLutBytes);          // [2 halves of 64 rows][N tokens][128 bytes], 128-byte swizzle
     const uint32_t xring = staging + (uint32_t)N * 256;
     const uint32_t wring = xring + (uint32_t)S * x_stage_bytes;
 
@@ -210,19 +223,27 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
     const uint32_t w_full = x_full + 8 * kPairMaxStages, w_empty = w_full + 8 * kPairMaxWStages;
     const uint32_t d_full = w_empty + 8 * kPairMaxWStages, d_empty = d_full + 16;
     volatile int *abort_flag = &s_abort;
+    if (kWide && smem_u32(smem) > lut_addr) {  // the host checks it too; both CTAs leave, since they have the same layout
+        if (threadIdx.x == 0 && atomicCAS(&p.status->code, 0, 109) == 0) p.status->detail = (int)smem_u32(smem);
+        return;
+    }
 
-    if (threadIdx.x == 0) {
-        s_abort = 0;
-        for (int i = 0; i < 4; ++i) s_fix[i] = 0;
-        for (int i = 0; i < kPairMaxStages; ++i) {
-            // leader: its own activation copy, four dequant warps of each CTA, the follower's activation copy
-            mbar_init(u_full + 8 * i, 10);
-            mbar_init(u_empty + 8 * i, 1);
-            mbar_init(x_full + 8 * i, 1);  // follower only
-        }
-        for (int i = 0; i < kPairMaxWStages; ++i) { mbar_init(w_full + 8 * i, 1); mbar_init(w_empty + 8 * i, 4); }
-        for (int i = 0; i < 2; ++i) { mbar_init(d_full + 8 * i, 1); mbar_init(d_empty + 8 * i, 8); }
+    if (warp == 1) {  // the barriers, 32 at a time
+        auto count = [](int i) {
+            if (i < kPairMaxStages) return 10;                            // u_full: two activation copies, four dequant warps of each CTA
+            if (i < 3 * kPairMaxStages + kPairMaxWStages) return 1;       // u_empty, x_full (follower only), w_full
+            if (i < 3 * kPairMaxStages + 2 * kPairMaxWStages) return 4;   // w_empty
+            return i < kPairBars - 2 ? 1 : 8;                             // d_full, d_empty
+        };
+        for (int i = lane; i < kPairBars; i += 32) mbar_init(u_full + 8 * i, count(i));
+        if (lane == 0) s_abort = 0;
+        if (lane < 4) s_fix[lane] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        __syncwarp();
+    }
+    if (warp == 2 && elect_one_sync()) {
+        prefetch_map(&tmap_x);
+        prefetch_map(&tmap_o);
     }
     if (warp == 3) {
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem_base)),
@@ -247,15 +268,16 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
         const uint32_t ch = (uint32_t)__half_as_ushort(__float2half_rn(cv));
         for (int e = first; e < 256; e += step) {
             const uint32_t v = __shfl_sync(0xffffffffu, ch, e >> 4) | (__shfl_sync(0xffffffffu, ch, e & 15) << 16);
-            asm volatile("st.shared.u32 [%0], %1;" ::"r"(lut_addr + (uint32_t)e * 128 + lane * 4), "r"(v) : "memory");
+            asm volatile("st.shared.u32 [%0], %1;" ::"r"(lut_addr + (uint32_t)e * (kWide ? 256 : 128) + lane * 4), "r"(v) : "memory");
         }
     };
     // Rest of the prologue, run by every warp inside its own role's branch: the table, then the barrier of the
     // pair, which publishes both CTAs' barriers and tables.
     // depend() comes after it in every role that needs it, and in whoever is about to make a bounded wait that
     // ends only after the kernels before this one.
+    auto table_share = [&] { build_table(p.ahead ? p.code[lane & 15] : s_code[lane & 15], warp, kPairWarps); };
     auto finish_prologue = [&]() -> uint32_t {
-        build_table(p.ahead ? p.code[lane & 15] : s_code[lane & 15], warp, kPairWarps);
+        table_share();
         tc_fence_before();
         cluster_sync_all();
         tc_fence_after();
@@ -286,17 +308,18 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
         float acc[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) acc[i] = 0.f;
-        for (int s = 0; s < nseg; s += 4) {  // four segments' loads in flight; the adds keep the order
-            float4 v[4][4];
+        constexpr int SG = DW == 16 ? 2 : 4;  // segments' loads in flight; the adds keep the order
+        for (int s = 0; s < nseg; s += SG) {
+            float4 v[SG][4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
+            for (int j = 0; j < SG; ++j)
                 if (s + j < nseg) {
                     const float4 *src = seg_ptr(s + j);
 #pragma unroll
                     for (int i = 0; i < 4; ++i) v[j][i] = __ldcg(src + i * kBlockRows);
                 }
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
+            for (int j = 0; j < SG; ++j)
                 if (s + j < nseg) {
 #pragma unroll
                     for (int i = 0; i < 4; ++i) { acc[4 * i] += v[j][i].x; acc[4 * i + 1] += v[j][i].y; acc[4 * i + 2] += v[j][i].z; acc[4 * i + 3] += v[j][i].w; }
@@ -395,8 +418,11 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
                 }
             }
         };
+        // The copies of a ring-full take longer than the rest of the prologue: the other warps do not wait for them.
+        table_share();
+        cluster_arrive();
         if (p.ahead) issue_until(min(SW, total));
-        tmem = finish_prologue();
+        cluster_wait();
         if (p.ahead) issue_until(min(SW + S, total));  // the stages the dequant warps empty before the first MMA
         depend();
         issue_until(total);
@@ -521,7 +547,8 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
             }
             rd.advance(p.nd);
         }
-        if (threadIdx.x == 32 * kPairEpilogueWarp0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+        // the stores have read the staging tile; the end of the kernel makes them visible
+        if (threadIdx.x == 32 * kPairEpilogueWarp0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
     } else {
         // ------------------------------------------------------------------ dequant
         tmem = finish_prologue();
@@ -530,13 +557,13 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
             const float cv = __ldcg(p.code + (lane & 15));
             // the kernel before has written another codebook: all the dequant warps see it, and nobody has looked anything up yet
             if (__any_sync(0xffffffffu, __float_as_uint(cv) != __float_as_uint(s_code[lane & 15]))) {
-                asm volatile("bar.sync 2, %0;" ::"n"(32 * kPairDequantWarps) : "memory");
-                build_table(cv, warp - kPairDequantWarp0, kPairDequantWarps);
-                asm volatile("bar.sync 2, %0;" ::"n"(32 * kPairDequantWarps) : "memory");
+                asm volatile("bar.sync 2, %0;" ::"n"(32 * DW) : "memory");
+                build_table(cv, warp - kPairDequantWarp0, DW);
+                asm volatile("bar.sync 2, %0;" ::"n"(32 * DW) : "memory");
             }
         }
         const int quarter = warp & 3, group = (warp - kPairDequantWarp0) >> 2;
-        const uint32_t lane_base = lut_addr + (uint32_t)lane * 4u;
+        const uint32_t lane_key = (kWide ? window : lut_addr) + (uint32_t)lane * 4u;
         const uint32_t a_lane = tmem + ((uint32_t)(32 * quarter) << 16) + a_off;
         // This thread's row inside a weight stage (see the weight-streaming kernel): word r%4 of 16-byte chunk
         // 2 kt + r/4 of the 128-byte row of (row group, step), XORed with that row's index mod 8.
@@ -571,10 +598,10 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
                     const uint32_t word = w[st0 + (i >> 2)][i & 3];
-                    v[4 * i] = pair_lookup(word, lane_base, 0x4440);
-                    v[4 * i + 1] = pair_lookup(word, lane_base, 0x4441);
-                    v[4 * i + 2] = pair_lookup(word, lane_base, 0x4442);
-                    v[4 * i + 3] = pair_lookup(word, lane_base, 0x4443);
+                    v[4 * i] = pair_lookup<kWide, 0>(word, lane_key);
+                    v[4 * i + 1] = pair_lookup<kWide, 1>(word, lane_key);
+                    v[4 * i + 2] = pair_lookup<kWide, 2>(word, lane_key);
+                    v[4 * i + 3] = pair_lookup<kWide, 3>(word, lane_key);
                 }
             };
             lookups(0);
@@ -631,6 +658,13 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
 // file) at the 1.7 GHz of a short run, or the tensor pipe's N/2 clocks, and what the dequantisation adds to them, at the
 // clock the power cap leaves it (measured at K = 4096: 14 us a wave of 128-token tiles, 22 of 224, 25 of 256).
 static double pair_step_us(int tok) { return std::max((tok / 4 + 61) / 1700.0, (tok / 2 + 8) / 1420.0); }
+
+// 16 dequant warps where they bound the tile, i.e. as long as the tensor pipe needs fewer clocks per step than the table
+// lookups and what goes with them; with them comes the table that one instruction per lookup addresses (pair_lookup), which leaves
+// too little shared memory for the stages of wider tiles.  Graph replay, us, 8 / 16 warps / 16 and the wide table: 11000x4104 at 43
+// tokens 13.5 / 12.6 / 12.5, 6144x4096 at 256 (96-token tiles) 15.5 / 14.5 / 14.1, 57344x8192 at 64 81 / 70 / 70, 8192x8192 at 192
+// 27.5 / 25.5 / 24.3; 57344x8192 at 256 (256-token tiles) 166 / 167, 28672x4096 at 224 47 / 46.
+static int pair_dequant_warps(int tile_tok) { return tile_tok <= 192 ? 16 : 8; }
 
 static int pair_kc(int tile_tok) { return tile_tok > 128 ? 64 : 128; }
 
@@ -701,7 +735,9 @@ static PairPlan pair_plan(const tuna_config &c)
     l.stages = (kPairTmemCols - l.nd * l.tile_tok) / slot;
     if (l.stages > kPairMaxStages) l.stages = kPairMaxStages;
     const int w_bytes = kBlockRows * l.kc / 2;
-    auto smem = [&](int s, int w) { return kPairLutBytes + l.tile_tok * 256 + s * l.tile_tok * l.kc + w * w_bytes; };
+    // dynamic shared memory begins 2 KB into the window (launch_pair checks it)
+    const int lut = pair_dequant_warps(l.tile_tok) == 16 ? kPairLutWide - 2048 + kPairLutWideBytes : kPairLutBytes;
+    auto smem = [&](int s, int w) { return lut + l.tile_tok * 256 + s * l.tile_tok * l.kc + w * w_bytes; };
     l.w_stages = kPairMaxWStages;
     while (l.stages > 4 && smem(l.stages, l.w_stages) > kPairSmemDynamic) --l.stages;
     while (l.w_stages > 4 && smem(l.stages, l.w_stages) > kPairSmemDynamic) --l.w_stages;
@@ -738,7 +774,7 @@ int gemm_umma_normalize_config(int m, int n, int k, int sm_count, tuna_config *c
     // what the launch takes, for whoever looks it up (stages follow from the token tile and stay 0)
     if (t == 0) c->tile_tok = pair_pick_tile_tok(m, n, k, pair_count(*c));
     if (c->row_blocks == 0) c->row_blocks = 1;
-    if (c->dequant_warps == 0) c->dequant_warps = kPairDequantWarps;
+    if (c->dequant_warps == 0) c->dequant_warps = pair_dequant_warps(c->tile_tok);
     if (c->k_accs == 0) c->k_accs = 1;
     return TUNA_OK;
 }
@@ -752,7 +788,7 @@ size_t gemm_umma_workspace_bytes(int m, int n, int k, const tuna_config &c, int 
     return partial_region_bytes(sm_count) + ((size_t)cut * 32 + 255) / 256 * 256;  // one counter per tile, CTA and TMEM lane quarter
 }
 
-template <int KC, int WMODE>
+template <int KC, int WMODE, int DW>
 static int launch_pair(const PairParams &p, const CUtensorMap &mq, const CUtensorMap &mx, const CUtensorMap &mo, int ctas, cudaStream_t stream)
 {
     static bool attr_set[64] = {false};  // one-time, per device, opt-in to large dynamic shared memory
@@ -762,14 +798,21 @@ static int launch_pair(const PairParams &p, const CUtensorMap &mq, const CUtenso
     {
         std::lock_guard<std::mutex> lock(mu);
         if (!attr_set[dev]) {
-            if (cudaFuncSetAttribute(gemm_w4a16_pair_kernel<KC, WMODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemDynamic) != cudaSuccess)
+            if (cudaFuncSetAttribute(gemm_w4a16_pair_kernel<KC, WMODE, DW>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemDynamic) != cudaSuccess)
+                return TUNA_ERR_NO_DEVICE;
+            // pair_plan counts on 1 KB of the system's and 1 KB of static shared memory before the dynamic part
+            cudaFuncAttributes fa;
+            int reserved = 0;
+            if (cudaFuncGetAttributes(&fa, gemm_w4a16_pair_kernel<KC, WMODE, DW>) != cudaSuccess ||
+                cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev) != cudaSuccess ||
+                fa.sharedSizeBytes + (size_t)reserved > 2048)
                 return TUNA_ERR_NO_DEVICE;
             attr_set[dev] = true;
         }
     }
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3((unsigned)ctas);
-    lc.blockDim = dim3(kPairThreads);
+    lc.blockDim = dim3(32 * (kPairDequantWarp0 + DW));
     lc.dynamicSmemBytes = kPairSmemDynamic;
     lc.stream = stream;
     cudaLaunchAttribute attr[2];
@@ -780,7 +823,7 @@ static int launch_pair(const PairParams &p, const CUtensorMap &mq, const CUtenso
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     lc.attrs = attr;
     lc.numAttrs = 2;
-    return cudaLaunchKernelEx(&lc, gemm_w4a16_pair_kernel<KC, WMODE>, p, mq, mx, mo) == cudaSuccess ? TUNA_OK : TUNA_ERR_LAUNCH;
+    return cudaLaunchKernelEx(&lc, gemm_w4a16_pair_kernel<KC, WMODE, DW>, p, mq, mx, mo) == cudaSuccess ? TUNA_OK : TUNA_ERR_LAUNCH;
 }
 
 int launch_gemm_umma(const GemmArgs &a, const tuna_config &c)
@@ -833,8 +876,16 @@ int launch_gemm_umma(const GemmArgs &a, const tuna_config &c)
     if (!make_tensor_map_2d(&mo, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, a.o, (uint64_t)a.m, (uint64_t)a.n, (uint64_t)a.m * 2, 64,
                             (uint32_t)l.tile_tok, CU_TENSOR_MAP_SWIZZLE_128B))
         return TUNA_ERR_NO_DEVICE;
-    if (l.kc == 64) return w_mode ? launch_pair<64, 1>(p, mq, mx, mo, 2 * pairs, a.stream) : launch_pair<64, 0>(p, mq, mx, mo, 2 * pairs, a.stream);
-    return w_mode ? launch_pair<128, 1>(p, mq, mx, mo, 2 * pairs, a.stream) : launch_pair<128, 0>(p, mq, mx, mo, 2 * pairs, a.stream);
+    switch (pair_dequant_warps(l.tile_tok) * 1000 + l.kc + w_mode) {
+        case 8064: return launch_pair<64, 0, 8>(p, mq, mx, mo, 2 * pairs, a.stream);
+        case 8065: return launch_pair<64, 1, 8>(p, mq, mx, mo, 2 * pairs, a.stream);
+        case 8128: return launch_pair<128, 0, 8>(p, mq, mx, mo, 2 * pairs, a.stream);
+        case 8129: return launch_pair<128, 1, 8>(p, mq, mx, mo, 2 * pairs, a.stream);
+        case 16064: return launch_pair<64, 0, 16>(p, mq, mx, mo, 2 * pairs, a.stream);
+        case 16065: return launch_pair<64, 1, 16>(p, mq, mx, mo, 2 * pairs, a.stream);
+        case 16128: return launch_pair<128, 0, 16>(p, mq, mx, mo, 2 * pairs, a.stream);
+        default: return launch_pair<128, 1, 16>(p, mq, mx, mo, 2 * pairs, a.stream);
+    }
 }
 
 }  // namespace tuna

@@ -101,9 +101,12 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar)
 {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_sync_all()
 {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    cluster_arrive();
+    cluster_wait();
 }
 // Named barrier of `threads` threads that answers, to all of them, whether any came with `v`.
 __device__ __forceinline__ bool bar_any(int id, int threads, bool v)
@@ -113,7 +116,7 @@ __device__ __forceinline__ bool bar_any(int id, int threads, bool v)
                  : "=r"(r)
                  : "r"(id), "r"(threads), "r"((uint32_t)v)
                  : "memory");
-    return r != 0;
+    return __any_sync(0xffffffffu, r != 0) != 0;  // the same in all lanes, and the compiler may rely on it
 }
 
 // True in exactly one lane of a converged warp.
@@ -123,6 +126,9 @@ __device__ __forceinline__ bool elect_one_sync()
     asm volatile("{\n .reg .pred P;\n elect.sync _|P, 0xffffffff;\n selp.u32 %0, 1, 0, P;\n}" : "=r"(e));
     return e != 0;
 }
+
+// Brings a tensor map (a kernel parameter) into the descriptor cache ahead of its first copy.
+__device__ __forceinline__ void prefetch_map(const CUtensorMap *map) { asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory"); }
 
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int c0, int c1, uint32_t bar)
 {
