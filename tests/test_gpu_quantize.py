@@ -91,6 +91,21 @@ def test_every_share_and_codebook_is_bit_exact(m, k, book):
     assert np.array_equal(q.cpu().numpy(), q_ref)
 
 
+# two thresholds in one of 64 buckets but not in one of 128, in one of 128 only, in one of either
+@pytest.mark.parametrize("codes", [(0.0, 0.04, 0.05), (0.0, 0.021, 0.0213), (0.04, 0.0402, 0.0404)])
+@pytest.mark.parametrize("m,k", [(16, 1000), (16, 4104)])
+def test_codes_whose_thresholds_share_buckets(codes, m, k):
+    w = (np.random.default_rng(k).standard_normal((m, k)) * 0.05).astype(np.float16)
+    w[1, : k // 2] = (np.arange(k // 2) / 2048).astype(np.float16)
+    w[1, 0] = 1
+    code = orc.NF4_CODE.copy()
+    code[7:10] = codes
+    q, (absmax, _) = tuna_b200.quantize(torch.from_numpy(w).cuda(), torch.from_numpy(code).cuda())
+    q_ref, a_ref, _ = orc.quantize_blockwise_dynamic_4bit(w, code)
+    assert np.array_equal(absmax.cpu().numpy(), a_ref)
+    assert np.array_equal(q.cpu().numpy(), q_ref)
+
+
 @pytest.mark.parametrize("m,k", [(2048, 8), (4096, 8), (4096, 64), (4096, 136), (8192, 128), (8192, 256)])
 @pytest.mark.parametrize("book", ["nf4", "unsorted"])
 def test_narrow_rows_on_both_sides_of_the_two_pass_line(m, k, book):

@@ -26,7 +26,7 @@
 // comparison per weight.  The table is exact because a threshold is filed under the bucket the same
 // FMA gives it.  Rows it cannot represent (two thresholds in one bucket, a zero, tiny or
 // non-finite absmax, codes that are equal, closer than fp32 can separate, or not finite) take the
-// literal expression.  28672x4096: 436 -> 80 us (0.68 -> 3.7 TB/s of its 294 MB).
+// literal expression.  28672x4096: 436 -> 67 us (0.68 -> 4.4 TB/s of its 294 MB).
 #include <cuda_fp16.h>
 #include <mutex>
 #include "common.cuh"
@@ -48,7 +48,8 @@ __constant__ float kNf4[16] = {-1.0f, -0.6961928009986877f, -0.5250730514526367f
 
 // The rows' tables lie side by side, bucket by bucket, each row's twice: lane l of a warp (row l % 8) looks up in column
 // l % 16, so that two lanes share a bank at most (rows' tables one after another, where random
-// lookups meet three or four at a time: 84 us against 80 on 28672x4096).
+// lookups meet three or four at a time: 84 us against 80 on 28672x4096; 64 buckets with a column per bank, and the code that
+// chooses between the two, 84: the lookups are not what bounds it any more, the phases' instructions are).
 constexpr int kTableCols = 16;
 constexpr int kThrStride = 17;  // words of a row's thresholds: the eight rows' lie in different banks
 
@@ -94,7 +95,7 @@ __global__ void __launch_bounds__(kQuantThreads) quantize_rows_kernel(const __ha
     __shared__ uint32_t s_bucket_scale[8];  // half2
     __shared__ uint32_t s_thr[8][kThrStride];  // fp16 bits of threshold i | its bucket << 16
     __shared__ int s_row_ok[8];
-    __shared__ uint32_t s_table[kBuckets * kTableCols];  // fp16 threshold | codes (below | (below ^ above) << 4) << 16
+    __shared__ uint32_t s_table[kBuckets * kTableCols];  // fp16 threshold | codes (below << 4 | (below ^ above)) << 16
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int rg = blockIdx.x / cluster, rank = blockIdx.x - rg * cluster;
@@ -199,7 +200,7 @@ __global__ void __launch_bounds__(kQuantThreads) quantize_rows_kernel(const __ha
 
     // ---- thresholds: thread (row, i) finds the smallest fp16 weight whose code lies above sorted code i
     if (tid < 128) {
-        const int row = tid >> 4, i = tid & 15;
+        const int row = tid & 7, i = tid >> 3;
         uint32_t thr = 0x7fffu, bkt = 255u;  // a NaN no weight compares >= to, in no bucket
         if (i < 15 && s_row_ok[row]) {
             const float s = s_scale[row], a = s_sorted[i], b = s_sorted[i + 1];
@@ -249,30 +250,19 @@ __global__ void __launch_bounds__(kQuantThreads) quantize_rows_kernel(const __ha
     }
     __syncthreads();
 
-    // ---- the rows' tables: lane (row r, l / 8) fills four of the warp's 16 buckets
+    // ---- the rows' tables: thread (row, i, half) fills every other bucket after threshold i - 1's up to threshold i's
+    // (filling by bucket, which counts the thresholds below each, was a quarter of the kernel's instructions: 28672x4096 75.2 us, so 67.3)
     {
-        const int row = lane & 7, b0 = warp * (kBuckets / 8) + (lane >> 3);
-        uint32_t below[4] = {}, hits[4] = {}, thr[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) thr[j] = 0x7fffu;
-        for (int i = 0; i < 15; ++i) {
-            const uint32_t t = s_thr[row][i], bt = t >> 16;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const uint32_t b = (uint32_t)(b0 + 4 * j);
-                below[j] += bt < b ? 1u : 0u;
-                if (bt == b) { ++hits[j]; thr[j] = t & 0xffffu; }
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const uint32_t b = (uint32_t)(b0 + 4 * j);
-            const uint32_t lo = s_sorted_idx[below[j]], hi = s_sorted_idx[min(below[j] + 1u, 15u)];
-            const uint32_t e = thr[j] | ((lo | ((lo ^ hi) << 4)) << 16);
+        const int row = tid & 7, i = (tid >> 3) & 15, half = tid >> 7;
+        const uint32_t t = s_thr[row][i], bkt = t >> 16, prev = i > 0 ? s_thr[row][i - 1] >> 16 : 0u;
+        const uint32_t lo = s_sorted_idx[i], hi = s_sorted_idx[min(i + 1, 15)];
+        const uint32_t codes = ((lo << 4) | (lo ^ hi)) << 16;
+        for (uint32_t b = prev + 1 + half; b <= min(bkt, (uint32_t)kBuckets - 1); b += 2) {
+            const uint32_t e = (b == bkt ? t & 0xffffu : 0x7fffu) | codes;
             s_table[b * kTableCols + row] = e;
             s_table[b * kTableCols + 8 + row] = e;
-            if (b > 0 && hits[j] > 1) s_row_ok[row] = 0;
         }
+        if (i > 0 && bkt == prev && bkt > 0 && bkt < kBuckets) s_row_ok[row] = 0;  // two thresholds in one bucket
     }
     __syncthreads();
 
@@ -292,14 +282,22 @@ __global__ void __launch_bounds__(kQuantThreads) quantize_rows_kernel(const __ha
                     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(e0[i]) : "r"(table + 4u * kTableCols * (b2 & 0xffu)));
                     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(e1[i]) : "r"(table + 4u * kTableCols * __byte_perm(b2, 0, 0x4442)));
                 }
-                uint32_t word = 0;
+                // two pairs at a time, a byte per weight: the code below in the high nibble, the difference to the one above in the low one
+                uint32_t half_word[2];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const uint32_t t2 = __byte_perm(e0[i], e1[i], 0x5410), c2 = __byte_perm(e0[i], e1[i], 0x7632);
-                    const uint32_t m = __hge2_mask(*reinterpret_cast<const __half2 *>(&u[i]), *reinterpret_cast<const __half2 *>(&t2));
-                    const uint32_t c = (c2 ^ ((c2 >> 4) & m)) & 0x000f000fu;  // code of the even column | odd column << 16
-                    word |= ((c << 4) | (c >> 16)) << (8 * i) & (0xffu << (8 * i));
+                for (int i = 0; i < 4; i += 2) {
+                    uint32_t c[2], m[2];
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        const uint32_t t2 = __byte_perm(e0[i + j], e1[i + j], 0x5410);
+                        m[j] = __hge2_mask(*reinterpret_cast<const __half2 *>(&u[i + j]), *reinterpret_cast<const __half2 *>(&t2));
+                        c[j] = __byte_perm(e0[i + j], e1[i + j], 0x0062);
+                    }
+                    const uint32_t codes = __byte_perm(c[0], c[1], 0x5410), above = __byte_perm(m[0], m[1], 0x6420);
+                    const uint32_t sel = codes ^ ((codes << 4) & above);                    // the code in each high nibble
+                    half_word[i >> 1] = (sel & 0x00f000f0u) | ((sel >> 12) & 0x000f000fu);  // even column high: bytes 0 and 2
                 }
+                const uint32_t word = __byte_perm(half_word[0], half_word[1], 0x6420);
                 *reinterpret_cast<uint32_t *>(dst + (size_t)kt * 32) = word;
             }
         } else {
@@ -407,14 +405,14 @@ __global__ void __launch_bounds__(256) quantize_pack_kernel(const __half *__rest
     }
 }
 
-// Whether two passes are the faster way.  A CTA of the single pass spends ~3 us on its row group before the first code,
-// whatever the width; on narrow rows the literal expression is done with them sooner.  The estimates (us) are fitted to 8 to
-// 229376 rows of 8 to 512 columns; two passes / one: 57344x8 17.7 / 51.0, 57344x128 33.3 / 52.3, 57344x256 55.0 / 55.3, 8192x64
-// 7.2 / 9.5, 4096x128 6.6 / 6.2, 2048x64 4.7 / 4.6.
+// Whether two passes are the faster way.  A CTA of the single pass spends ~1.8 us on its row group before the first code,
+// whatever the width; on many very narrow rows the literal expression is done with them sooner.  The estimates (us) are fitted to 8 to
+// 229376 rows of 8 to 512 columns; two passes / one: 57344x8 17.4 / 30.4, 57344x64 22.0 / 30.8, 57344x128 33.2 / 31.5, 8192x64
+// 6.9 / 6.4, 8192x128 8.6 / 6.5, 4096x64 5.7 / 3.9.
 static bool quantize_in_two_passes(int m, int k, int sm_count)
 {
     const double groups_per_sm = (m / 8) / (double)sm_count;
-    return 4.6 + groups_per_sm * (0.15 + 0.00355 * k) < 2.6 + groups_per_sm / 3 * (3.0 + 0.001 * k);
+    return 4.6 + groups_per_sm * (0.15 + 0.00355 * k) < 2.2 + groups_per_sm / 3 * (1.72 + 0.001 * k);
 }
 
 cudaError_t launch_quantize(const void *w, const void *code, void *code_out, void *q, void *absmax, int m, int k, int sm_count,
