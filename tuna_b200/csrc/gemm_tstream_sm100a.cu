@@ -111,6 +111,8 @@ constexpr int kTsMaxWStages = 16;     // weight ring: as many stages as shared m
 constexpr int kTsLutBytes = 256 * 128;    // byte -> half2 table: 256 entries, 32 copies (one per bank) of 4 bytes
 constexpr int kTsSmemTotal = 227 * 1024;             // static + dynamic shared memory of a CTA on sm_100
 constexpr int kTsSmemDynamic = kTsSmemTotal - 1024;  // the static part (barriers) stays below 1 KB
+constexpr int kTsBars = 2 * kTsMaxASlots + 2 * kTsMaxXStages + 4 + 2 * kTsMaxWStages;
+constexpr int kTsXWarp = 1, kTsWeightWarp = 2, kTsEpilogueWarp0 = 4;
 constexpr int kTsDequantWarp0 = 8;
 #ifndef TS_DEQUANT_WARPS
 #define TS_DEQUANT_WARPS 16
@@ -266,7 +268,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_w4a16_tstream_kernel(const
     static_assert(N_TILE > 32 || kXS * kXStageBytes + 4096 <= 0x10000, "the activation ring must end below the lookup table");
     static_assert(kXStageBytes % 1024 == 0 && kSlotBytes % 1024 == 0, "swizzle atoms are 1024 bytes");
     extern __shared__ __align__(1024) uint8_t smem[];
-    __shared__ __align__(8) uint64_t bars[2 * kTsMaxASlots + 2 * kTsMaxXStages + 4 + 2 * kTsMaxWStages];
+    __shared__ __align__(8) uint64_t bars[kTsBars];
     __shared__ uint32_t s_tmem_base;
     __shared__ int s_abort;
     // The cut tiles of the CTA's range, at most its first [0] and its last [1], that this CTA finishes at its end
@@ -317,42 +319,49 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_w4a16_tstream_kernel(const
     const int u_begin = cta * p.units_q + min(cta, p.units_r);
     const int n_units = p.units_q + (cta < p.units_r ? 1 : 0);
 
-    if (threadIdx.x == 0) {
-        s_abort = 0;
-        for (int i = 0; i < 8; ++i) s_fix[i >> 2][i & 3] = 0;
-        for (int i = 0; i < kTsMaxASlots; ++i) { mbar_init(a_full + 8 * i, 4 * kHalves); mbar_init(a_empty + 8 * i, 1); }
-        for (int i = 0; i < kTsMaxXStages; ++i) { mbar_init(x_full + 8 * i, 1); mbar_init(x_empty + 8 * i, 1); }
-        for (int i = 0; i < 2; ++i) { mbar_init(d_full + 8 * i, 1); mbar_init(d_empty + 8 * i, 4); }
-        for (int i = 0; i < kTsMaxWStages; ++i) { mbar_init(w_full + 8 * i, 1); mbar_init(w_empty + 8 * i, 4 * kHalves); }
+    // The weight producer initialises the barriers, 32 at a time, and goes on to its copies without waiting for anyone:
+    // issuing a ring-full takes longer than the rest of the prologue.
+    if (warp == kTsWeightWarp) {
+        auto count = [](int i) {
+            if (i < kTsMaxASlots) return 4 * kHalves;                  // a_full
+            i -= 2 * kTsMaxASlots + 2 * kTsMaxXStages + 4;
+            if (i < -2 || (i >= 0 && i < kTsMaxWStages)) return 1;     // a_empty, x_full, x_empty, d_full; w_full
+            return i < 0 ? 4 : 4 * kHalves;                            // d_empty; w_empty
+        };
+        for (int i = lane; i < kTsBars; i += 32) mbar_init(bar0 + 8 * i, count(i));
+        if (lane == 0) s_abort = 0;
+        if (lane < 8) s_fix[lane >> 2][lane & 3] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == 0) {
-        __syncwarp();  // lane 0 comes from the branch above, and the allocation wants a converged warp
+        __syncwarp();
+    } else if (warp == kTsXWarp) {
+        if (elect_one_sync()) prefetch_map(&L.g[0].map_x);
+    } else if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem_base)),
                      "r"(kTsTmemCols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    __syncthreads();  // barriers initialised: the weight producer may start
 
     const int quarter = warp & 3;          // the 32 tensor-memory lanes this warp may access
     const int total_slots = n_units * RB;
 
-    // Rest of the prologue, run by every warp inside its own role's branch: the byte -> half2
-    // table (even column = high nibble in the low half), one copy per bank - the codebook is a
-    // constant, so this needs no dependency wait - then the CTA barrier that publishes the table and the
+    // Rest of the prologue, run by every other warp inside its own role's branch: the byte -> half2
+    // table (even column = high nibble in the low half), one copy per bank, by the epilogue and dequant warps - the
+    // codebook is a constant, so this needs no dependency wait - then the CTA barrier that publishes barriers, table and
     // tensor-memory base.  Only what reads or writes data of the kernels before this one waits for
     // them (depend(): the copies of x, the epilogue, and before their bounded waits the MMA warp and
     // whoever has filled its ring), so the dequant warps fill the A-slot ring meanwhile.
     auto finish_prologue = [&]() -> uint32_t {
-        const float cv = p.code[lane & 15];
-        const uint32_t ch = (uint32_t)__half_as_ushort(__float2half_rn(cv));
-        for (int e = warp; e < 256; e += kTsThreads / 32) {
-            const uint32_t v = __shfl_sync(0xffffffffu, ch, e >> 4) | (__shfl_sync(0xffffffffu, ch, e & 15) << 16);
-            asm volatile("st.shared.u32 [%0], %1;" ::"r"(lut_addr + (uint32_t)e * (kLut256 ? 256 : 128) + lane * 4), "r"(v) : "memory");
+        if (warp >= kTsEpilogueWarp0) {
+            const float cv = p.code[lane & 15];
+            const uint32_t ch = (uint32_t)__half_as_ushort(__float2half_rn(cv));
+            for (int e = warp - kTsEpilogueWarp0; e < 256; e += kTsThreads / 32 - kTsEpilogueWarp0) {
+                const uint32_t v = __shfl_sync(0xffffffffu, ch, e >> 4) | (__shfl_sync(0xffffffffu, ch, e & 15) << 16);
+                asm volatile("st.shared.u32 [%0], %1;" ::"r"(lut_addr + (uint32_t)e * (kLut256 ? 256 : 128) + lane * 4), "r"(v) : "memory");
+            }
         }
         tc_fence_before();
-        __syncthreads();
+        asm volatile("bar.sync 1, %0;" ::"n"(kTsThreads) : "memory");
         tc_fence_after();
         TS_PROF_MARK(1)
         return s_tmem_base;
@@ -390,10 +399,10 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_w4a16_tstream_kernel(const
             }
         }
     };
-    // Adds the partials of GR four-token groups from group g0 on of 32 rows (block rb, quarter q of the tile) over its
+    // Adds the partials of GR four-token groups from group g0 on (the last group that exists stands in for those after it) of 32 rows (block rb, quarter q of the tile) over its
     // segments, which CTAs `first` .. first + nseg - 1 wrote, and stores the rows.  The loads of SG segments are
     // in flight at a time, the adds keep the range order.
-    auto add_partials = [&](auto gr, auto sg, const TsGemm &G, int tile, int first, int nseg, int q, int rb, int g0) __attribute__((always_inline)) {
+    auto add_partials = [&](auto gr, auto sg, const TsGemm &G, int tile, int first, int nseg, int q, int rb, int g0, int last) __attribute__((always_inline)) {
         constexpr int GR = decltype(gr)::value, SG = decltype(sg)::value;
         const int row = (tile * RB + rb) * kBlockRows + row_in_block(q);
         if (row >= G.m) return;
@@ -408,9 +417,9 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_w4a16_tstream_kernel(const
             for (int j = 0; j < SG; ++j) {
                 const int seg = min(sgm + j, nseg - 1);
                 const float4 *src = reinterpret_cast<const float4 *>(p.partials + (size_t)(2 * (first + seg) + (seg == 0 ? 1 : 0)) * slot_floats) +
-                                    ((size_t)rb * (N_TILE / 4) + g0) * kBlockRows + 32 * q + lane;
+                                    (size_t)rb * (N_TILE / 4) * kBlockRows + 32 * q + lane;
 #pragma unroll
-                for (int i = 0; i < GR; ++i) a[j][i] = __ldcg(src + i * kBlockRows);
+                for (int i = 0; i < GR; ++i) a[j][i] = __ldcg(src + min(g0 + i, last) * kBlockRows);
             }
 #pragma unroll
             for (int j = 0; j < SG; ++j) {
@@ -423,16 +432,16 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_w4a16_tstream_kernel(const
         store_row(G, row, 4 * g0, acc, sc);
     };
     // The flagged quarters of a tile whose partials are all there, shared out over warps `w0`, w0 + step, ... : a warp
-    // takes four tokens of 32 rows at a time (small code: it runs once per CTA, out of a cold instruction cache),
-    // in exchange launches 16, whole sectors of a peer's slab.
+    // takes eight tokens of 32 rows at a time, so that all of a tile is in flight at once (28672x4096 at 16 tokens, two row blocks: by
+    // four 18.0 us, by eight 17.7), in exchange launches 16, whole sectors of a peer's slab.
     auto finish_tile = [&](const TsGemm &G, int tile, int first, int nseg, const int *flagged, int w0, int step) __attribute__((always_inline)) {
-        const int groups4 = token_groups(G), per = p.n_peers > 0 ? 4 : 1, rb_shift = RB >> 1;
-        for (int item = w0; item * per < 4 * RB * groups4; item += step) {
+        const int groups4 = token_groups(G), per = p.n_peers > 0 ? 4 : 2, rb_shift = RB >> 1;
+        for (int item = w0; (item >> (2 + rb_shift)) * per < groups4; item += step) {
             const int q = item & 3, rest = item >> 2;
-            const int g = rest >> rb_shift, rb = rest & (RB - 1);  // RB is 1, 2 or 4
+            const int g = (rest >> rb_shift) * per, rb = rest & (RB - 1);  // RB is 1, 2 or 4
             if (!flagged[q]) continue;
-            if (per == 1) add_partials(Int<1>(), Int<4>(), G, tile, first, nseg, q, rb, g);
-            else add_partials(Int<4>(), Int<2>(), G, tile, first, nseg, q, rb, 4 * g);
+            if (per == 2) add_partials(Int<2>(), Int<4>(), G, tile, first, nseg, q, rb, g, groups4 - 1);
+            else add_partials(Int<4>(), Int<2>(), G, tile, first, nseg, q, rb, g, groups4 - 1);
         }
     };
     auto first_cta = [&](const TsGemm &G, int tile) { return ts_cta_of_unit(p, G.unit0 + tile * G.chunks); };
@@ -445,13 +454,13 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_w4a16_tstream_kernel(const
         // issues the MMAs and the commits.  Descriptors (K-major, 128-byte swizzle): the high word
         // is constant (8-token groups 1024 bytes apart, version 1, layout type 2), the low word is the
         // start address; 16 columns further along K is 32 bytes further inside the 128-byte row.
-        tmem = finish_prologue();
-        depend();
         constexpr uint32_t idesc = make_idesc(N_TILE);
         constexpr uint32_t desc_hi = (1024u >> 4) | (1u << 14) | (2u << 29);
         Ring ra, rx, rd;
         TsCursor cur;
         cur.init(L, u_begin, n_units);
+        tmem = finish_prologue();
+        depend();
         bool ok = true;
         for (int u = 0; ok && u < n_units; ++u, cur.next(L)) {
             const bool seg_first = cur.seg_first, seg_last = cur.seg_last();
@@ -496,84 +505,75 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_w4a16_tstream_kernel(const
             rx.advance(kXS);
             if (seg_last) rd.advance(2);
         }
-    } else if (warp == 1 || warp == 3) {
+    } else if (warp == 3) {
         // ------------------------------------------------------------------ no role after the prologue
         tmem = finish_prologue();
-    } else if (warp == 2) {
-        // ------------------------------------------------------------------ copy producer
-        // One elected lane of the converged warp issues every TMA copy of the CTA: per slot the
-        // packed weights (16 row groups x kChunkK 32-bit words; one 3-D box, or one 2-D box per
-        // step) into the weight ring, and per unit kChunkK/64 boxes of x (tile_tok tokens x 64
-        // columns, L2 resident; tokens past n and columns past k zero-filled) into the activation
-        // ring, released by the MMAs' commit.  The weights are constants:
-        // the first ring-full of their copies is issued before the dependency wait (and before
-        // this warp joins the rest of the prologue); x may come from the kernel before this one.
-        Ring rw, rn;
-        int sl = 0, w_rb = 0, xu = 0;
-        TsCursor wc, xc;
-        wc.init(L, u_begin, n_units);
+    } else if (warp == kTsXWarp) {
+        // ------------------------------------------------------------------ copy producer of the activations
+        // One elected lane of the converged warp issues, per unit, kChunkK/64 boxes of x (tile_tok tokens x 64
+        // columns, L2 resident; tokens past n and columns past k zero-filled) into the activation ring, released by the
+        // MMAs' commit.
+        Ring rn;
+        TsCursor xc;
         xc.init(L, u_begin, n_units);
-        bool ok = true;
-        auto issue_x = [&](bool blocking) {
-            // as many activation copies as have a free stage (all the outstanding ones if `blocking`)
-            while (ok && xu < n_units) {
-                if (blocking) ok = mbar_wait_warp(x_empty + 8 * rn.idx, rn.phase ^ 1, abort_flag, p.status, 9);
-                else if (!(__all_sync(0xffffffffu, mbar_test_wait(x_empty + 8 * rn.idx, rn.phase ^ 1)) != 0)) break;
-                if (!ok) break;
-                if (elect_one_sync()) {
-                    mbar_expect_tx(x_full + 8 * rn.idx, kXStageBytes);
-#pragma unroll
-                    for (int t = 0; t < kXTiles; ++t)
-                        tma_load_2d(xring + (uint32_t)rn.idx * kXStageBytes + (uint32_t)t * kXTileBytes, &L.g[xc.g].map_x,
-                                    xc.chunk * kChunkK + 64 * t, p.tok0, x_full + 8 * rn.idx);
-                }
-                __syncwarp();
-                rn.advance(kXS);
-                ++xu;
-                xc.next(L);
-            }
-        };
-        auto issue_w_until = [&](int end, bool with_x) {
-            for (; ok && sl < end; ++sl) {
-                if (with_x) issue_x(false);
-                TS_PROF_BEGIN
-                ok = mbar_wait_warp(w_empty + 8 * rw.idx, rw.phase ^ 1, abort_flag, p.status, 1);
-                TS_PROF_END(0)
-                if (!ok) break;
-                if (elect_one_sync()) {
-                    const TsGemm &G = L.g[wc.g];
-                    mbar_expect_tx(w_full + 8 * rw.idx, kSlotBytes);
-                    if (WMODE == 1) {
-                        tma_load_5d(w_stage(rw.idx), &G.map_q, 0, 0, 0, wc.chunk * (STEPS / 2), (wc.tile * RB + w_rb) * 4, w_full + 8 * rw.idx);
-                    } else if (G.q3d) {
-                        tma_load_3d(w_stage(rw.idx), &G.map_q, 0, (wc.tile * RB + w_rb) * 16, wc.chunk * STEPS, w_full + 8 * rw.idx);
-                    } else {
-#pragma unroll
-                        for (int st = 0; st < STEPS; ++st)
-                            tma_load_2d(w_stage(rw.idx) + (uint32_t)st * kStepBytes, &G.map_q, wc.chunk * kChunkK + 32 * st,
-                                        (wc.tile * RB + w_rb) * 16, w_full + 8 * rw.idx);
-                    }
-                }
-                __syncwarp();
-                rw.advance(WS);
-                if (++w_rb == RB) {
-                    w_rb = 0;
-                    wc.next(L);
-                }
-            }
-        };
-        issue_w_until(min(WS, total_slots), false);
-        tmem = finish_prologue();
+        finish_prologue();
         depend();
-        issue_w_until(total_slots, true);
-        issue_x(true);
+        for (int u = 0; u < n_units; ++u, xc.next(L)) {
+            if (!mbar_wait_warp(x_empty + 8 * rn.idx, rn.phase ^ 1, abort_flag, p.status, 9)) break;
+            if (elect_one_sync()) {
+                mbar_expect_tx(x_full + 8 * rn.idx, kXStageBytes);
+#pragma unroll
+                for (int t = 0; t < kXTiles; ++t)
+                    tma_load_2d(xring + (uint32_t)rn.idx * kXStageBytes + (uint32_t)t * kXTileBytes, &L.g[xc.g].map_x,
+                                xc.chunk * kChunkK + 64 * t, p.tok0, x_full + 8 * rn.idx);
+            }
+            __syncwarp();
+            rn.advance(kXS);
+        }
+    } else if (warp == kTsWeightWarp) {
+        // ------------------------------------------------------------------ copy producer of the weights
+        // Per slot one elected lane of the converged warp issues the packed weights (16 row groups x kChunkK 32-bit words;
+        // one 5-D or 3-D box, or one 2-D box per step) into the weight ring.  The weights are constants:
+        // the first ring-full of their copies is issued before the dependency wait.
+        asm volatile("bar.arrive 1, %0;" ::"n"(kTsThreads) : "memory");
+        Ring rw;
+        int w_rb = 0;
+        TsCursor wc;
+        wc.init(L, u_begin, n_units);
+        for (int sl = 0; sl < total_slots; ++sl) {
+            if (sl == WS) depend();
+            TS_PROF_BEGIN
+            const bool ok = mbar_wait_warp(w_empty + 8 * rw.idx, rw.phase ^ 1, abort_flag, p.status, 1);
+            TS_PROF_END(0)
+            if (!ok) break;
+            if (elect_one_sync()) {
+                const TsGemm &G = L.g[wc.g];
+                mbar_expect_tx(w_full + 8 * rw.idx, kSlotBytes);
+                if (WMODE == 1) {
+                    tma_load_5d(w_stage(rw.idx), &G.map_q, 0, 0, 0, wc.chunk * (STEPS / 2), (wc.tile * RB + w_rb) * 4, w_full + 8 * rw.idx);
+                } else if (G.q3d) {
+                    tma_load_3d(w_stage(rw.idx), &G.map_q, 0, (wc.tile * RB + w_rb) * 16, wc.chunk * STEPS, w_full + 8 * rw.idx);
+                } else {
+#pragma unroll
+                    for (int st = 0; st < STEPS; ++st)
+                        tma_load_2d(w_stage(rw.idx) + (uint32_t)st * kStepBytes, &G.map_q, wc.chunk * kChunkK + 32 * st,
+                                    (wc.tile * RB + w_rb) * 16, w_full + 8 * rw.idx);
+                }
+            }
+            __syncwarp();
+            rw.advance(WS);
+            if (++w_rb == RB) {
+                w_rb = 0;
+                wc.next(L);
+            }
+        }
     } else if (warp < kTsDequantWarp0) {
         // ------------------------------------------------------------------ epilogue
-        tmem = finish_prologue();
-        depend();
         Ring rd;
         TsCursor cur;
         cur.init(L, u_begin, n_units);
+        tmem = finish_prologue();
+        depend();
         int u = 0;
         while (u < n_units) {
             // the segment: chunks [c0, c1) of tile `tile` of GEMM `cur.g`
