@@ -1,0 +1,81 @@
+"""The native front of `matmul`: what it takes, what it leaves to the Python checks, and the workspaces it uses."""
+
+import threading
+
+import pytest
+import torch
+
+import tuna_b200
+from oracle import tuna_oracle as orc
+from tests.gpu_util import check_parity, make_case
+from tuna_b200 import _lib
+
+M, N, K = 64, 3, 128
+
+
+def _args(device):
+    return {"x": torch.zeros((N, K), dtype=torch.float16, device=device), "q": torch.zeros((M // 8, K // 8, 32), dtype=torch.uint8, device=device),
+            "s": torch.ones(M, device=device), "c": torch.linspace(-1, 1, 16, device=device),
+            "o": torch.empty((N, M), dtype=torch.float16, device=device), "m": M, "n": N, "k": K}
+
+
+def test_leaves_everything_unusual_to_python():
+    call = _lib.load_fast_call().matmul
+    a = _args("cpu")
+    for args in ((), (1, 2, 3, 4, 5, 6, 7, 8), tuple(a.values()), (*list(a.values())[:5], 1 << 70, 3, 8), (*list(a.values())[:5], 64.0, 3, 128)):
+        assert call(*args) is False
+
+
+class _Sub(torch.Tensor):
+    pass
+
+
+BAD = {"cpu x": ("x", lambda t: t.cpu()), "type of x": ("x", lambda t: t.float()), "strides of x": ("x", lambda t: t.t().contiguous().t()),
+       "size of q": ("q", lambda t: t[1:]), "no tensor": ("s", lambda t: 1.0), "type of c": ("c", lambda t: t.half()), "size of o": ("o", lambda t: t[:, 1:].contiguous()),
+       "m": ("m", lambda v: 68), "n": ("n", lambda v: -3), "k": ("k", lambda v: 0)}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("what", BAD)
+def test_bad_arguments_raise_what_the_python_checks_raise(what):
+    a = _args("cuda")
+    ws = tuna_b200.workspace_for(M, N, K, a["x"].device)
+    tuna_b200.matmul(*a.values())  # a workspace is registered: the native way is open
+    assert _lib.load_fast_call().matmul(*a.values()) is True
+    name, change = BAD[what]
+    a[name] = change(a[name])
+    assert _lib.load_fast_call().matmul(*a.values()) is False
+    raised = []
+    for kw in ({}, {"workspace": ws}):  # with a workspace of its own a call takes the Python way
+        with pytest.raises(Exception) as e:
+            tuna_b200.matmul(*a.values(), **kw)
+        raised.append((e.type, str(e.value)))
+    assert raised[0] == raised[1]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shapes", [[(64, 3, 128), (4096, 17, 4104), (40000, 5, 64), (64, 3, 128)], [(512, 300, 512), (64, 1, 8)]])
+def test_streams_threads_and_growing_workspaces(shapes):
+    """The same GEMMs on the default stream, on two streams of their own and from threads, small shapes before large ones."""
+    errors = []
+
+    def work(stream):
+        try:
+            with torch.cuda.stream(stream):
+                for m, n, k in shapes:
+                    host, (x, q, s, c) = make_case(m, n, k, m + n)
+                    for xs in (x, x.as_subclass(_Sub)):  # a subclass takes the Python way
+                        o = torch.full((n, m), float("nan"), dtype=torch.float16, device="cuda")
+                        tuna_b200.matmul(xs, q, s, c, o, m, n, k)
+                        stream.synchronize()
+                        check_parity(o.cpu().numpy(), orc.matmul_ref(*host, m, n, k), 1e-2)
+        except BaseException as e:  # noqa: BLE001
+            errors.append(e)
+
+    work(torch.cuda.current_stream())
+    threads = [threading.Thread(target=work, args=(torch.cuda.Stream(),)) for _ in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors[0]

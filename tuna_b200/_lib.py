@@ -106,6 +106,23 @@ def load():
     return _lib
 
 
+_fast_call = None
+
+
+def load_fast_call():
+    """The extension module that checks and launches the common case of `ops.matmul`, bound to the library."""
+    global _fast_call
+    if _fast_call is None:
+        lib = load()
+        try:
+            from . import _fast_call as module
+        except ImportError as e:
+            raise ImportError("tuna_b200/_fast_call.so is missing or does not fit this torch: build it with `python -m tuna_b200.build`") from e
+        module.bind(ctypes.cast(lib.tuna_matmul, c_void_p).value)
+        _fast_call = module
+    return _fast_call
+
+
 class TunaError(RuntimeError):
     def __init__(self, status: int):
         self.status = status

@@ -10,12 +10,14 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
 HERE = Path(__file__).resolve().parent
 CSRC = HERE / "csrc"
 LIB = HERE / "libtuna_b200.so"
+FAST_CALL = HERE / "_fast_call.so"
 SOURCES = ["tuna_api.cu", "host_util.cu", "dequant_sm100a.cu", "quantize_sm100a.cu", "gemm_stream_sm100a.cu", "gemm_tstream_sm100a.cu", "gemm_pair_sm100a.cu", "exchange_sm100a.cu", "ref_symbols.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -70,7 +72,26 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         if r.returncode:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("link failed")
+    _build_fast_call(force)
     return LIB
+
+
+def _build_fast_call(force: bool) -> None:
+    """The native front of `ops.matmul` (csrc/fast_call.cpp): an extension module against the headers of the torch it runs with."""
+    src = CSRC / "fast_call.cpp"
+    if not force and not _stale(FAST_CALL, [src]):
+        return
+    import torch
+
+    root = Path(torch.__file__).resolve().parent
+    cuda = Path(_nvcc()).resolve().parent.parent if os.path.sep in _nvcc() else Path("/usr/local/cuda")
+    include = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include", cuda / "include", sysconfig.get_paths()["include"]]
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *(f"-I{p}" for p in include), str(src), "-o", str(FAST_CALL), f"-L{root / 'lib'}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode:
+        sys.stderr.write(r.stdout + r.stderr)
+        raise RuntimeError("the build of fast_call.cpp failed")
 
 
 if __name__ == "__main__":

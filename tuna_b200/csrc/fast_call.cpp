@@ -1,0 +1,101 @@
+// The argument checks and the launch of `ops.matmul` in one native call.  In Python they take 8 us of host time, more than the
+// kernel of a small layer (4096x4096 at 1 token 6.8 us), so a decode step's small GEMMs waited for the host.
+//
+// matmul(x, q, s, c, o, m, n, k) answers True when the GEMM was launched and False when anything is not as the
+// common case has it - a wrong type, device, layout or size, no workspace yet, one too small, a status that is
+// not TUNA_OK.  Nothing has been launched then, and ops.py takes the call through its own checks, which raise what is wrong.
+#include <torch/csrc/autograd/python_variable.h>
+#include <ATen/core/Tensor.h>
+#include <c10/cuda/CUDAStream.h>
+#include <c10/cuda/CUDAFunctions.h>
+#include <map>
+#include <utility>
+
+namespace {
+
+using MatmulFn = int (*)(const void *q, const void *x, const void *code, const void *absmax, void *o, int m, int n, int k, void *workspace,
+                         size_t workspace_bytes, void *stream);
+
+MatmulFn g_matmul = nullptr;
+
+struct Workspace {
+    void *ptr;
+    size_t bytes;
+};
+// By device and stream, as ops.py keeps the tensors themselves (it registers each one it allocates, and keeps it alive).  Every access holds the GIL.
+std::map<std::pair<int, void *>, Workspace> g_workspaces;
+
+// The tensor of `o` if it is a plain contiguous CUDA tensor of `numel` elements of `type` on `device` (-1: any), else null.
+const at::Tensor *plain(PyObject *o, at::ScalarType type, int64_t numel, int device)
+{
+    if (!THPVariable_CheckExact(o)) return nullptr;  // subclasses take the Python way
+    const at::Tensor &t = THPVariable_Unpack(o);
+    if (!t.defined() || !t.is_cuda() || t.scalar_type() != type || t.layout() != at::kStrided || t.numel() != numel || !t.is_contiguous()) return nullptr;
+    if (device >= 0 && t.get_device() != device) return nullptr;
+    return &t;
+}
+
+bool launch(PyObject *const *args)
+{
+    long long dim[3];
+    for (int i = 0; i < 3; ++i) {
+        if (!PyLong_CheckExact(args[5 + i])) return false;
+        int overflow = 0;
+        dim[i] = PyLong_AsLongLongAndOverflow(args[5 + i], &overflow);
+        if (overflow || dim[i] <= 0 || dim[i] > 0x7fffffff) return false;
+    }
+    const long long m = dim[0], n = dim[1], k = dim[2];
+    const at::Tensor *x = plain(args[0], at::kHalf, n * k, -1);
+    if (!x) return false;
+    const int device = x->get_device();
+    const at::Tensor *q = plain(args[1], at::kByte, m * k / 2, device), *s = plain(args[2], at::kFloat, m, device),
+                     *c = plain(args[3], at::kFloat, 16, device), *o = plain(args[4], at::kHalf, n * m, device);
+    if (!q || !s || !c || !o || device != c10::cuda::current_device()) return false;
+    void *stream = c10::cuda::getCurrentCUDAStream(device).stream();
+    const auto ws = g_workspaces.find({device, stream});
+    if (ws == g_workspaces.end()) return false;
+    const int st = g_matmul(q->const_data_ptr(), x->const_data_ptr(), c->const_data_ptr(), s->const_data_ptr(), o->mutable_data_ptr(), (int)m, (int)n,
+                            (int)k, ws->second.ptr, ws->second.bytes, stream);
+    return st == 0;
+}
+
+PyObject *fast_matmul(PyObject *, PyObject *const *args, Py_ssize_t nargs)
+{
+    bool done = false;
+    try {
+        done = nargs == 8 && g_matmul && launch(args);
+    } catch (...) {  // a tensor without storage of its own (vmap, a trace): the Python way says what is wrong
+    }
+    return PyBool_FromLong(done);
+}
+
+// set_workspace(device, stream, pointer, bytes)
+PyObject *set_workspace(PyObject *, PyObject *args)
+{
+    int device;
+    unsigned long long stream, ptr, bytes;
+    if (!PyArg_ParseTuple(args, "iKKK", &device, &stream, &ptr, &bytes)) return nullptr;
+    g_workspaces[{device, (void *)stream}] = {(void *)ptr, (size_t)bytes};
+    Py_RETURN_NONE;
+}
+
+// bind(address of tuna_matmul)
+PyObject *bind(PyObject *, PyObject *args)
+{
+    unsigned long long fn;
+    if (!PyArg_ParseTuple(args, "K", &fn)) return nullptr;
+    g_matmul = (MatmulFn)fn;
+    Py_RETURN_NONE;
+}
+
+PyMethodDef methods[] = {
+    {"matmul", (PyCFunction)(void (*)(void))fast_matmul, METH_FASTCALL, nullptr},
+    {"set_workspace", set_workspace, METH_VARARGS, nullptr},
+    {"bind", bind, METH_VARARGS, nullptr},
+    {nullptr, nullptr, 0, nullptr},
+};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_fast_call", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__fast_call() { return PyModule_Create(&module); }

@@ -69,6 +69,8 @@ def workspace_for(m: int, n: int, k: int, device) -> torch.Tensor:
     if ws is None or ws.numel() < need:
         ws = torch.zeros(max(need, 1 << 20), dtype=torch.uint8, device=device)
         _workspaces[key] = ws
+        if device.index is not None:  # the one that a native call on this device and stream uses
+            _lib.load_fast_call().set_workspace(device.index, key[1], ws.data_ptr(), ws.numel())
     return ws
 
 
@@ -87,6 +89,16 @@ def lookup_config(m: int, n: int, k: int) -> TunaConfig:
     return cfg
 
 
+def _bind_fast_matmul(*args):
+    """The first call: loads the native front of `matmul` and puts it in this function's place."""
+    global _fast_matmul
+    _fast_matmul = _lib.load_fast_call().matmul
+    return _fast_matmul(*args)
+
+
+_fast_matmul = _bind_fast_matmul
+
+
 def matmul(x, q, s, c, o, m: int, n: int, k: int, *, config: TunaConfig | None = None, workspace=None) -> None:
     """`tuna.matmul(x, q, s, c, o, m, n, k)` (extension.cpp:26-38).
 
@@ -94,6 +106,8 @@ def matmul(x, q, s, c, o, m: int, n: int, k: int, *, config: TunaConfig | None =
     (codebook); o fp16 [n,m], overwritten.  Enqueued on the current stream of
     x's device.
     """
+    if config is None and workspace is None and _fast_matmul(x, q, s, c, o, m, n, k):
+        return  # the common case, checked and launched natively; anything else comes through here
     dev = x.device if isinstance(x, torch.Tensor) else None
     _expect(x, "x", torch.float16, n * k)
     _expect(q, "q", torch.uint8, m * k // 2, dev)
