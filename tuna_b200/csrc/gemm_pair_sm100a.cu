@@ -451,6 +451,11 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
                 if (++c == p.chunks) c = 0;
             }
         }
+        // The MMAs' commits arrive at both CTAs' barriers: neither leaves before the last ones have, one per stage in use.
+        for (int i = min(S, total); ok && i > 0; --i, ru.advance(S)) {
+            if (total < S && i == total) ru = Ring();
+            ok = mbar_wait_warp(u_empty + 8 * ru.idx, total < S ? 0u : ru.phase ^ 1, abort_flag, p.status, 110);
+        }
     } else if (warp == 3) {
         tmem = finish_prologue();
     } else if (warp < kPairDequantWarp0) {
@@ -547,8 +552,7 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
             }
             rd.advance(p.nd);
         }
-        // the stores have read the staging tile; the end of the kernel makes them visible
-        if (threadIdx.x == 32 * kPairEpilogueWarp0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        if (threadIdx.x == 32 * kPairEpilogueWarp0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     } else {
         // ------------------------------------------------------------------ dequant
         tmem = finish_prologue();
