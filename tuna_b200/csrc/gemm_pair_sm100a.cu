@@ -659,9 +659,11 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
 // ------------------------------------------------------------------ host side
 
 // Microseconds per 16 columns of K of a tile of `tok` tokens: the wavefronts of shared memory (see the head of the
-// file) at the 1.7 GHz of a short run, or the tensor pipe's N/2 clocks, and what the dequantisation adds to them, at the
-// clock the power cap leaves it (measured at K = 4096: 14 us a wave of 128-token tiles, 22 of 224, 25 of 256).
-static double pair_step_us(int tok) { return std::max((tok / 4 + 61) / 1700.0, (tok / 2 + 8) / 1420.0); }
+// file; with 16 dequant warps 54 beside the activations' instead of 61) at the 1.7 GHz of a short run, or the tensor pipe's N/2 clocks, and
+// what the dequantisation adds to them, at the clock the power cap leaves it (measured at K = 4096: 14 us a wave of 128-token tiles, 22 of
+// 224, 25 of 256).  The line between many waves of 128 tokens and fewer of wider tiles follows from it: 29568x8320 at 243 tokens 98 us in tiles of 128,
+// 118 of 256; 20608x8576 at 497 134 and 143; 8704x27264 at 195 89 and (224) 93; 1280x28544 at 398 36 and (160) 33.
+static double pair_step_us(int tok) { return std::max((tok / 4 + 54) / 1700.0, (tok / 2 + 8) / 1420.0); }
 
 // 16 dequant warps where they bound the tile, i.e. as long as the tensor pipe needs fewer clocks per step than the table
 // lookups and what goes with them; with them comes the table that one instruction per lookup addresses (pair_lookup), which leaves
@@ -680,9 +682,17 @@ struct PairSplit {
 };
 
 // What cutting costs beyond the work itself: partial sums written, an arrival, partial sums read by the finishing
-// CTA.  Measured (us, 2 to 8 segments): 32-token tiles 6 to 7, 64 4 to 8, 128 8 to 11, 256 14 to 20; an uncut launch 0.5 to 4.
-static double pair_cut_us(int tile_tok, int segs) { return 5.0 + 0.025 * tile_tok + 0.05 * std::max(0, tile_tok - 128) + segs * (0.25 + 0.002 * tile_tok); }
-constexpr double kPairUncutUs = 1.5;
+// CTA.  Measured (us, 2 to 10 segments): 32-token tiles 6 to 7, 64 4 to 8, 128 12 to 18 (more pieces than warps), 256 14 to 20; an uncut launch
+// 0.5 to 4.  Where whole tiles follow the cut ones, adding up hides behind them.
+static double pair_cut_us(int tile_tok, int segs, bool hidden)
+{
+    const double adding = hidden ? 0.05 * std::max(0, tile_tok - 128) : 0.06 * std::max(0, std::min(tile_tok, 160) - 64) + 0.01 * std::max(0, tile_tok - 160);
+    return 5.0 + 0.025 * tile_tok + adding + segs * (0.25 + 0.002 * tile_tok);
+}
+constexpr double kPairUncutUs = 0.9;
+// What a wave of whole tiles costs beside its steps: the epilogue, where there is one accumulator buffer only (pair_plan), else the turn from
+// one tile to the next.  33280x1408 at 2025 tokens: 139 us in tiles of 160, 167 of 256; 29312x512 at 292 four waves of 160 12.6, five of 128 14.1.
+static double pair_wave_us(int tile_tok) { return tile_tok > 192 ? 1.0 : 0.3; }
 
 static PairSplit pair_split(int m, int n, int k, int tile_tok, int pairs)
 {
@@ -694,16 +704,19 @@ static PairSplit pair_split(int m, int n, int k, int tile_tok, int pairs)
     const double work_us = row_tiles * (full * tile_us + last_us) / pairs;   // per pair, evenly cut
     const long long waves = tiles / pairs;
     const int rest = (int)(tiles - waves * pairs);
-    PairSplit best = {0, 0, kPairUncutUs + (waves == 0 ? tile_us : (waves + (rest ? 1 : 0)) * (work_us * pairs / tiles))};
+    const double wave_end = pair_wave_us(tile_tok);
+    // a wave of tiles of two widths takes as long as something between their mean and the wider one
+    const double wave_us = 0.5 * (tile_us + work_us * pairs / tiles) + wave_end;
+    PairSplit best = {0, 0, kPairUncutUs + (waves == 0 ? tile_us + wave_end : (waves + (rest ? 1 : 0)) * wave_us)};
     auto consider = [&](int sk_tiles, int sk_pairs, double us) {
         if (us < best.us) best = {sk_tiles, sk_pairs, us};
     };
-    if (rest > 0 && waves > 0) consider(pairs + rest, pairs, work_us + pair_cut_us(tile_tok, 2));
+    if (rest > 0 && waves > 0) consider(pairs + rest, pairs, work_us + waves * wave_end + pair_cut_us(tile_tok, 2, waves > 1));
     if (waves == 0) {
         int s = 2;
-        for (; s * tiles <= pairs && s <= chunks; ++s) consider((int)tiles, s * (int)tiles, tile_us / s + pair_cut_us(tile_tok, s));
+        for (; s * tiles <= pairs && s <= chunks; ++s) consider((int)tiles, s * (int)tiles, tile_us / s + pair_cut_us(tile_tok, s, false));
         // all pairs, where whole segments leave more than a tenth of them idle
-        if (s <= chunks && (s - 1) * tiles * 10 < pairs * 9) consider((int)tiles, pairs, work_us + pair_cut_us(tile_tok, s + 1));
+        if (s <= chunks && (s - 1) * tiles * 10 < pairs * 9) consider((int)tiles, pairs, work_us + pair_cut_us(tile_tok, s + 1, false) + 0.03 * tile_tok);
     }
     return best;
 }
