@@ -37,9 +37,10 @@
 //                The warp stays converged and one elected lane issues (a lone diverged thread
 //                running this loop needed ~80 clocks per MMA instead of ~12); a slot is 8 or 16
 //                MMAs per wait and commit, because that fixed cost per slot is what limits it
-//   warps 1, 3   idle (they only help to build the lookup table)
-//   warp 2       copy producer: TMA boxes of packed weights into the weight ring and of x (fp16
-//                [n,k], L2 resident; one box per 64 columns) into the activation ring
+//   warp 1       copy producer of x (fp16 [n,k], L2 resident; one box per 64 columns) into the activation ring
+//   warp 2       copy producer of the packed weights (TMA boxes into the weight ring); it initialises the barriers and issues the
+//                first ring-full ahead of everything: 2000 clocks that the others waited for (4096x4096 at 1 token 7.3 -> 6.8 us a call)
+//   warp 3       no role
 //   warps 4-7    epilogue: tcgen05.ld of the accumulator, fp32 scale by absmax, fp16 store,
 //                split-K partials and fix-up
 //   warps 8-23   dequant: ld.shared.u32 -> prmt + ld.shared table lookups -> tcgen05.st into the A
@@ -57,7 +58,7 @@
 // result does not depend on arrival order (the reference adds fp16 partials with atomicAdd, kernel.cu:2739-2745).  No
 // floating-point atomics, no zero-filled output.  This tail is what a single small GEMM waits for: at 28672x4096 and 16
 // tokens the last MMA was done at 16.7 us of 24.1.  Hence only token groups that exist are exchanged, one
-// acquire-release atomic per warp replaces two fences, and at the end of the range all 24 warps add up the tile, four
+// acquire-release atomic per warp replaces two fences, and at the end of the range all 24 warps add up the tile, eight
 // tokens of 32 rows each, instead of four warps 16 tokens at a time (graph replay, 16 tokens unless said, us):
 // 4096x4096 10.3 -> 9.9, 57344x8192 67.0 -> 65.2, 4096x4096 at 64 tokens 20.1 -> 14.2, 768x4096 at 64 49.7 -> 12.9; with that
 // code in one place only, outside the roles, 4096x4096 7.8, 57344x8192 53.5, 4096x4096 at 64 10.9.
@@ -800,7 +801,7 @@ static void ts_pick_split(int m, int n, int k, int sm_count, tuna_config *c)
             const long long per = (units + ctas - 1) / ctas;
             const bool whole = ctas % tiles == 0 && chunks % (ctas / tiles) == 0;
             double us = per * unit_us;
-            if (whole && ctas == tiles) us = 1.15 * us + 3.6 + 0.2 * groups;  // fewer SMs draw on HBM
+            if (whole && ctas == tiles) us = 1.15 * us + 3.1 + 0.2 * groups;  // fewer SMs draw on HBM
             else if (whole) us += 4.8 + (0.3 + 0.1 * rb) * groups + 0.17 * (ctas / tiles);
             else us += 6.3 + 0.55 * groups + 0.12 * rb * (groups - 1) + 0.17 * (ctas / tiles);
             if (best < 0 || us < best) {
