@@ -434,14 +434,17 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_w4a16_tstream_kernel(const
     };
     // The flagged quarters of a tile whose partials are all there, shared out over warps `w0`, w0 + step, ... : a warp
     // takes eight tokens of 32 rows at a time, so that all of a tile is in flight at once (28672x4096 at 16 tokens, two row blocks: by
-    // four 18.0 us, by eight 17.7), in exchange launches 16, whole sectors of a peer's slab.
+    // four 18.0 us, by eight 17.7), four of them where that takes no second round and there are more than four segments, eight of which
+    // are in flight then (1152x3328 at 11 tokens 6.4 -> 6.0), in exchange launches 16, whole sectors of a peer's slab.
     auto finish_tile = [&](const TsGemm &G, int tile, int first, int nseg, const int *flagged, int w0, int step) __attribute__((always_inline)) {
-        const int groups4 = token_groups(G), per = p.n_peers > 0 ? 4 : 2, rb_shift = RB >> 1;
+        const int groups4 = token_groups(G), rb_shift = RB >> 1;
+        const int per = p.n_peers > 0 ? 4 : nseg <= 4 || (groups4 << (2 + rb_shift)) > step ? 2 : 1;
         for (int item = w0; (item >> (2 + rb_shift)) * per < groups4; item += step) {
             const int q = item & 3, rest = item >> 2;
             const int g = (rest >> rb_shift) * per, rb = rest & (RB - 1);  // RB is 1, 2 or 4
             if (!flagged[q]) continue;
-            if (per == 2) add_partials(Int<2>(), Int<4>(), G, tile, first, nseg, q, rb, g, groups4 - 1);
+            if (per == 1) add_partials(Int<1>(), Int<8>(), G, tile, first, nseg, q, rb, g, groups4 - 1);
+            else if (per == 2) add_partials(Int<2>(), Int<4>(), G, tile, first, nseg, q, rb, g, groups4 - 1);
             else add_partials(Int<4>(), Int<2>(), G, tile, first, nseg, q, rb, g, groups4 - 1);
         }
     };
