@@ -33,3 +33,15 @@ def test_looked_up_configuration_gives_the_same_bits(m, k, n):
     st1, by_config, _ = run_matmul(dev, m, n, k, cfg=cfg)
     assert st0 == 0 and st1 == 0
     assert torch.equal(by_default, by_config)
+
+
+# cut tiles that are added up by four tokens (more than four segments, one round of the CTA's warps) and by eight, with a last group alone
+@pytest.mark.parametrize("m,n,k", [(640, 12, 1408), (1152, 11, 3328), (1792, 12, 4224), (888, 2, 8104), (4096, 16, 4096), (2688, 18, 7296), (768, 15, 2304)])
+def test_cut_tiles_added_up_by_four_and_by_eight_tokens(m, n, k):
+    host, dev = make_case(m, n, k, seed=m + n)
+    st, out, holder = run_matmul(dev, m, n, k)
+    assert st == 0
+    check_parity(out.cpu().numpy(), orc.matmul_ref(*host, m, n, k), 1e-2)
+    assert holder.guards_intact()
+    again = run_matmul(dev, m, n, k)[1]
+    assert torch.equal(out, again)
