@@ -1,6 +1,8 @@
 """The native front of `matmul`: what it takes, what it leaves to the Python checks, and the workspaces it uses."""
 
+import ctypes
 import threading
+import weakref
 
 import pytest
 import torch
@@ -8,7 +10,7 @@ import torch
 import tuna_b200
 from oracle import tuna_oracle as orc
 from tests.gpu_util import check_parity, make_case
-from tuna_b200 import _lib
+from tuna_b200 import _lib, ops
 
 M, N, K = 64, 3, 128
 
@@ -79,3 +81,67 @@ def test_streams_threads_and_growing_workspaces(shapes):
     for t in threads:
         t.join()
     assert not errors, errors[0]
+
+
+def test_threads_that_share_a_stream_keep_the_larger_workspace(monkeypatch):
+    """A thread that meets no workspace is held up between allocating a small one and storing it; another one stores a larger one."""
+    small, large, key = 2 << 20, 4 << 20, (0, 0x5EED)
+    allocated, go = threading.Event(), threading.Event()
+    zeros = torch.zeros
+
+    def slow_zeros(size, **kw):
+        t = zeros(size, **kw)
+        if size == small:
+            allocated.set()
+            assert go.wait(20)
+        return t
+
+    monkeypatch.setattr(ops, "_stream_ptr", lambda device: key[1])
+    monkeypatch.setattr(ops, "_workspace_bytes", lambda index, m, n, k: m)
+    monkeypatch.setattr(ops.torch, "zeros", slow_zeros)
+    got = []
+    thread = threading.Thread(target=lambda: got.append(ops.workspace_for(small, 1, 1, "cpu:0")))
+    try:
+        thread.start()
+        assert allocated.wait(20)
+        got.append(ops.workspace_for(large, 1, 1, "cpu:0"))
+        go.set()
+        thread.join(20)
+        assert len(got) == 2 and got[0].numel() == got[1].numel() == large
+        assert got[0] is got[1] is _lib.workspaces[key]
+        assert _lib.load_fast_call().workspace(*key) == (got[0].data_ptr(), large)  # what a native launch is given
+        ops.workspace_for(8 << 20, 1, 1, "cpu:0")
+        assert _lib.load_fast_call().workspace(*key) == (_lib.workspaces[key].data_ptr(), 8 << 20)
+    finally:
+        go.set()
+        _lib.workspaces.pop(key, None)
+    assert _lib.load_fast_call().workspace(*key) is None
+
+
+@pytest.fixture
+def stub():
+    """Puts a function in the place of tuna_matmul: nothing is launched."""
+    fast = _lib.load_fast_call()
+    yield lambda address: fast.bind(address, _lib.workspaces)
+    fast.bind(ctypes.cast(_lib.load().tuna_matmul, ctypes.c_void_p).value, _lib.workspaces)
+
+
+@pytest.mark.gpu
+def test_a_launch_holds_the_workspace_it_was_given(stub):
+    a = _args("cuda")
+    tuna_b200.matmul(*a.values())
+    key = (0, torch.cuda.current_stream().cuda_stream)
+    seen = []
+
+    def replaced_meanwhile(*args):
+        ref, size = weakref.ref(_lib.workspaces[key]), _lib.workspaces[key].numel()
+        seen.append((args[8], args[9]) == (ref().data_ptr(), size))
+        _lib.workspaces[key] = torch.zeros(size, dtype=torch.uint8, device="cuda")
+        seen.append(ref() is not None)
+        return 0
+
+    proto = ctypes.CFUNCTYPE(ctypes.c_int, *([ctypes.c_void_p] * 5), *([ctypes.c_int] * 3), ctypes.c_void_p, ctypes.c_size_t, ctypes.c_void_p)
+    callback = proto(replaced_meanwhile)
+    stub(ctypes.cast(callback, ctypes.c_void_p).value)
+    assert _lib.load_fast_call().matmul(*a.values()) is True
+    assert seen == [True, True]

@@ -107,6 +107,9 @@ def load():
 
 
 _fast_call = None
+# (device index, stream) -> the workspace tensor of `matmul` there.  ops.py fills it and both ways of a call look it up here, each
+# holding the tensor while it uses it, so that a larger one may take its place at any time.
+workspaces: dict = {}
 
 
 def load_fast_call():
@@ -118,7 +121,7 @@ def load_fast_call():
             from . import _fast_call as module
         except ImportError as e:
             raise ImportError("tuna_b200/_fast_call.so is missing or does not fit this torch: build it with `python -m tuna_b200.build`") from e
-        module.bind(ctypes.cast(lib.tuna_matmul, c_void_p).value)
+        module.bind(ctypes.cast(lib.tuna_matmul, c_void_p).value, workspaces)
         _fast_call = module
     return _fast_call
 

@@ -8,8 +8,6 @@
 #include <ATen/core/Tensor.h>
 #include <c10/cuda/CUDAStream.h>
 #include <c10/cuda/CUDAFunctions.h>
-#include <map>
-#include <utility>
 
 namespace {
 
@@ -17,13 +15,26 @@ using MatmulFn = int (*)(const void *q, const void *x, const void *code, const v
                          size_t workspace_bytes, void *stream);
 
 MatmulFn g_matmul = nullptr;
+PyObject *g_workspaces = nullptr;  // the dict (device, stream) -> tensor that ops.py fills: there is no other record of them
 
+// The workspace of a device and stream, with a reference of the caller's own: another thread may put a larger one in its
+// place while this one is in use.  Null where there is none.
 struct Workspace {
-    void *ptr;
-    size_t bytes;
+    PyObject *tensor = nullptr;
+    Workspace(int device, void *stream)
+    {
+        PyObject *key = Py_BuildValue("(iK)", device, (unsigned long long)stream);
+        PyObject *found = key ? PyDict_GetItemWithError(g_workspaces, key) : nullptr;
+        Py_XDECREF(key);
+        if (found && THPVariable_Check(found)) tensor = Py_NewRef(found);
+        PyErr_Clear();
+    }
+    ~Workspace() { Py_XDECREF(tensor); }
+    Workspace(const Workspace &) = delete;
+    Workspace &operator=(const Workspace &) = delete;
+    void *ptr() const { return THPVariable_Unpack(tensor).mutable_data_ptr(); }
+    size_t bytes() const { return THPVariable_Unpack(tensor).nbytes(); }
 };
-// By device and stream, as ops.py keeps the tensors themselves (it registers each one it allocates, and keeps it alive).  Every access holds the GIL.
-std::map<std::pair<int, void *>, Workspace> g_workspaces;
 
 // The tensor of `o` if it is a plain contiguous CUDA tensor of `numel` elements of `type` on `device` (-1: any), else null.
 const at::Tensor *plain(PyObject *o, at::ScalarType type, int64_t numel, int device)
@@ -52,10 +63,10 @@ bool launch(PyObject *const *args)
                      *c = plain(args[3], at::kFloat, 16, device), *o = plain(args[4], at::kHalf, n * m, device);
     if (!q || !s || !c || !o || device != c10::cuda::current_device()) return false;
     void *stream = c10::cuda::getCurrentCUDAStream(device).stream();
-    const auto ws = g_workspaces.find({device, stream});
-    if (ws == g_workspaces.end()) return false;
+    const Workspace ws(device, stream);
+    if (!ws.tensor) return false;
     const int st = g_matmul(q->const_data_ptr(), x->const_data_ptr(), c->const_data_ptr(), s->const_data_ptr(), o->mutable_data_ptr(), (int)m, (int)n,
-                            (int)k, ws->second.ptr, ws->second.bytes, stream);
+                            (int)k, ws.ptr(), ws.bytes(), stream);
     return st == 0;
 }
 
@@ -69,28 +80,32 @@ PyObject *fast_matmul(PyObject *, PyObject *const *args, Py_ssize_t nargs)
     return PyBool_FromLong(done);
 }
 
-// set_workspace(device, stream, pointer, bytes)
-PyObject *set_workspace(PyObject *, PyObject *args)
+// workspace(device, stream) -> (address, bytes) of the one that a launch there uses, or None
+PyObject *workspace(PyObject *, PyObject *args)
 {
     int device;
-    unsigned long long stream, ptr, bytes;
-    if (!PyArg_ParseTuple(args, "iKKK", &device, &stream, &ptr, &bytes)) return nullptr;
-    g_workspaces[{device, (void *)stream}] = {(void *)ptr, (size_t)bytes};
-    Py_RETURN_NONE;
+    unsigned long long stream;
+    if (!PyArg_ParseTuple(args, "iK", &device, &stream)) return nullptr;
+    if (!g_workspaces) Py_RETURN_NONE;
+    const Workspace ws(device, (void *)stream);
+    if (!ws.tensor) Py_RETURN_NONE;
+    return Py_BuildValue("(KK)", (unsigned long long)ws.ptr(), (unsigned long long)ws.bytes());
 }
 
-// bind(address of tuna_matmul)
+// bind(address of tuna_matmul, dict of the workspaces)
 PyObject *bind(PyObject *, PyObject *args)
 {
     unsigned long long fn;
-    if (!PyArg_ParseTuple(args, "K", &fn)) return nullptr;
+    PyObject *workspaces;
+    if (!PyArg_ParseTuple(args, "KO!", &fn, &PyDict_Type, &workspaces)) return nullptr;
     g_matmul = (MatmulFn)fn;
+    Py_XSETREF(g_workspaces, Py_NewRef(workspaces));
     Py_RETURN_NONE;
 }
 
 PyMethodDef methods[] = {
     {"matmul", (PyCFunction)(void (*)(void))fast_matmul, METH_FASTCALL, nullptr},
-    {"set_workspace", set_workspace, METH_VARARGS, nullptr},
+    {"workspace", workspace, METH_VARARGS, nullptr},
     {"bind", bind, METH_VARARGS, nullptr},
     {nullptr, nullptr, 0, nullptr},
 };

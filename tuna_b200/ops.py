@@ -11,13 +11,15 @@ from __future__ import annotations
 import contextlib
 import ctypes
 import functools
+import threading
 
 import torch
 
 from . import _lib
 from ._lib import TunaConfig, check
 
-_workspaces: dict = {}
+_workspaces = _lib.workspaces
+_workspaces_lock = threading.Lock()
 
 
 def _stream_ptr(device) -> int:
@@ -68,9 +70,12 @@ def workspace_for(m: int, n: int, k: int, device) -> torch.Tensor:
     ws = _workspaces.get(key)
     if ws is None or ws.numel() < need:
         ws = torch.zeros(max(need, 1 << 20), dtype=torch.uint8, device=device)
-        _workspaces[key] = ws
-        if device.index is not None:  # the one that a native call on this device and stream uses
-            _lib.load_fast_call().set_workspace(device.index, key[1], ws.data_ptr(), ws.numel())
+        with _workspaces_lock:  # threads that share the stream may have allocated meanwhile: the largest stays
+            now = _workspaces.get(key)
+            if now is None or now.numel() < ws.numel():
+                _workspaces[key] = ws
+            else:
+                ws = now
     return ws
 
 
