@@ -1,6 +1,7 @@
 """The native front of `matmul`: what it takes, what it leaves to the Python checks, and the workspaces it uses."""
 
 import ctypes
+import subprocess
 import threading
 import weakref
 
@@ -145,3 +146,31 @@ def test_a_launch_holds_the_workspace_it_was_given(stub):
     stub(ctypes.cast(callback, ctypes.c_void_p).value)
     assert _lib.load_fast_call().matmul(*a.values()) is True
     assert seen == [True, True]
+
+
+@pytest.mark.gpu
+def test_other_threads_run_while_a_launch_waits(stub, tmp_path):
+    """A launch that waits (the stream's queue is full) for what another Python thread does."""
+    src, so = tmp_path / "wait.c", tmp_path / "wait.so"
+    src.write_text("#include <unistd.h>\nvolatile int entered, go;\n"
+                   "int wait_for_go(void) { entered = 1; for (int i = 0; i < 500; ++i) { if (go) return 0; usleep(10000); } return 99; }\n")
+    subprocess.run(["gcc", "-shared", "-fPIC", str(src), "-o", str(so)], check=True)
+    lib = ctypes.CDLL(str(so))
+    entered, go = (ctypes.c_int.in_dll(lib, name) for name in ("entered", "go"))
+    a = _args("cuda")
+    tuna_b200.matmul(*a.values())
+    stop = threading.Event()
+
+    def other():
+        while not entered.value and not stop.wait(0.001):
+            pass
+        go.value = 1
+
+    thread = threading.Thread(target=other)
+    thread.start()
+    try:
+        stub(ctypes.cast(lib.wait_for_go, ctypes.c_void_p).value)
+        assert _lib.load_fast_call().matmul(*a.values()) is True
+    finally:
+        stop.set()
+        thread.join()

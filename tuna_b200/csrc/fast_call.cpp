@@ -36,6 +36,13 @@ struct Workspace {
     size_t bytes() const { return THPVariable_Unpack(tensor).nbytes(); }
 };
 
+// The interpreter lock is released for this object's life: a launch waits where the stream's queue is full, and other
+// threads - one of which may be what the stream waits for - have to run meanwhile.
+struct Unlocked {
+    PyThreadState *state = PyEval_SaveThread();
+    ~Unlocked() { PyEval_RestoreThread(state); }
+};
+
 // The tensor of `o` if it is a plain contiguous CUDA tensor of `numel` elements of `type` on `device` (-1: any), else null.
 const at::Tensor *plain(PyObject *o, at::ScalarType type, int64_t numel, int device)
 {
@@ -65,9 +72,12 @@ bool launch(PyObject *const *args)
     void *stream = c10::cuda::getCurrentCUDAStream(device).stream();
     const Workspace ws(device, stream);
     if (!ws.tensor) return false;
-    const int st = g_matmul(q->const_data_ptr(), x->const_data_ptr(), c->const_data_ptr(), s->const_data_ptr(), o->mutable_data_ptr(), (int)m, (int)n,
-                            (int)k, ws.ptr(), ws.bytes(), stream);
-    return st == 0;
+    const void *qp = q->const_data_ptr(), *xp = x->const_data_ptr(), *cp = c->const_data_ptr(), *sp = s->const_data_ptr();
+    void *op = o->mutable_data_ptr(), *wp = ws.ptr();
+    const size_t bytes = ws.bytes();
+    const MatmulFn matmul = g_matmul;
+    const Unlocked unlocked;  // the caller's arguments and `ws` keep the tensors
+    return matmul(qp, xp, cp, sp, op, (int)m, (int)n, (int)k, wp, bytes, stream) == 0;
 }
 
 PyObject *fast_matmul(PyObject *, PyObject *const *args, Py_ssize_t nargs)
