@@ -122,9 +122,9 @@ def test_threads_that_share_a_stream_keep_the_larger_workspace(monkeypatch):
 @pytest.fixture
 def stub():
     """Puts a function in the place of tuna_matmul: nothing is launched."""
-    fast = _lib.load_fast_call()
+    fast, real = _lib.load_fast_call(), ctypes.cast(_lib.load().tuna_matmul, ctypes.c_void_p).value
     yield lambda address: fast.bind(address, _lib.workspaces)
-    fast.bind(ctypes.cast(_lib.load().tuna_matmul, ctypes.c_void_p).value, _lib.workspaces)
+    fast.bind(real, _lib.workspaces)
 
 
 @pytest.mark.gpu
@@ -174,3 +174,35 @@ def test_other_threads_run_while_a_launch_waits(stub, tmp_path):
     finally:
         stop.set()
         thread.join()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("status,answer", [(0, True), (-4, False), (-6, -6), (-9, -9)])
+def test_a_failed_call_is_not_made_again(stub, monkeypatch, status, answer):
+    """Only a workspace that is too small (-4, before any launch) leaves the call to Python; a call of several passes may have launched some."""
+    a = _args("cuda")
+    tuna_b200.matmul(*a.values())
+    calls = []
+    proto = ctypes.CFUNCTYPE(ctypes.c_int, *([ctypes.c_void_p] * 5), *([ctypes.c_int] * 3), ctypes.c_void_p, ctypes.c_size_t, ctypes.c_void_p)
+    callback = proto(lambda *args: calls.append(args) or status)
+    monkeypatch.setattr(_lib.load(), "tuna_matmul", lambda *args: pytest.fail("the Python way was taken") if status != -4 else 0)
+    stub(ctypes.cast(callback, ctypes.c_void_p).value)
+    assert _lib.load_fast_call().matmul(*a.values()) == answer
+    if status in (0, -4):
+        tuna_b200.matmul(*a.values())
+    else:
+        with pytest.raises(tuna_b200.TunaError) as e:
+            tuna_b200.matmul(*a.values())
+        assert e.value.status == status
+    assert len(calls) == 2
+
+
+@pytest.mark.gpu
+def test_a_misaligned_slice_raises_what_the_python_way_raises():
+    a = _args("cuda")
+    ws = tuna_b200.workspace_for(M, N, K, a["x"].device)
+    a["x"] = torch.zeros(N * K + 1, dtype=torch.float16, device="cuda")[1:].view(N, K)
+    for kw in ({}, {"workspace": ws}):
+        with pytest.raises(tuna_b200.TunaError) as e:
+            tuna_b200.matmul(*a.values(), **kw)
+        assert e.value.status == -3

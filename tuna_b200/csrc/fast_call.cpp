@@ -2,12 +2,14 @@
 // kernel of a small layer (4096x4096 at 1 token 6.8 us), so a decode step's small GEMMs waited for the host.
 //
 // matmul(x, q, s, c, o, m, n, k) answers True when the GEMM was launched and False when anything is not as the
-// common case has it - a wrong type, device, layout or size, no workspace yet, one too small, a status that is
-// not TUNA_OK.  Nothing has been launched then, and ops.py takes the call through its own checks, which raise what is wrong.
+// common case has it - a wrong type, device, layout or size, no workspace yet, one too small.  Nothing has been launched
+// then, and ops.py takes the call through its own checks, which raise what is wrong.  Any other status of the
+// library is the answer itself: a call of several launches may have made some of them, and is not made again.
 #include <torch/csrc/autograd/python_variable.h>
 #include <ATen/core/Tensor.h>
 #include <c10/cuda/CUDAStream.h>
 #include <c10/cuda/CUDAFunctions.h>
+#include "../../include/tuna_b200.h"
 
 namespace {
 
@@ -53,41 +55,44 @@ const at::Tensor *plain(PyObject *o, at::ScalarType type, int64_t numel, int dev
     return &t;
 }
 
-bool launch(PyObject *const *args)
+constexpr int kPythonWay = 1;  // no status of the library: those are negative or TUNA_OK
+
+int launch(PyObject *const *args)
 {
     long long dim[3];
     for (int i = 0; i < 3; ++i) {
-        if (!PyLong_CheckExact(args[5 + i])) return false;
+        if (!PyLong_CheckExact(args[5 + i])) return kPythonWay;
         int overflow = 0;
         dim[i] = PyLong_AsLongLongAndOverflow(args[5 + i], &overflow);
-        if (overflow || dim[i] <= 0 || dim[i] > 0x7fffffff) return false;
+        if (overflow || dim[i] <= 0 || dim[i] > 0x7fffffff) return kPythonWay;
     }
     const long long m = dim[0], n = dim[1], k = dim[2];
     const at::Tensor *x = plain(args[0], at::kHalf, n * k, -1);
-    if (!x) return false;
+    if (!x) return kPythonWay;
     const int device = x->get_device();
     const at::Tensor *q = plain(args[1], at::kByte, m * k / 2, device), *s = plain(args[2], at::kFloat, m, device),
                      *c = plain(args[3], at::kFloat, 16, device), *o = plain(args[4], at::kHalf, n * m, device);
-    if (!q || !s || !c || !o || device != c10::cuda::current_device()) return false;
+    if (!q || !s || !c || !o || device != c10::cuda::current_device()) return kPythonWay;
     void *stream = c10::cuda::getCurrentCUDAStream(device).stream();
     const Workspace ws(device, stream);
-    if (!ws.tensor) return false;
+    if (!ws.tensor) return kPythonWay;
     const void *qp = q->const_data_ptr(), *xp = x->const_data_ptr(), *cp = c->const_data_ptr(), *sp = s->const_data_ptr();
     void *op = o->mutable_data_ptr(), *wp = ws.ptr();
     const size_t bytes = ws.bytes();
     const MatmulFn matmul = g_matmul;
     const Unlocked unlocked;  // the caller's arguments and `ws` keep the tensors
-    return matmul(qp, xp, cp, sp, op, (int)m, (int)n, (int)k, wp, bytes, stream) == 0;
+    const int st = matmul(qp, xp, cp, sp, op, (int)m, (int)n, (int)k, wp, bytes, stream);
+    return st == TUNA_ERR_WORKSPACE ? kPythonWay : st;
 }
 
 PyObject *fast_matmul(PyObject *, PyObject *const *args, Py_ssize_t nargs)
 {
-    bool done = false;
+    int st = kPythonWay;
     try {
-        done = nargs == 8 && g_matmul && launch(args);
+        if (nargs == 8 && g_matmul) st = launch(args);
     } catch (...) {  // a tensor without storage of its own (vmap, a trace): the Python way says what is wrong
     }
-    return PyBool_FromLong(done);
+    return st == TUNA_OK || st == kPythonWay ? PyBool_FromLong(st == TUNA_OK) : PyLong_FromLong(st);
 }
 
 // workspace(device, stream) -> (address, bytes) of the one that a launch there uses, or None

@@ -111,8 +111,12 @@ def matmul(x, q, s, c, o, m: int, n: int, k: int, *, config: TunaConfig | None =
     (codebook); o fp16 [n,m], overwritten.  Enqueued on the current stream of
     x's device.
     """
-    if config is None and workspace is None and _fast_matmul(x, q, s, c, o, m, n, k):
-        return  # the common case, checked and launched natively; anything else comes through here
+    if config is None and workspace is None:
+        done = _fast_matmul(x, q, s, c, o, m, n, k)
+        if done is True:
+            return  # the common case, checked and launched natively
+        if done is not False:
+            check(done)  # an error of the launch itself; where the arguments need a look, the checks below
     dev = x.device if isinstance(x, torch.Tensor) else None
     _expect(x, "x", torch.float16, n * k)
     _expect(q, "q", torch.uint8, m * k // 2, dev)
