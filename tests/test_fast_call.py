@@ -3,6 +3,7 @@
 import ctypes
 import subprocess
 import threading
+import types
 import weakref
 
 import pytest
@@ -11,7 +12,7 @@ import torch
 import tuna_b200
 from oracle import tuna_oracle as orc
 from tests.gpu_util import check_parity, make_case
-from tuna_b200 import _lib, ops
+from tuna_b200 import _lib, build, ops
 
 M, N, K = 64, 3, 128
 
@@ -206,3 +207,54 @@ def test_a_misaligned_slice_raises_what_the_python_way_raises():
         with pytest.raises(tuna_b200.TunaError) as e:
             tuna_b200.matmul(*a.values(), **kw)
         assert e.value.status == -3
+
+
+def _missing():
+    raise ImportError("no such module")
+
+
+FRONTS = {"missing": _missing, "another torch": lambda: types.SimpleNamespace(stamp=_lib.fast_call_stamp() + "1"), "no stamp": lambda: types.SimpleNamespace()}
+
+
+@pytest.fixture
+def unfit_front(request, monkeypatch):
+    _lib.load_fast_call.cache_clear()
+    monkeypatch.setattr(_lib, "_import_fast_call", FRONTS[request.param])
+    monkeypatch.setattr(ops, "_fast_matmul", ops._bind_fast_matmul)
+    yield
+    _lib.load_fast_call.cache_clear()
+
+
+@pytest.mark.parametrize("unfit_front", FRONTS, indirect=True)
+def test_without_a_front_that_fits_the_python_checks_take_the_call(unfit_front):
+    a = _args("cpu")
+    with pytest.warns(RuntimeWarning, match="python -m tuna_b200.build"):
+        with pytest.raises(ValueError, match="must be a CUDA tensor"):
+            tuna_b200.matmul(*a.values())
+    assert _lib.load_fast_call() is None
+
+
+@pytest.mark.gpu
+@pytest.mark.filterwarnings("ignore::RuntimeWarning")
+@pytest.mark.parametrize("unfit_front", FRONTS, indirect=True)
+def test_matmul_without_a_front_that_fits(unfit_front):
+    host, (x, q, s, c) = make_case(64, 3, 128, 1)
+    o = torch.full((3, 64), float("nan"), dtype=torch.float16, device="cuda")
+    tuna_b200.matmul(x, q, s, c, o, 64, 3, 128)
+    check_parity(o.cpu().numpy(), orc.matmul_ref(*host, 64, 3, 128), 1e-2)
+
+
+def test_the_build_makes_a_front_for_another_torch_again(monkeypatch):
+    assert not build._fast_call_stale()
+    monkeypatch.setattr(torch, "__version__", torch.__version__ + "1")
+    assert build._fast_call_stale()
+    monkeypatch.undo()
+    monkeypatch.setattr(build, "FAST_CALL", build.FAST_CALL.with_name("_fast_call.none.so"))
+    assert build._fast_call_stale()
+
+
+def test_the_build_does_without_a_front_that_cannot_be_built(monkeypatch, tmp_path, capsys):
+    monkeypatch.setattr(build, "FAST_CALL", tmp_path / "_fast_call.so")
+    monkeypatch.setenv("CXX", "false")
+    build._build_fast_call(False)
+    assert not build.FAST_CALL.exists() and "not built" in capsys.readouterr().err

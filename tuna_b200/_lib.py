@@ -3,6 +3,9 @@
 from __future__ import annotations
 
 import ctypes
+import functools
+import sysconfig
+import warnings
 from ctypes import c_char_p, c_int, c_int32, c_size_t, c_void_p
 from pathlib import Path
 
@@ -106,24 +109,40 @@ def load():
     return _lib
 
 
-_fast_call = None
 # (device index, stream) -> the workspace tensor of `matmul` there.  ops.py fills it and both ways of a call look it up here, each
 # holding the tensor while it uses it, so that a larger one may take its place at any time.
 workspaces: dict = {}
 
 
-def load_fast_call():
-    """The extension module that checks and launches the common case of `ops.matmul`, bound to the library."""
-    global _fast_call
-    if _fast_call is None:
-        lib = load()
-        try:
-            from . import _fast_call as module
-        except ImportError as e:
-            raise ImportError("tuna_b200/_fast_call.so is missing or does not fit this torch: build it with `python -m tuna_b200.build`") from e
-        module.bind(ctypes.cast(lib.tuna_matmul, c_void_p).value, workspaces)
-        _fast_call = module
+def fast_call_stamp() -> str:
+    """What the extension module has to be built for: its code contains the layouts of this torch's and Python's objects."""
+    import torch
+
+    return f"tuna_b200 _fast_call for torch {torch.__version__}, {sysconfig.get_config_var('SOABI')}"
+
+
+def _import_fast_call():
+    from . import _fast_call
+
     return _fast_call
+
+
+@functools.lru_cache(maxsize=None)
+def load_fast_call():
+    """The extension module that checks and launches the common case of `ops.matmul`, bound to the library; None, with a
+    warning, where it is missing or was built for another torch or Python: every call goes through the Python checks then."""
+    lib = load()
+    try:
+        module = _import_fast_call()
+    except ImportError as e:
+        why = str(e)
+    else:
+        if getattr(module, "stamp", None) == fast_call_stamp():
+            module.bind(ctypes.cast(lib.tuna_matmul, c_void_p).value, workspaces)
+            return module
+        why = f"it was built for another one than: {fast_call_stamp()}"
+    warnings.warn(f"tuna_b200: matmul's calls are checked in Python, its extension module cannot be used ({why}): `python -m tuna_b200.build` builds it", RuntimeWarning, stacklevel=3)
+    return None
 
 
 class TunaError(RuntimeError):

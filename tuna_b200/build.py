@@ -14,10 +14,12 @@ import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
+from . import _lib
+
 HERE = Path(__file__).resolve().parent
 CSRC = HERE / "csrc"
 LIB = HERE / "libtuna_b200.so"
-FAST_CALL = HERE / "_fast_call.so"
+FAST_CALL = HERE / ("_fast_call" + sysconfig.get_config_var("EXT_SUFFIX"))
 SOURCES = ["tuna_api.cu", "host_util.cu", "dequant_sm100a.cu", "quantize_sm100a.cu", "gemm_stream_sm100a.cu", "gemm_tstream_sm100a.cu", "gemm_pair_sm100a.cu", "exchange_sm100a.cu", "ref_symbols.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -76,22 +78,30 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     return LIB
 
 
+def _fast_call_stale() -> bool:
+    """Whether the extension is older than its sources or was built for another torch or Python than these."""
+    return (_stale(FAST_CALL, [CSRC / "fast_call.cpp", HERE.parent / "include" / "tuna_b200.h"])
+            or _lib.fast_call_stamp().encode() + b"\0" not in FAST_CALL.read_bytes())
+
+
 def _build_fast_call(force: bool) -> None:
-    """The native front of `ops.matmul` (csrc/fast_call.cpp): an extension module against the headers of the torch it runs with."""
-    src = CSRC / "fast_call.cpp"
-    if not force and not _stale(FAST_CALL, [src]):
-        return
+    """The native front of `ops.matmul` (csrc/fast_call.cpp): an extension module against the headers of the torch it runs with.
+
+    Beside a torch without CUDA there is nothing to build it against, and nothing that would call it."""
     import torch
 
     root = Path(torch.__file__).resolve().parent
+    if not (root / "lib" / "libc10_cuda.so").exists() or not (force or _fast_call_stale()):
+        return
     cuda = Path(_nvcc()).resolve().parent.parent if os.path.sep in _nvcc() else Path("/usr/local/cuda")
     include = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include", cuda / "include", sysconfig.get_paths()["include"]]
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
-           *(f"-I{p}" for p in include), str(src), "-o", str(FAST_CALL), f"-L{root / 'lib'}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
+           f'-DFAST_CALL_STAMP="{_lib.fast_call_stamp()}"', *(f"-I{p}" for p in include), str(CSRC / "fast_call.cpp"), "-o", str(FAST_CALL),
+           f"-L{root / 'lib'}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
     r = subprocess.run(cmd, capture_output=True, text=True)
-    if r.returncode:
-        sys.stderr.write(r.stdout + r.stderr)
-        raise RuntimeError("the build of fast_call.cpp failed")
+    if r.returncode:  # no Python headers, say: the library is complete without it
+        FAST_CALL.unlink(missing_ok=True)
+        sys.stderr.write(r.stdout + r.stderr + "fast_call.cpp was not built: matmul will check its calls in Python\n")
 
 
 if __name__ == "__main__":

@@ -128,4 +128,13 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_fast_call", nullptr, -1, methods,
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__fast_call() { return PyModule_Create(&module); }
+// torch's layouts are compiled in: _lib.py uses the module, and build.py keeps it, only where this names the torch and Python at hand.
+#ifndef FAST_CALL_STAMP
+#error "build.py says what this is built for"
+#endif
+PyMODINIT_FUNC PyInit__fast_call()
+{
+    PyObject *m = PyModule_Create(&module);
+    if (m && PyModule_AddStringConstant(m, "stamp", FAST_CALL_STAMP) < 0) Py_CLEAR(m);
+    return m;
+}
