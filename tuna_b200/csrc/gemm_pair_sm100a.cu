@@ -49,6 +49,7 @@
 #include <mutex>
 #include "common.cuh"
 #include "launchers.h"
+#include "ring_plan.h"
 #include "sm100_ptx.cuh"
 #include "tcgen05.cuh"
 
@@ -57,13 +58,7 @@ namespace tuna {
 constexpr int kPairRows = 2 * kBlockRows;   // rows of a tile
 constexpr int kPairEpilogueWarp0 = 4;
 constexpr int kPairDequantWarp0 = 8;
-constexpr int kPairTmemCols = 512;
-constexpr int kPairLutBytes = 256 * 128;    // byte -> half2 table: 256 entries, one copy per bank
-constexpr int kPairLutWide = 4096, kPairLutWideBytes = 256 * 256;  // its place and size with 256 bytes per entry (pair_lookup)
-constexpr int kPairMaxStages = 8;           // unit stages: activations in shared memory + an A slot in tensor memory
-constexpr int kPairMaxWStages = 8;
 constexpr int kPairBars = 3 * kPairMaxStages + 2 * kPairMaxWStages + 4;
-constexpr int kPairSmemDynamic = 226 * 1024;
 constexpr int kPairTokGroup = 8;            // token tiles of a wave's working set
 // Up to here weights and codebook are taken from ahead of the dependency wait, as the weight-streaming kernels do (the
 // header's contract); more tokens see ordinary stream order.  There the weights are read after the wait, and the lookup table
@@ -586,7 +581,7 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
             ring.idx += by;
             while (ring.idx >= depth) { ring.idx -= depth; ring.phase ^= 1u; }
         };
-        Ring rw, ru;
+        Ring rw, ru;  // the groups share both rings: rings_shareable() says when they may
         skip(rw, group, SW);
         skip(ru, group, S);
         for (int u = group; u < total; u += kPairGroups) {
@@ -665,15 +660,6 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
 // 118 of 256; 20608x8576 at 497 134 and 143; 8704x27264 at 195 89 and (224) 93; 1280x28544 at 398 36 and (160) 33.
 static double pair_step_us(int tok) { return std::max((tok / 4 + 54) / 1700.0, (tok / 2 + 8) / 1420.0); }
 
-// 16 dequant warps where they bound the tile, i.e. as long as the tensor pipe needs fewer clocks per step than the table
-// lookups and what goes with them; with them comes the table that one instruction per lookup addresses (pair_lookup), which leaves
-// too little shared memory for the stages of wider tiles.  Graph replay, us, 8 / 16 warps / 16 and the wide table: 11000x4104 at 43
-// tokens 13.5 / 12.6 / 12.5, 6144x4096 at 256 (96-token tiles) 15.5 / 14.5 / 14.1, 57344x8192 at 64 81 / 70 / 70, 8192x8192 at 192
-// 27.5 / 25.5 / 24.3; 57344x8192 at 256 (256-token tiles) 166 / 167, 28672x4096 at 224 47 / 46.
-static int pair_dequant_warps(int tile_tok) { return tile_tok <= 192 ? 16 : 8; }
-
-static int pair_kc(int tile_tok) { return tile_tok > 128 ? 64 : 128; }
-
 // How the tiles of a launch are handed out (see the head of the file): sk_tiles of them are cut along K over
 // sk_pairs pairs, the others go out in whole waves.
 struct PairSplit {
@@ -734,32 +720,10 @@ static int pair_pick_tile_tok(int m, int n, int k, int pairs)
     return best;
 }
 
-struct PairPlan {
-    int tile_tok, kc, stages, w_stages, nd;
-};
-
 static int pair_count(const tuna_config &c) { return c.ctas / 2 > 0 ? c.ctas / 2 : 1; }
 
 // of a normalized configuration
-static PairPlan pair_plan(const tuna_config &c)
-{
-    PairPlan l;
-    l.tile_tok = c.tile_tok < 32 ? 32 : c.tile_tok;
-    l.kc = pair_kc(l.tile_tok);
-    const int slot = l.kc / 2;
-    // two accumulator buffers (the epilogue of one tile overlaps the MMAs of the next) where they leave four A slots
-    l.nd = 2 * l.tile_tok + 4 * slot <= kPairTmemCols ? 2 : 1;
-    l.stages = (kPairTmemCols - l.nd * l.tile_tok) / slot;
-    if (l.stages > kPairMaxStages) l.stages = kPairMaxStages;
-    const int w_bytes = kBlockRows * l.kc / 2;
-    // dynamic shared memory begins 2 KB into the window (launch_pair checks it)
-    const int lut = pair_dequant_warps(l.tile_tok) == 16 ? kPairLutWide - 2048 + kPairLutWideBytes : kPairLutBytes;
-    auto smem = [&](int s, int w) { return lut + l.tile_tok * 256 + s * l.tile_tok * l.kc + w * w_bytes; };
-    l.w_stages = kPairMaxWStages;
-    while (l.stages > 4 && smem(l.stages, l.w_stages) > kPairSmemDynamic) --l.stages;
-    while (l.w_stages > 4 && smem(l.stages, l.w_stages) > kPairSmemDynamic) --l.w_stages;
-    return l;
-}
+static PairPlan pair_plan(const tuna_config &c) { return pair_plan(c.tile_tok < 32 ? 32 : c.tile_tok); }
 
 // The fields of an explicit configuration describe a tile of one SM - `row_blocks` x 128 rows x `tile_tok` tokens in stages
 // of 64 columns - and what does not fit one SM's tensor or shared memory is refused, although this kernel takes no
@@ -817,12 +781,12 @@ static int launch_pair(const PairParams &p, const CUtensorMap &mq, const CUtenso
         if (!attr_set[dev]) {
             if (cudaFuncSetAttribute(gemm_w4a16_pair_kernel<KC, WMODE, DW>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemDynamic) != cudaSuccess)
                 return TUNA_ERR_NO_DEVICE;
-            // pair_plan counts on 1 KB of the system's and 1 KB of static shared memory before the dynamic part
+            // pair_plan counts on 1 KB of the system's and up to 1 KB of static shared memory before the dynamic part
             cudaFuncAttributes fa;
             int reserved = 0;
             if (cudaFuncGetAttributes(&fa, gemm_w4a16_pair_kernel<KC, WMODE, DW>) != cudaSuccess ||
                 cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev) != cudaSuccess ||
-                fa.sharedSizeBytes + (size_t)reserved > 2048)
+                fa.sharedSizeBytes + (size_t)reserved > kPairSmemStart)
                 return TUNA_ERR_NO_DEVICE;
             attr_set[dev] = true;
         }

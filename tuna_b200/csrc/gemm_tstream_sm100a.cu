@@ -73,6 +73,7 @@
 #include <mutex>
 #include "common.cuh"
 #include "launchers.h"
+#include "ring_plan.h"
 #include "sm100_ptx.cuh"
 #include "tcgen05.cuh"
 
@@ -194,6 +195,35 @@ __device__ __forceinline__ uint32_t ts_lookup256(uint32_t w, uint32_t key, uint3
 template <int V>
 struct Int { static constexpr int value = V; };
 
+// Weight stages below the lookup table, and all of them, where the first one starts at shared address `w_low`.
+__host__ __device__ constexpr int ts_low_stages(bool lut256, uint32_t w_low, uint32_t slot_bytes)
+{
+    return lut256 && w_low < 0x10000u ? (int)((0x10000u - w_low) / slot_bytes) : 0;
+}
+__host__ __device__ constexpr int ts_w_stages(bool lut256, uint32_t w_low, uint32_t smem_end, uint32_t slot_bytes)
+{
+    const int n = ts_low_stages(lut256, w_low, slot_bytes) + (int)((smem_end - (lut256 ? 0x20000u : w_low)) / slot_bytes);
+    return n < kTsMaxWStages ? n : kTsMaxWStages;
+}
+// Columns of one accumulator buffer (32 is the allocation granule), and A slots behind the two of them.
+__host__ __device__ constexpr int ts_acc_cols(int row_blocks, int tile_tok) { return row_blocks * tile_tok < 32 ? 32 : row_blocks * tile_tok; }
+__host__ __device__ constexpr int ts_a_slots(int acc_cols, int steps)
+{
+    const int n = (kTsTmemCols - 2 * acc_cols) / (16 * steps);
+    return n < kTsMaxASlots ? n : kTsMaxASlots;
+}
+// Whether the dequant groups may share the rings (ring_plan.h) wherever dynamic shared memory begins, which is checked to be in the first 4 KB.
+constexpr bool ts_rings_shareable(int tile_tok, int steps, bool lut256, uint32_t x_ring_bytes)
+{
+    for (int rb = 1; rb == 1 || rb * tile_tok <= 64; rb *= 2)
+        for (uint32_t dyn0 = 1024; dyn0 <= 4096; dyn0 += 1024) {
+            const uint32_t w_low = dyn0 + (lut256 ? 0u : kTsLutBytes) + x_ring_bytes;
+            const int w = ts_w_stages(lut256, w_low, dyn0 + kTsSmemDynamic, 16 * 32 * 4 * steps);
+            if (!rings_shareable(w, ts_a_slots(ts_acc_cols(rb, tile_tok), steps), kTsDequantWarps / steps)) return false;
+        }
+    return true;
+}
+
 // The CTA whose range holds unit u.
 __device__ __forceinline__ int ts_cta_of_unit(const TsParams &p, int u)
 {
@@ -296,13 +326,10 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_w4a16_tstream_kernel(const
     const uint32_t lut_addr = kLut256 ? 0x10000u : dyn0;
     const uint32_t xring = kLut256 ? dyn0 : dyn0 + kTsLutBytes;
     const uint32_t w_low = xring + kXS * kXStageBytes;                       // first weight stage
-    const int n_low = (kLut256 && w_low < 0x10000u) ? (int)((0x10000u - w_low) / kSlotBytes) : 0;   // weight stages below the table
+    const int n_low = ts_low_stages(kLut256, w_low, kSlotBytes);  // weight stages below the table
     const uint32_t w_high = kLut256 ? 0x20000u : w_low;
-#ifdef TS_WS_LIMIT  // timing experiment: fewer weight stages in flight
-    const int WS = min(TS_WS_LIMIT, n_low + (int)((smem_end - w_high) / kSlotBytes));
-#else
-    const int WS = min(kTsMaxWStages, n_low + (int)((smem_end - w_high) / kSlotBytes));
-#endif
+    const int WS = ts_w_stages(kLut256, w_low, smem_end, kSlotBytes);
+    static_assert(ts_rings_shareable(N_TILE, STEPS, kLut256, kXS * kXStageBytes), "a dequant group could pass its wait for a weight stage a phase early");
     auto w_stage = [&](int i) -> uint32_t { return i < n_low ? w_low + (uint32_t)i * kSlotBytes : w_high + (uint32_t)(i - n_low) * kSlotBytes; };
     if (kLut256 && dyn0 > 4096u) {  // the layout above assumes that dynamic shared memory starts within the first 4 KB
         if (threadIdx.x == 0 && atomicCAS(&p.status->code, 0, 97) == 0) p.status->detail = (int)dyn0;
@@ -946,10 +973,9 @@ static long long ts_fill_gemm(TsGemm *g, const void *q, const void *x, const flo
 static void ts_fill_common(TsParams *p, const tuna_config &c, int steps, void *workspace, int sm_count)
 {
     p->row_blocks = c.row_blocks;
-    p->acc_cols = c.row_blocks * c.tile_tok < 32 ? 32 : c.row_blocks * c.tile_tok;  // 32-column allocation granule
+    p->acc_cols = ts_acc_cols(c.row_blocks, c.tile_tok);
     p->a_base = 2 * p->acc_cols;
-    p->a_slots = (kTsTmemCols - p->a_base) / (16 * steps);
-    if (p->a_slots > kTsMaxASlots) p->a_slots = kTsMaxASlots;
+    p->a_slots = ts_a_slots(p->acc_cols, steps);
     p->partials = (float *)workspace;
     p->counters = (unsigned int *)((uint8_t *)workspace + partial_region_bytes(sm_count));
 }
