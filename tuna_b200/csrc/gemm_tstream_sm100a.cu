@@ -429,12 +429,16 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_w4a16_tstream_kernel(const
     };
     // Adds the partials of GR four-token groups from group g0 on (the last group that exists stands in for those after it) of 32 rows (block rb, quarter q of the tile) over its
     // segments, which CTAs `first` .. first + nseg - 1 wrote, and stores the rows.  The loads of SG segments are
-    // in flight at a time, the adds keep the range order.
+    // in flight at a time, the adds keep the range order.  Their addresses are 32-bit offsets into the partial sums (partial_region_bytes, far
+    // below 4 GB): this runs once per CTA, out of a cold instruction cache, and with 64-bit arithmetic per load eight in flight took longer than four
+    // (768x2304 at 15 tokens, nine segments, by four / by eight / so: 5.63 / 6.06 / 5.63 us; 1152x3328 at 11 6.14 / 6.06 / 5.72).
     auto add_partials = [&](auto gr, auto sg, const TsGemm &G, int tile, int first, int nseg, int q, int rb, int g0, int last) __attribute__((always_inline)) {
         constexpr int GR = decltype(gr)::value, SG = decltype(sg)::value;
         const int row = (tile * RB + rb) * kBlockRows + row_in_block(q);
         if (row >= G.m) return;
         const float sc = G.absmax[row];
+        const uint32_t slot_bytes = (uint32_t)slot_floats * 4u;
+        const uint32_t at = (uint32_t)(2 * first) * slot_bytes + (uint32_t)(rb * (N_TILE / 4) * kBlockRows + 32 * q + lane) * 16u;
         float acc[4 * GR];
 #pragma unroll
         for (int i = 0; i < 4 * GR; ++i) acc[i] = 0.f;
@@ -444,10 +448,10 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_w4a16_tstream_kernel(const
 #pragma unroll
             for (int j = 0; j < SG; ++j) {
                 const int seg = min(sgm + j, nseg - 1);
-                const float4 *src = reinterpret_cast<const float4 *>(p.partials + (size_t)(2 * (first + seg) + (seg == 0 ? 1 : 0)) * slot_floats) +
-                                    (size_t)rb * (N_TILE / 4) * kBlockRows + 32 * q + lane;
+                const uint32_t off = at + (uint32_t)(2 * seg + (seg == 0 ? 1 : 0)) * slot_bytes;
 #pragma unroll
-                for (int i = 0; i < GR; ++i) a[j][i] = __ldcg(src + min(g0 + i, last) * kBlockRows);
+                for (int i = 0; i < GR; ++i)
+                    a[j][i] = __ldcg(reinterpret_cast<const float4 *>(reinterpret_cast<const char *>(p.partials) + (off + (uint32_t)min(g0 + i, last) * (kBlockRows * 16u))));
             }
 #pragma unroll
             for (int j = 0; j < SG; ++j) {
