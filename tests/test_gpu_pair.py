@@ -36,6 +36,20 @@ def test_token_tiles(tile_tok, m, k):
     _run(m, 2 * tile_tok + 7, k, seed=tile_tok, tile_tok=tile_tok)
 
 
+# short tiles and long ones, several per pair
+@pytest.mark.parametrize("tile_tok", [32, 64, 96, 128, 160, 192, 224])
+@pytest.mark.parametrize("k", [136, 640, 5128])
+def test_short_and_long_tiles(tile_tok, k):
+    _run(1032, tile_tok + 9, k, seed=tile_tok + k, tile_tok=tile_tok, ctas=6)
+
+
+# few and many segments of a tile, added up in pieces of 8 and of 16 columns, with tokens and rows left over
+@pytest.mark.parametrize("ctas", [4, 10, 34, 148])
+@pytest.mark.parametrize("n,tile_tok", [(20, 32), (32, 32), (60, 64), (96, 96), (100, 64), (190, 192), (250, 256)])
+def test_segments_of_cut_tiles(n, tile_tok, ctas):
+    _run(264, n, 8200, seed=n + ctas, tile_tok=tile_tok, ctas=ctas)
+
+
 # m and k of every weight view: 5-D runs, 3-D boxes (k % 32 == 0), 2-D boxes (any k); fewer rows than a tile, row remainders
 @pytest.mark.parametrize("m,k", [(8, 8), (256, 64), (264, 96), (520, 136), (1032, 1000), (2048, 2112)])
 @pytest.mark.parametrize("n", [70, 250])

@@ -65,6 +65,10 @@ __device__ __forceinline__ uint4 ldg_stream_pred(const void *p, unsigned pred)
     return v;
 }
 
+// A compile-time number as an argument.
+template <int V>
+struct Int { static constexpr int value = V; };
+
 // Error word shared by the kernels that contain bounded waits.
 struct DeviceStatus {
     int code;      // 0 = ok, otherwise where a wait gave up

@@ -283,47 +283,52 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
     const uint32_t a_off = (uint32_t)p.nd * d_cols;  // first A slot
     const uint32_t leader_u_full = map_to_rank(u_full, 0), leader_d_empty = map_to_rank(d_empty, 0);
 
-    // Adds the partials of columns [col, col + 16) of TMEM lane 32*quarter + lane over all segments of a tile, in K
-    // order, and stores the row.
-    auto fix_piece = [&](int tile, int quarter, int col) {
-        int rt, tt;
-        pair_tile(p, tile, rt, tt);
-        const int row_in_block = WMODE == 1 ? 32 * quarter + lane : 8 * lane_row_group(quarter, lane) + (lane & 7);
-        const int row = rt * kPairRows + rank * kBlockRows + row_in_block;
+    // The first CTA pair of a cut tile's segments, and their number.
+    auto tile_segments = [&](int tile, int &first) {
         auto pair_of = [&](int unit) {
             const int big = p.sk_r * (p.sk_q + 1);
             return unit < big ? unit / (p.sk_q + 1) : p.sk_r + (unit - big) / p.sk_q;
         };
-        const int first = pair_of(tile * p.chunks), nseg = pair_of((tile + 1) * p.chunks - 1) - first + 1;
-        const size_t slot_floats = (size_t)kBlockRows * N;
+        first = pair_of(tile * p.chunks);
+        return pair_of((tile + 1) * p.chunks - 1) - first + 1;
+    };
+    // Adds the partials of COLS columns from `col` on of TMEM lane 32*quarter + lane over all segments of a tile, in K
+    // order, and stores the row.  The loads of SG segments are in flight at a time, the adds keep the order; their addresses are 32-bit offsets into the
+    // partial sums (partial_region_bytes, far below 4 GB), which is less code for a part that runs once.
+    auto fix_piece = [&](auto cols_, auto sg, int tile, int first, int nseg, int quarter, int col) {
+        constexpr int COLS = decltype(cols_)::value, SG = decltype(sg)::value;
+        int rt, tt;
+        pair_tile(p, tile, rt, tt);
+        const int row_in_block = WMODE == 1 ? 32 * quarter + lane : 8 * lane_row_group(quarter, lane) + (lane & 7);
+        const int row = rt * kPairRows + rank * kBlockRows + row_in_block;
+        const uint32_t slot_bytes = (uint32_t)N * (kBlockRows * 4u);
+        const uint32_t at = (uint32_t)(2 * (2 * first + rank)) * slot_bytes + (uint32_t)(col / 4 * kBlockRows + 32 * quarter + lane) * 16u;
         auto seg_ptr = [&](int s) {
-            return reinterpret_cast<const float4 *>(p.partials + (size_t)(2 * (2 * (first + s) + rank) + (s == 0 ? 1 : 0)) * slot_floats) +
-                   (size_t)(col / 4) * kBlockRows + 32 * quarter + lane;
+            return reinterpret_cast<const float4 *>(reinterpret_cast<const char *>(p.partials) + (at + (uint32_t)(4 * s + (s == 0 ? 1 : 0)) * slot_bytes));
         };
-        float acc[16];
+        float acc[COLS];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) acc[i] = 0.f;
-        constexpr int SG = DW == 16 ? 2 : 4;  // segments' loads in flight; the adds keep the order
+        for (int i = 0; i < COLS; ++i) acc[i] = 0.f;
         for (int s = 0; s < nseg; s += SG) {
-            float4 v[SG][4];
+            float4 v[SG][COLS / 4];
 #pragma unroll
             for (int j = 0; j < SG; ++j)
                 if (s + j < nseg) {
                     const float4 *src = seg_ptr(s + j);
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) v[j][i] = __ldcg(src + i * kBlockRows);
+                    for (int i = 0; i < COLS / 4; ++i) v[j][i] = __ldcg(src + i * kBlockRows);
                 }
 #pragma unroll
             for (int j = 0; j < SG; ++j)
                 if (s + j < nseg) {
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) { acc[4 * i] += v[j][i].x; acc[4 * i + 1] += v[j][i].y; acc[4 * i + 2] += v[j][i].z; acc[4 * i + 3] += v[j][i].w; }
+                    for (int i = 0; i < COLS / 4; ++i) { acc[4 * i] += v[j][i].x; acc[4 * i + 1] += v[j][i].y; acc[4 * i + 2] += v[j][i].z; acc[4 * i + 3] += v[j][i].w; }
                 }
         }
         if (row < p.m) {
             const float sc = p.absmax[row];
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
+            for (int i = 0; i < COLS; ++i) {
                 const int tok = tt * N + col + i;
                 if (tok < p.n) p.o[(size_t)tok * p.m + row] = __float2half_rn(acc[i] * sc);
             }
@@ -525,11 +530,8 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive_cluster(leader_d_empty + 8 * rd.idx);
-                auto pair_of = [&](int unit) {
-                    const int big = p.sk_r * (p.sk_q + 1);
-                    return unit < big ? unit / (p.sk_q + 1) : p.sk_r + (unit - big) / p.sk_q;
-                };
-                const int nseg = pair_of((segs.tile + 1) * p.chunks - 1) - pair_of(segs.tile * p.chunks) + 1;
+                int first;
+                const int nseg = tile_segments(segs.tile, first);
                 unsigned int *counter = p.counters + (size_t)(2 * segs.tile + rank) * 4 + quarter;
                 unsigned int old = 0;
                 // releases the warp's partials (the __syncwarp above orders them before it) and acquires the others'
@@ -539,7 +541,7 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
                     if (lane == 0) *counter = 0;  // leave the counter clean for the next call
                     // the pair's last segment: all warps of the CTA finish it together, below
                     if (segs.more()) {
-                        for (int col = 0; col < cols; col += 16) fix_piece(segs.tile, quarter, col);
+                        for (int col = 0; col < cols; col += 16) fix_piece(Int<16>(), Int<DW == 8 ? 4 : 2>(), segs.tile, first, nseg, quarter, col);
                     } else if (lane == 0) {
                         s_fix[quarter] = 1;
                     }
@@ -629,18 +631,26 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
     __syncwarp();
     __syncthreads();
     {
-        // tiles whose last partials this CTA wrote in its last segment: 16-token pieces over all warps
-        int fix_tile = -1, cols = 0;
+        // the tile whose last partials this CTA wrote in its last segment: (piece, quarter) over all warps
+        int tile = -1, cols = 0, first = 0, nseg = 0;
         PairSegs s;
         s.init(p, pair, pairs);
         if (s_fix[0] | s_fix[1] | s_fix[2] | s_fix[3]) {
-            while (s.next(p)) fix_tile = s.tile;
+            while (s.next(p)) tile = s.tile;
             int rt, tt;
-            pair_tile(p, fix_tile, rt, tt);
+            pair_tile(p, tile, rt, tt);
             cols = pair_tile_cols(p, tt);
+            nseg = tile_segments(tile, first);
         }
-        for (int item = warp; item < cols / 4; item += kPairWarps)  // (piece, quarter)
-            if (s_fix[item & 3]) fix_piece(fix_tile, item & 3, (item >> 2) * 16);
+        // 24 warps have registers for half as many loads in flight as 16: twice the segments where there is a warp for every eight columns
+        // (16 columns of two segments / 8 of four, us: 800x6464 at 52 tokens 10.7 / 10.3, 512x27392 at 60 13.1 / 12.1; where that takes a second
+        // round of pieces, 64-token tiles, 768x22400 at 97 16.1 / 16.9)
+        if (DW == 16 && cols / 8 * 4 <= kPairWarps) {
+            if ((warp >> 2) * 8 < cols && s_fix[warp & 3]) fix_piece(Int<8>(), Int<4>(), tile, first, nseg, warp & 3, (warp >> 2) * 8);
+        } else {
+            for (int item = warp; (item >> 2) * 16 < cols; item += kPairWarps)
+                if (s_fix[item & 3]) fix_piece(Int<16>(), Int<DW == 16 ? 2 : 4>(), tile, first, nseg, item & 3, (item >> 2) * 16);
+        }
     }
     tc_fence_before();
     __syncwarp();

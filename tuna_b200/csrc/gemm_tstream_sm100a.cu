@@ -192,9 +192,6 @@ __device__ __forceinline__ uint32_t ts_lookup256(uint32_t w, uint32_t key, uint3
     return v;
 }
 
-template <int V>
-struct Int { static constexpr int value = V; };
-
 // Weight stages below the lookup table, and all of them, where the first one starts at shared address `w_low`.
 __host__ __device__ constexpr int ts_low_stages(bool lut256, uint32_t w_low, uint32_t slot_bytes)
 {
