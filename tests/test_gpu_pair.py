@@ -36,7 +36,7 @@ def test_token_tiles(tile_tok, m, k):
     _run(m, 2 * tile_tok + 7, k, seed=tile_tok, tile_tok=tile_tok)
 
 
-# short tiles and long ones, several per pair
+# short tiles (8 dequant warps) and long ones (16 up to 192 tokens), several per pair
 @pytest.mark.parametrize("tile_tok", [32, 64, 96, 128, 160, 192, 224])
 @pytest.mark.parametrize("k", [136, 640, 5128])
 def test_short_and_long_tiles(tile_tok, k):

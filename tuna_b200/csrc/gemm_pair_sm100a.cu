@@ -23,7 +23,7 @@
 //   warp 3      tensor-memory allocation
 //   warps 4-7   epilogue: tensor memory -> registers -> scale by absmax -> fp16 -> stmatrix into a
 //               staging tile -> TMA store; split-K partials and fix-up
-//   warps 8 on   dequant (8 or 16, pair_dequant_warps): packed bytes (shared memory) -> byte->half2 table lookups -> tcgen05.st.  A
+//   warps 8 on   dequant (8 or 16, pair_split): packed bytes (shared memory) -> byte->half2 table lookups -> tcgen05.st.  A
 //               thread owns one weight row (= one TMEM lane): a 32-bit word of the packed layout is
 //               8 consecutive columns of one row (test.py:58-65), i.e. four TMEM columns in K order
 // The dequantised fp16 weights never touch shared or global memory.  The scale is constant along K
@@ -180,7 +180,7 @@ __device__ __forceinline__ uint32_t pair_lookup(uint32_t w, uint32_t lane_key)
 //      that reads global memory in runs of 256 bytes (m % 32 == 0 and k % 64 == 0); TMEM lane l holds row l;
 //   0  [step][row group][128 bytes]: one 3-D box per stage (k % 32 == 0) or one 2-D box per step; rows
 //      assigned to lanes by lane_row_group().
-// DW: dequant warps, 8 or 16 (pair_dequant_warps).
+// DW: dequant warps, 8 or 16 (pair_split).
 template <int KC, int WMODE, int DW>
 __global__ void __launch_bounds__(32 * (kPairDequantWarp0 + DW), 1)
 gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_constant__ CUtensorMap tmap_q,
@@ -663,56 +663,85 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
 
 // ------------------------------------------------------------------ host side
 
-// Microseconds per 16 columns of K of a tile of `tok` tokens: the wavefronts of shared memory (see the head of the
-// file; with 16 dequant warps 54 beside the activations' instead of 61) at the 1.7 GHz of a short run, or the tensor pipe's N/2 clocks, and
-// what the dequantisation adds to them, at the clock the power cap leaves it (measured at K = 4096: 14 us a wave of 128-token tiles, 22 of
-// 224, 25 of 256).  The line between many waves of 128 tokens and fewer of wider tiles follows from it: 29568x8320 at 243 tokens 98 us in tiles of 128,
-// 118 of 256; 20608x8576 at 497 134 and 143; 8704x27264 at 195 89 and (224) 93; 1280x28544 at 398 36 and (160) 33.
-static double pair_step_us(int tok) { return std::max((tok / 4 + 54) / 1700.0, (tok / 2 + 8) / 1420.0); }
+// The estimates below are fitted to 12000 launches (graph replay, short runs): 350 shapes of 512 to 55000 rows, 512 to 28000 columns and
+// 25 to 3900 tokens in every token tile, with 8 and 16 dequant warps, uncut and cut in every way that pair_split considers.  What they choose
+// takes 0.7 % longer than the fastest launch of its shape in the mean, 11 % at worst; with 16 warps wherever they fit and cuts priced by their number of
+// segments alone it was 4 % and 38 %.
+
+// Microseconds per 16 columns of K of a tile of `tok` tokens: the clocks of the lookups and what goes with them plus the activations'
+// at the 1.7 GHz of a short run, or the tensor pipe's N/2 clocks and what the dequantisation adds to them, at the clock the power cap leaves it.
+static double pair_step_us(int tok, int warps) { return std::max((tok / 4 + (warps == 16 ? 50 : 71)) / 1700.0, (tok / 2 + 8) / 1420.0); }
 
 // How the tiles of a launch are handed out (see the head of the file): sk_tiles of them are cut along K over
 // sk_pairs pairs, the others go out in whole waves.
 struct PairSplit {
     int sk_tiles, sk_pairs;
+    int warps;  // dequant warps
     double us;  // the estimate
 };
 
-// What cutting costs beyond the work itself: partial sums written, an arrival, partial sums read by the finishing
-// CTA.  Measured (us, 2 to 10 segments): 32-token tiles 6 to 7, 64 4 to 8, 128 12 to 18 (more pieces than warps), 256 14 to 20; an uncut launch
-// 0.5 to 4.  Where whole tiles follow the cut ones, adding up hides behind them.
-static double pair_cut_us(int tile_tok, int segs, bool hidden)
+// What an uncut launch takes beside its steps.  16 dequant warps convert four stages at once and the MMAs of all four are still to come: on
+// short tiles that takes longer than what the warps save (us, 8 / 16: 3192x1048 at 613 tokens, 128-token tiles, 9.1 / 9.6; 12496x512 at 738 12.9 / 13.5;
+// 2048x4096 at 1140 16.5 / 16.4; 6144x4096 at 256, 96-token tiles, 15.8 / 14.5).  Where the weights come after the dependency wait, narrow tiles
+// have most of the dequantisation still before them then and want the warps (1792x896 at 78 tokens, 32-token tiles, 5.2 / 4.8; 2944x768 at 100,
+// 64-token tiles, 5.1 / 4.9; ahead of it 3072x768 at 60 3.9 / 4.0).
+static double pair_uncut_us(int cols, int warps, bool ahead)
 {
-    const double adding = hidden ? 0.05 * std::max(0, tile_tok - 128) : 0.06 * std::max(0, std::min(tile_tok, 160) - 64) + 0.01 * std::max(0, tile_tok - 160);
-    return 5.0 + 0.025 * tile_tok + adding + segs * (0.25 + 0.002 * tile_tok);
+    return 2.6 + 0.007 * cols + (warps == 16 ? 0.7 : (ahead ? 0.0 : std::max(0.0, 0.7 - 0.0055 * cols)));
 }
-constexpr double kPairUncutUs = 0.9;
-// What a wave of whole tiles costs beside its steps: the epilogue, where there is one accumulator buffer only (pair_plan), else the turn from
-// one tile to the next.  33280x1408 at 2025 tokens: 139 us in tiles of 160, 167 of 256; 29312x512 at 292 four waves of 160 12.6, five of 128 14.1.
-static double pair_wave_us(int tile_tok) { return tile_tok > 192 ? 1.0 : 0.3; }
+constexpr double kPairWaveUs = 0.1;  // from one wave of whole tiles to the next
+// What cutting costs: partial sums written, an arrival, and adding them up.
+static double pair_cut_us(int cols, int warps) { return 5.2 + 0.03 * cols + 0.045 * std::max(0, cols - 128) + (warps == 16 ? 0.35 : 0.0); }
+// Adding up `segs` segments of a tile at the end of a CTA: a round is as many loads as its warps have in flight.
+static double pair_add_us(int cols, int warps, int segs)
+{
+    const int rounds = warps == 8 ? div_up(segs, 4) * div_up(cols / 4, 16) : (cols == 32 ? div_up(segs, 4) : div_up(segs, 2) * div_up(cols / 4, 24));
+    return 0.83 * rounds;
+}
+// Ranges that do not end where a tile does: their CTAs work on two tiles, and a tile has one segment more (528x4480 at 44 tokens, 35 chunks a
+// tile: four segments 10.2 us, five 8.4).
+constexpr double kPairRaggedUs = 2.5;
+// Cut tiles in front of whole ones.
+constexpr double kPairMixedUs = 3.6;
+// A launch that leaves half of the pairs idle: the next one starts on those (6272x1792 at 42 tokens: one tile of 64 per 256 rows 6.5 us, two
+// of 32 8.0).
+constexpr double kPairOverlapUs = 1.2;
 
 static PairSplit pair_split(int m, int n, int k, int tile_tok, int pairs)
 {
-    const int row_tiles = div_up(m, kPairRows), full = n / tile_tok, last = n - full * tile_tok;
-    const int tok_tiles = full + (last ? 1 : 0), chunks = div_up(k, pair_kc(tile_tok));
+    const int row_tiles = div_up(m, kPairRows), full = n / tile_tok, last = n - full * tile_tok, last_cols = (last + 31) / 32 * 32;
+    const int tok_tiles = full + (last ? 1 : 0), chunks = div_up(k, pair_kc(tile_tok)), cols = full ? tile_tok : last_cols;
     const long long tiles = (long long)row_tiles * tok_tiles;
-    const double steps = k / 16.0, last_us = last ? steps * pair_step_us((last + 31) / 32 * 32) : 0.0;
-    const double tile_us = full ? steps * pair_step_us(tile_tok) : last_us;  // of the widest tile
-    const double work_us = row_tiles * (full * tile_us + last_us) / pairs;   // per pair, evenly cut
     const long long waves = tiles / pairs;
     const int rest = (int)(tiles - waves * pairs);
-    const double wave_end = pair_wave_us(tile_tok);
-    // a wave of tiles of two widths takes as long as something between their mean and the wider one
-    const double wave_us = 0.5 * (tile_us + work_us * pairs / tiles) + wave_end;
-    PairSplit best = {0, 0, kPairUncutUs + (waves == 0 ? tile_us + wave_end : (waves + (rest ? 1 : 0)) * wave_us)};
-    auto consider = [&](int sk_tiles, int sk_pairs, double us) {
-        if (us < best.us) best = {sk_tiles, sk_pairs, us};
-    };
-    if (rest > 0 && waves > 0) consider(pairs + rest, pairs, work_us + waves * wave_end + pair_cut_us(tile_tok, 2, waves > 1));
-    if (waves == 0) {
-        int s = 2;
-        for (; s * tiles <= pairs && s <= chunks; ++s) consider((int)tiles, s * (int)tiles, tile_us / s + pair_cut_us(tile_tok, s, false));
-        // all pairs, where whole segments leave more than a tenth of them idle
-        if (s <= chunks && (s - 1) * tiles * 10 < pairs * 9) consider((int)tiles, pairs, work_us + pair_cut_us(tile_tok, s + 1, false) + 0.03 * tile_tok);
+    const double steps = k / 16.0;
+    auto overlap = [&](long long busy) { return 2 * busy <= pairs ? kPairOverlapUs : 0.0; };
+    PairSplit best = {0, 0, 0, 0.0};
+    for (int warps = pair_dequant_warps(tile_tok); warps >= 8; warps -= 8) {
+        const double last_us = last ? steps * pair_step_us(last_cols, warps) : 0.0;
+        const double tile_us = full ? steps * pair_step_us(tile_tok, warps) : last_us;  // of the widest tile
+        const double work_us = row_tiles * (full * tile_us + last_us) / pairs;          // per pair, evenly cut
+        auto consider = [&](int sk_tiles, int sk_pairs, double us) {
+            if (best.warps == 0 || us < best.us) best = {sk_tiles, sk_pairs, warps, us};
+        };
+        const double uncut_us = pair_uncut_us(cols, warps, n <= kPairAheadTokens), cut_us = pair_cut_us(cols, warps);
+        // a wave of tiles of two widths takes as long as something between their mean and the wider one
+        const double wave_us = 0.5 * (tile_us + work_us * pairs / tiles) + kPairWaveUs;
+        consider(0, 0, waves == 0 ? uncut_us + tile_us + kPairWaveUs - overlap(tiles) : uncut_us + (waves + (rest ? 1 : 0)) * wave_us);
+        // where there is more than one wave of whole tiles, adding up hides behind them
+        if (rest > 0 && waves > 0)
+            consider(pairs + rest, pairs, work_us + waves * kPairWaveUs + cut_us + kPairMixedUs + (waves > 1 ? 0.0 : pair_add_us(cols, warps, 2)));
+        if (waves == 0) {
+            int s = 2;
+            for (; s * tiles <= pairs && s <= chunks; ++s) {
+                const bool ragged = chunks % s != 0;
+                consider((int)tiles, s * (int)tiles,
+                         tile_us * div_up(chunks, s) / chunks + cut_us + pair_add_us(cols, warps, s + ragged) + (ragged ? kPairRaggedUs : 0.0) - overlap(s * tiles));
+            }
+            // all pairs, where whole segments leave more than a tenth of them idle
+            if (s <= chunks && (s - 1) * tiles * 10 < pairs * 9)
+                consider((int)tiles, pairs, work_us + cut_us + pair_add_us(cols, warps, pairs / (int)tiles + 1) + kPairRaggedUs);
+        }
     }
     return best;
 }
@@ -733,7 +762,7 @@ static int pair_pick_tile_tok(int m, int n, int k, int pairs)
 static int pair_count(const tuna_config &c) { return c.ctas / 2 > 0 ? c.ctas / 2 : 1; }
 
 // of a normalized configuration
-static PairPlan pair_plan(const tuna_config &c) { return pair_plan(c.tile_tok < 32 ? 32 : c.tile_tok); }
+static int pair_tile_tok(const tuna_config &c) { return c.tile_tok < 32 ? 32 : c.tile_tok; }
 
 // The fields of an explicit configuration describe a tile of one SM - `row_blocks` x 128 rows x `tile_tok` tokens in stages
 // of 64 columns - and what does not fit one SM's tensor or shared memory is refused, although this kernel takes no
@@ -765,7 +794,7 @@ int gemm_umma_normalize_config(int m, int n, int k, int sm_count, tuna_config *c
     // what the launch takes, for whoever looks it up (stages follow from the token tile and stay 0)
     if (t == 0) c->tile_tok = pair_pick_tile_tok(m, n, k, pair_count(*c));
     if (c->row_blocks == 0) c->row_blocks = 1;
-    if (c->dequant_warps == 0) c->dequant_warps = pair_dequant_warps(c->tile_tok);
+    if (c->dequant_warps == 0) c->dequant_warps = pair_split(m, n, k, pair_tile_tok(*c), pair_count(*c)).warps;
     if (c->k_accs == 0) c->k_accs = 1;
     return TUNA_OK;
 }
@@ -773,8 +802,7 @@ int gemm_umma_normalize_config(int m, int n, int k, int sm_count, tuna_config *c
 size_t gemm_umma_workspace_bytes(int m, int n, int k, const tuna_config &c, int sm_count)
 {
     (void)k;
-    const PairPlan l = pair_plan(c);
-    const long long tiles = (long long)div_up(m, kPairRows) * div_up(n, l.tile_tok);
+    const long long tiles = (long long)div_up(m, kPairRows) * div_up(n, pair_tile_tok(c));
     const long long cut = tiles < sm_count ? tiles : sm_count;  // fewer than two waves of tiles are cut along K
     return partial_region_bytes(sm_count) + ((size_t)cut * 32 + 255) / 256 * 256;  // one counter per tile, CTA and TMEM lane quarter
 }
@@ -819,7 +847,9 @@ static int launch_pair(const PairParams &p, const CUtensorMap &mq, const CUtenso
 
 int launch_gemm_umma(const GemmArgs &a, const tuna_config &c)
 {
-    const PairPlan l = pair_plan(c);
+    int pairs = pair_count(c);
+    const PairSplit split = pair_split(a.m, a.n, a.k, pair_tile_tok(c), pairs);
+    const PairPlan l = pair_plan(pair_tile_tok(c), pair_kc(pair_tile_tok(c)), split.warps);
     PairParams p;
     std::memset(&p, 0, sizeof(p));
     p.code = a.code; p.absmax = a.absmax; p.o = (__half *)a.o;
@@ -835,8 +865,6 @@ int launch_gemm_umma(const GemmArgs &a, const tuna_config &c)
     p.partials = (float *)a.workspace;
     p.counters = (unsigned int *)((uint8_t *)a.workspace + partial_region_bytes(a.sm_count));
 
-    int pairs = pair_count(c);
-    const PairSplit split = pair_split(a.m, a.n, a.k, l.tile_tok, pairs);
     const long long tiles_ll = (long long)p.row_tiles * p.tok_tiles;
     // the kernel numbers tiles, the units (tile, chunk) of cut tiles and a pair's units in 32 bits
     constexpr long long kLimit = 1ll << 30;
@@ -867,7 +895,7 @@ int launch_gemm_umma(const GemmArgs &a, const tuna_config &c)
     if (!make_tensor_map_2d(&mo, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, a.o, (uint64_t)a.m, (uint64_t)a.n, (uint64_t)a.m * 2, 64,
                             (uint32_t)l.tile_tok, CU_TENSOR_MAP_SWIZZLE_128B))
         return TUNA_ERR_NO_DEVICE;
-    switch (pair_dequant_warps(l.tile_tok) * 1000 + l.kc + w_mode) {
+    switch (split.warps * 1000 + l.kc + w_mode) {
         case 8064: return launch_pair<64, 0, 8>(p, mq, mx, mo, 2 * pairs, a.stream);
         case 8065: return launch_pair<64, 1, 8>(p, mq, mx, mo, 2 * pairs, a.stream);
         case 8128: return launch_pair<128, 0, 8>(p, mq, mx, mo, 2 * pairs, a.stream);

@@ -24,11 +24,11 @@ constexpr int kPairMaxWStages = 8;
 constexpr int kPairSmemDynamic = 226 * 1024;
 constexpr int kPairSmemStart = 2048;        // where in the shared window dynamic shared memory begins (launch_pair checks it)
 
-// 16 dequant warps where they bound the tile, i.e. as long as the tensor pipe needs fewer clocks per step than the table
-// lookups and what goes with them; with them comes the table that one instruction per lookup addresses (pair_lookup), which leaves
-// too little shared memory for the stages of wider tiles.  Graph replay, us, 8 / 16 warps / 16 and the wide table: 11000x4104 at 43
+// The most dequant warps of a tile, 8 or 16: 16 as long as the tensor pipe needs fewer clocks per step than the table lookups and
+// what goes with them; with them comes the table that one instruction per lookup addresses (pair_lookup), which leaves too little shared
+// memory for the stages of wider tiles.  Graph replay, us, 8 / 16 warps / 16 and the wide table: 11000x4104 at 43
 // tokens 13.5 / 12.6 / 12.5, 6144x4096 at 256 (96-token tiles) 15.5 / 14.5 / 14.1, 57344x8192 at 64 81 / 70 / 70, 8192x8192 at 192
-// 27.5 / 25.5 / 24.3; 57344x8192 at 256 (256-token tiles) 166 / 167, 28672x4096 at 224 47 / 46.
+// 27.5 / 25.5 / 24.3; 57344x8192 at 256 (256-token tiles) 166 / 167, 28672x4096 at 224 47 / 46.  Fewer on short tiles (pair_split).
 constexpr int pair_dequant_warps(int tile_tok) { return tile_tok <= 192 ? 16 : 8; }
 
 constexpr int pair_kc(int tile_tok) { return tile_tok > 128 ? 64 : 128; }
@@ -40,8 +40,8 @@ struct PairPlan {
     bool fits;             // shared memory holds it
 };
 
-// of tiles of `tile_tok` tokens with stages of `kc` columns
-constexpr PairPlan pair_plan(int tile_tok, int kc)
+// of tiles of `tile_tok` tokens with stages of `kc` columns and `warps` dequant warps
+constexpr PairPlan pair_plan(int tile_tok, int kc, int warps)
 {
     PairPlan l = {tile_tok, kc, 0, kPairMaxWStages, 1, false};
     const int slot = kc / 2, w_bytes = 128 * kc / 2;
@@ -49,7 +49,7 @@ constexpr PairPlan pair_plan(int tile_tok, int kc)
     if (2 * tile_tok + 4 * slot <= kPairTmemCols) l.nd = 2;
     l.stages = (kPairTmemCols - l.nd * tile_tok) / slot;
     if (l.stages > kPairMaxStages) l.stages = kPairMaxStages;
-    const int groups = pair_dequant_warps(tile_tok) / 4;
+    const int groups = warps / 4;
     const int lut = groups == 4 ? kPairLutWide - kPairSmemStart + kPairLutWideBytes : kPairLutBytes;
     const int beside = kPairSmemDynamic - lut - tile_tok * 256;  // what the table and the staging tile leave
     while (l.stages > 4 && l.stages * tile_tok * kc + l.w_stages * w_bytes > beside) --l.stages;
@@ -58,12 +58,13 @@ constexpr PairPlan pair_plan(int tile_tok, int kc)
     l.fits = l.stages * tile_tok * kc + l.w_stages * w_bytes <= beside && rings_shareable(l.w_stages, l.stages, groups);
     return l;
 }
-constexpr PairPlan pair_plan(int tile_tok) { return pair_plan(tile_tok, pair_kc(tile_tok)); }
+constexpr PairPlan pair_plan(int tile_tok, int kc) { return pair_plan(tile_tok, kc, pair_dequant_warps(tile_tok)); }
 
 constexpr bool pair_plans_fit()
 {
     for (int t = 32; t <= 256; t += 32)
-        if (!pair_plan(t).fits) return false;
+        for (int warps = 8; warps <= pair_dequant_warps(t); warps += 8)
+            if (!pair_plan(t, pair_kc(t), warps).fits) return false;
     return true;
 }
 static_assert(pair_plans_fit(), "every token tile has its rings");
