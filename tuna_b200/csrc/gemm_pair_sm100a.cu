@@ -666,7 +666,9 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
 // The estimates below are fitted to 12000 launches (graph replay, short runs): 350 shapes of 512 to 55000 rows, 512 to 28000 columns and
 // 25 to 3900 tokens in every token tile, with 8 and 16 dequant warps, uncut and cut in every way that pair_split considers.  What they choose
 // takes 0.7 % longer than the fastest launch of its shape in the mean, 11 % at worst; with 16 warps wherever they fit and cuts priced by their number of
-// segments alone it was 4 % and 38 %.
+// segments alone it was 4 % and 38 %.  Under the power cap 170 shapes of 3e10 operations or more took 3 % longer than the fastest launch, 27 % at worst
+// (1280x25784 at 2475 tokens: 65 uncut tiles of 192 that walk K together 187 us, 128-token tiles cut 148); constants fitted to both kinds of runs 2 %, but on
+// other shapes they were no faster (60 of 2e10 operations or more under the cap: +0.1 %; 160 in short runs: the same mean, 12 instead of 6 % at worst).
 
 // Microseconds per 16 columns of K of a tile of `tok` tokens: the clocks of the lookups and what goes with them plus the activations'
 // at the 1.7 GHz of a short run, or the tensor pipe's N/2 clocks and what the dequantisation adds to them, at the clock the power cap leaves it.

@@ -39,7 +39,7 @@
 //                MMAs per wait and commit, because that fixed cost per slot is what limits it
 //   warp 1       copy producer of x (fp16 [n,k], L2 resident; one box per 64 columns) into the activation ring
 //   warp 2       copy producer of the packed weights (TMA boxes into the weight ring); it initialises the barriers and issues the
-//                first ring-full ahead of everything: 2000 clocks that the others waited for (4096x4096 at 1 token 7.3 -> 6.8 us a call)
+//                first ring-full ahead of everything: 2000 clocks that the others waited for (4096x4096 at 1 token 7.3 -> 6.8 us, graph replay)
 //   warp 3       no role
 //   warps 4-7    epilogue: tcgen05.ld of the accumulator, fp32 scale by absmax, fp16 store,
 //                split-K partials and fix-up
@@ -463,7 +463,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_w4a16_tstream_kernel(const
     // The flagged quarters of a tile whose partials are all there, shared out over warps `w0`, w0 + step, ... : a warp
     // takes eight tokens of 32 rows at a time, so that all of a tile is in flight at once (28672x4096 at 16 tokens, two row blocks: by
     // four 18.0 us, by eight 17.7), four of them where that takes no second round and there are more than four segments, eight of which
-    // are in flight then (1152x3328 at 11 tokens 6.4 -> 6.0), in exchange launches 16, whole sectors of a peer's slab.
+    // are in flight then (1152x3328 at 11 tokens 6.1 -> 5.7), in exchange launches 16, whole sectors of a peer's slab.
     auto finish_tile = [&](const TsGemm &G, int tile, int first, int nseg, const int *flagged, int w0, int step) __attribute__((always_inline)) {
         const int groups4 = token_groups(G), rb_shift = RB >> 1;
         const int per = p.n_peers > 0 ? 4 : nseg <= 4 || (groups4 << (2 + rb_shift)) > step ? 2 : 1;

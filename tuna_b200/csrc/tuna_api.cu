@@ -63,11 +63,13 @@ static int resolve_config(int m, int n, int k, int sm_count, const tuna_config *
             if (kTable[i].m == m && kTable[i].k == k && kTable[i].n_bucket == b) { c = kTable[i].cfg; break; }
     }
     // No table entry: the tcgen05 weight-streaming kernel up to 24 tokens (the regime bound by HBM), the
-    // kernel on CTA pairs above, which stages half of the tokens per SM.  Measured (us, weight streaming / pairs):
-    // 57344x8192 at 64 tokens 83 / 73, at 32 57 / 67, at 16 54 / 66; 28672x4096 at 64 28.0 / 25.3, at 32 23.2 / 24.8, at 24 21.0 / 24.5;
-    // 4096x4096 at 64 10.9 / 10.7, at 32 8.9 / 9.8; 14336x4096 at 32 15.2 / 14.7, at 24 14.5 / 14.7; 11000x4104 at 32 15.1 / 13.9,
-    // at 24 13.5 / 13.9; 2048x2048 at 32 6.5 / 6.2; 512x512 at 32 4.0 / 3.5, at 24 4.0 / 3.5.  Between 25 and 32 tokens either
-    // leads by up to 15 %, by the shape: the line is where nothing that ran on the pair kernel gets slower.
+    // kernel on CTA pairs above, which stages half of the tokens per SM.  Measured (graph replay, us, weight streaming / pairs):
+    // 57344x8192 at 16 tokens 56.3 / 57.3, at 24 59.4 / 57.3, at 32 61.4 / 58.4; 28672x4096 at 16 19.3 / 20.5, at 20 20.9 / 20.5, at 24
+    // 22.5 / 20.5, at 32 23.3 / 20.9, at 64 28.7 / 22.9; 14336x4096 at 16 13.1 / 12.9, at 24 14.1 / 13.1; 11000x4104 at 16 12.0 / 12.3, at 24
+    // 12.9 / 12.4, at 32 15.3 / 12.4; 10240x8192 at 24 17.0 / 18.4, at 32 18.4 / 18.7; 6144x4096 at 24 9.7 / 9.7; 4096x14336 at 24 14.3 / 14.9, at
+    // 40 17.2 / 16.8; 4096x4096 at 24 7.8 / 9.6, at 32 8.0 / 9.7, at 64 10.2 / 10.0; 2048x2048 at 24 5.7 / 5.9; 512x512 at 16 3.3 / 3.4, at 24
+    // 3.9 / 3.4.  So the token count alone does not draw the line: from 17 to 24 tokens the pair kernel leads by up to 10 % on the matrices that
+    // fill it, from 25 to 40 the other one by up to 17 % on those that do not.
     if (c.path == TUNA_PATH_AUTO) {
         const tuna_config none = {};
         const bool by_shape = !user || std::memcmp(user, &none, sizeof(none)) == 0;
@@ -107,8 +109,10 @@ static int launch_gemm(const GemmArgs &a, const tuna_config &c)
 }
 
 // Whether equal-shape GEMMs share persistent launches of the sequence kernel: every token count it
-// takes (us as launches of the sequence kernel / as calls on the kernel each would take alone: eight 4096x14336 of 16
-// tokens 53 / 115, of 64 83 / 152; eight 28672x4096 of 64 164 / 197; two 57344x8192 of 16 94 / 112, but of 64 161 / 147).
+// takes (graph replay, us, as launches of the sequence kernel / as calls on the kernel each would take alone: eight 4096x14336 of 16
+// tokens 54 / 100, of 64 85 / 133; eight 28672x4096 of 16 100 / 149, of 43 157 / 169, of 64 165 / 171; eight 11000x4104 of 43 69 / 107; sixteen
+// 1024x1024 of 64 13 / 67; two 57344x8192 of 16 100 / 108, but of 43 156 / 127 and of 64 163 / 132: where a matrix fills the pairs for
+// several waves the calls are faster by now).
 static bool batched_as_sequence(const tuna_config &c, int n) { return c.path != TUNA_PATH_STREAM && n <= 64; }
 
 }  // namespace tuna
