@@ -10,8 +10,9 @@
 // of its 2048 weights, 16 for their packed bytes, ~13 for the tensor-memory stores - 189 at N = 256
 // against 128 clocks, which is where the one-SM version of this kernel stopped (0.69 of cuBLAS'
 // bf16 rate).  A CTA pair (cta_group::2, M = 256) stages half of the tokens per SM: 125 at N = 256.  ncu at 57344x8192 and 256
-// tokens counts 48 of them per step for lookups and weight bytes and 32 for the MMAs' operand reads, and sees the tensor
-// pipe active for 87 % of the SMs' active clocks (the one-SM kernel: 49 % of the launch, this one 82 %).
+// tokens in 256-token tiles counts 48 of them per step for lookups and weight bytes and 32 for the MMAs' operand reads, and sees the tensor
+// pipe active for 87 % of the SMs' active clocks (the one-SM kernel: 49 % of the launch, this one 82 %); in 128-token tiles with 16 dequant warps,
+// twice the lookups, 91 and 85 %.
 //
 // One persistent CTA pair per two SMs; each CTA dequantizes its own 128 rows into its own tensor
 // memory, the leader (rank 0) issues the MMAs for both.  16 or 24 warps per CTA:
