@@ -664,16 +664,20 @@ gemm_w4a16_pair_kernel(const __grid_constant__ PairParams p, const __grid_consta
 
 // ------------------------------------------------------------------ host side
 
-// The estimates below are fitted to 12000 launches (graph replay, short runs): 350 shapes of 512 to 55000 rows, 512 to 28000 columns and
-// 25 to 3900 tokens in every token tile, with 8 and 16 dequant warps, uncut and cut in every way that pair_split considers.  What they choose
-// takes 0.7 % longer than the fastest launch of its shape in the mean, 11 % at worst; with 16 warps wherever they fit and cuts priced by their number of
-// segments alone it was 4 % and 38 %.  Under the power cap 170 shapes of 3e10 operations or more took 3 % longer than the fastest launch, 27 % at worst
-// (1280x25784 at 2475 tokens: 65 uncut tiles of 192 that walk K together 187 us, 128-token tiles cut 148); constants fitted to both kinds of runs 2 %, but on
-// other shapes they were no faster (60 of 2e10 operations or more under the cap: +0.1 %; 160 in short runs: the same mean, 12 instead of 6 % at worst).
+// The estimates below are fitted to 16000 launches: in short runs (graph replay) 350 shapes of 512 to 55000 rows, 512 to 28000 columns and
+// 25 to 3900 tokens in every token tile, with 8 and 16 dequant warps, uncut and cut in every way that pair_split considers; and 170 shapes of
+// 3e10 operations or more under the power cap.  What they choose takes 0.7 % (short runs) and 1.9 % (power cap) longer than the fastest launch of its shape
+// in the mean, 16 % at worst; with 16 warps wherever they fit and cuts priced by their number of segments alone it was 4 and 3.7 %, and 38 % at worst.  Fitted
+// to the short runs alone it was 0.7 and 3 %, and on 40 other shapes whose activations are a good part of L2 or more 1.4 % slower than so.  Those are
+// the least predictable: 6 % longer than the fastest launch in the mean, 31 % at worst (tiles out of step no longer share what L2 holds).
 
-// Microseconds per 16 columns of K of a tile of `tok` tokens: the clocks of the lookups and what goes with them plus the activations'
-// at the 1.7 GHz of a short run, or the tensor pipe's N/2 clocks and what the dequantisation adds to them, at the clock the power cap leaves it.
-static double pair_step_us(int tok, int warps) { return std::max((tok / 4 + (warps == 16 ? 50 : 71)) / 1700.0, (tok / 2 + 8) / 1420.0); }
+// Microseconds per 16 columns of K of a tile of `tok` tokens: the clocks of the lookups and what goes with them plus the activations',
+// at the 1.7 GHz of a short run, or the tensor pipe's N/2 clocks and what the dequantisation adds to them, at a clock between that and the one
+// that the power cap leaves (128 / 192 / 256 tokens: 0.052 / 0.075 / 0.101 in short runs, 0.059 / 0.088 / 0.117 under the cap).
+static double pair_step_us(int tok, int warps)
+{
+    return std::max((warps == 16 ? 50 + 0.25 * tok : 73 + 0.26 * tok) / 1700.0, (tok / 2 + 14) / 1540.0);
+}
 
 // How the tiles of a launch are handed out (see the head of the file): sk_tiles of them are cut along K over
 // sk_pairs pairs, the others go out in whole waves.
@@ -690,22 +694,21 @@ struct PairSplit {
 // 64-token tiles, 5.1 / 4.9; ahead of it 3072x768 at 60 3.9 / 4.0).
 static double pair_uncut_us(int cols, int warps, bool ahead)
 {
-    return 2.6 + 0.007 * cols + (warps == 16 ? 0.7 : (ahead ? 0.0 : std::max(0.0, 0.7 - 0.0055 * cols)));
+    return 2.6 + 0.007 * cols + (warps == 16 ? 0.95 : (ahead ? 0.0 : std::max(0.0, 0.7 - 0.006 * cols)));
 }
-constexpr double kPairWaveUs = 0.1;  // from one wave of whole tiles to the next
 // What cutting costs: partial sums written, an arrival, and adding them up.
-static double pair_cut_us(int cols, int warps) { return 5.2 + 0.03 * cols + 0.045 * std::max(0, cols - 128) + (warps == 16 ? 0.35 : 0.0); }
+static double pair_cut_us(int cols, int warps) { return 5.2 + 0.029 * cols + 0.008 * std::max(0, cols - 128) + (warps == 16 ? 0.65 : 0.0); }
 // Adding up `segs` segments of a tile at the end of a CTA: a round is as many loads as its warps have in flight.
 static double pair_add_us(int cols, int warps, int segs)
 {
     const int rounds = warps == 8 ? div_up(segs, 4) * div_up(cols / 4, 16) : (cols == 32 ? div_up(segs, 4) : div_up(segs, 2) * div_up(cols / 4, 24));
-    return 0.83 * rounds;
+    return 0.9 * rounds;
 }
 // Ranges that do not end where a tile does: their CTAs work on two tiles, and a tile has one segment more (528x4480 at 44 tokens, 35 chunks a
 // tile: four segments 10.2 us, five 8.4).
-constexpr double kPairRaggedUs = 2.5;
+static double pair_ragged_us(int cols) { return 2.0 + 0.01 * cols; }
 // Cut tiles in front of whole ones.
-constexpr double kPairMixedUs = 3.6;
+constexpr double kPairMixedUs = 1.7;
 // A launch that leaves half of the pairs idle: the next one starts on those (6272x1792 at 42 tokens: one tile of 64 per 256 rows 6.5 us, two
 // of 32 8.0).
 constexpr double kPairOverlapUs = 1.2;
@@ -729,21 +732,21 @@ static PairSplit pair_split(int m, int n, int k, int tile_tok, int pairs)
         };
         const double uncut_us = pair_uncut_us(cols, warps, n <= kPairAheadTokens), cut_us = pair_cut_us(cols, warps);
         // a wave of tiles of two widths takes as long as something between their mean and the wider one
-        const double wave_us = 0.5 * (tile_us + work_us * pairs / tiles) + kPairWaveUs;
-        consider(0, 0, waves == 0 ? uncut_us + tile_us + kPairWaveUs - overlap(tiles) : uncut_us + (waves + (rest ? 1 : 0)) * wave_us);
+        const double wave_us = (tile_us + 2 * work_us * pairs / tiles) / 3;
+        consider(0, 0, waves == 0 ? uncut_us + tile_us - overlap(tiles) : uncut_us + (waves + (rest ? 1 : 0)) * wave_us);
         // where there is more than one wave of whole tiles, adding up hides behind them
         if (rest > 0 && waves > 0)
-            consider(pairs + rest, pairs, work_us + waves * kPairWaveUs + cut_us + kPairMixedUs + (waves > 1 ? 0.0 : pair_add_us(cols, warps, 2)));
+            consider(pairs + rest, pairs, work_us + cut_us + kPairMixedUs + (waves > 1 ? 0.0 : pair_add_us(cols, warps, 2)));
         if (waves == 0) {
             int s = 2;
             for (; s * tiles <= pairs && s <= chunks; ++s) {
                 const bool ragged = chunks % s != 0;
                 consider((int)tiles, s * (int)tiles,
-                         tile_us * div_up(chunks, s) / chunks + cut_us + pair_add_us(cols, warps, s + ragged) + (ragged ? kPairRaggedUs : 0.0) - overlap(s * tiles));
+                         tile_us * div_up(chunks, s) / chunks + cut_us + pair_add_us(cols, warps, s + ragged) + (ragged ? pair_ragged_us(cols) : 0.0) - overlap(s * tiles));
             }
             // all pairs, where whole segments leave more than a tenth of them idle
             if (s <= chunks && (s - 1) * tiles * 10 < pairs * 9)
-                consider((int)tiles, pairs, work_us + cut_us + pair_add_us(cols, warps, pairs / (int)tiles + 1) + kPairRaggedUs);
+                consider((int)tiles, pairs, work_us + cut_us + pair_add_us(cols, warps, pairs / (int)tiles + 1) + pair_ragged_us(cols));
         }
     }
     return best;
